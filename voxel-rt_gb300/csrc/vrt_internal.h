@@ -112,6 +112,12 @@ namespace vrt {
 int refresh_masks(vrt_world* w, uint64_t first, uint64_t count, cudaStream_t s);
 // Rebuild the masks of the voxel box [x0,x1)x[y0,y1)x[z0,z1) (clipped).
 int refresh_masks_box(vrt_world* w, int x0, int y0, int z0, int x1, int y1, int z1, cudaStream_t s);
+// fixDepthField (render.cpp:226-253) for the voxels of the box [x0,x1)x[y0,y1)x[z0,z1)
+// (clipped to the world); with r2 > 0 only for those of the sphere |v - c|^2 < r2^2
+// (removeSphere's second loop, level.cpp:43-55).  Reads solidity from the brick masks,
+// which have to be up to date.
+int launch_fix_depth_field(vrt_world* w, int x0, int y0, int z0, int x1, int y1, int z1, int cx, int cy, int cz,
+                           int r2, cudaStream_t s);
 // Bring the stop masks and their directed distances up to date (allocated on first use),
 // and make stream s wait until they are: the rebuild may have run on another stream.
 int refresh_stop(vrt_world* w, cudaStream_t s);

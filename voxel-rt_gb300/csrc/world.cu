@@ -1,7 +1,7 @@
 // Device-resident worlds: the voxel words (the reference's SSBO), the derived occupancy
 // hierarchy, and the edit kernels that replace the reference's CPU world code:
 //   removeSphere  level.cpp:30-56        -> remove_sphere_kernel + mask refresh + depth refresh
-//   fixDepthField render.cpp:226-253     -> fix_depth_field_kernel
+//   fixDepthField render.cpp:226-253     -> fix_depth_field_kernel (world_passes.cu)
 //   placeVoxel    render.cpp:256-262     -> place_voxel_kernel
 //   initVoxels    level.cpp:82-138       -> init_reference_layers_kernel + init_reference_trees_kernel
 //   updateGeometry/updatePartialGeometry render.cpp:199-223 -> vrt_world_upload (+ mask refresh)
@@ -9,10 +9,8 @@
 
 #include <algorithm>
 #include <climits>
-#include <cmath>
 #include <cstdio>
 #include <cstring>
-#include <mutex>
 #include <vector>
 
 #include "vrt_internal.h"
@@ -288,8 +286,14 @@ int refresh_stop(vrt_world* w, cudaStream_t s) {
     return VRT_OK;
 }
 
-// The words of the box [x0,x1)x[y0,y1)x[z0,z1) changed: the z-major copy must follow there.
-static void mark_words_z(vrt_world* w, int x0, int y0, int z0, int x1, int y1, int z1) {
+// The words of the box [x0,x1)x[y0,y1)x[z0,z1) changed (clipped to the world): the stop
+// masks and, there, the z-major copy must follow.
+static void mark_words(vrt_world* w, int x0, int y0, int z0, int x1, int y1, int z1) {
+    x0 = std::max(x0, 0); y0 = std::max(y0, 0); z0 = std::max(z0, 0);
+    x1 = std::min(x1, w->L.W); y1 = std::min(y1, w->L.H); z1 = std::min(z1, w->L.W);
+    if (x0 >= x1 || y0 >= y1 || z0 >= z1) return;
+    w->stop_stale = true;
+    if (!w->d_words_z) return;
     int* b = w->z_dirty;
     if (b[0] >= b[3]) {
         b[0] = x0; b[1] = y0; b[2] = z0; b[3] = x1; b[4] = y1; b[5] = z1;
@@ -364,8 +368,7 @@ int refresh_masks_box(vrt_world* w, int x0, int y0, int z0, int x1, int y1, int 
     x0 = std::max(x0, 0); y0 = std::max(y0, 0); z0 = std::max(z0, 0);
     x1 = std::min(x1, L.W); y1 = std::min(y1, L.H); z1 = std::min(z1, L.W);
     if (x0 >= x1 || y0 >= y1 || z0 >= z1) return VRT_OK;
-    w->stop_stale = true;
-    if (w->d_words_z) mark_words_z(w, x0, y0, z0, x1, y1, z1);
+    mark_words(w, x0, y0, z0, x1, y1, z1);
     int bx0 = x0 >> 2, by0 = y0 >> 2, bz0 = z0 >> 2;
     int bx1 = (x1 + 3) >> 2, by1 = (y1 + 3) >> 2, bz1 = (z1 + 3) >> 2;
     uint64_t nb = (uint64_t)(bx1 - bx0) * (by1 - by0) * (bz1 - bz0);
@@ -427,136 +430,6 @@ __global__ void remove_sphere_kernel(int32_t* __restrict__ words, Layout L, int 
 __global__ void place_voxel_kernel(int32_t* words, Layout L, int x, int y, int z, int32_t v) {
     if (x >= 0 && y >= 0 && z >= 0 && x < L.W && y < L.H && z < L.W)
         words[(uint64_t)x + (uint64_t)L.W * y + (uint64_t)L.W * L.H * z] = v;
-}
-
-// Depth-field offsets of computeDepthIndices (render.cpp:66-100), reduced to what
-// fixDepthField (render.cpp:226-253) can use.  fixDepthField keeps, over the solid
-// neighbours in the radius-7 sphere whose shrunk distance d beats the running value
-// (start -6), the value (d <= -2 ? d : 0); the running value only grows and that map
-// is monotone, so the result is g(max d) over solid neighbours with d > -6, whatever
-// the visiting order.  The table therefore holds the sphere offsets with d > -6 sorted
-// by decreasing d, and the kernel stops at the first solid neighbour.
-struct DepthOff {
-    float dist;
-    int8_t x, y, z, pad;
-};
-__constant__ DepthOff c_depth_offs[1536];  // 1413 offsets of the radius-7 sphere have d > -6
-__constant__ int c_depth_count;
-__device__ DepthOff g_depth_offs[1536];    // the same table, read by the lanes of a warp at once
-static std::once_flag g_depth_once;
-static int g_depth_count = 0;
-static std::vector<DepthOff> g_depth_table;
-
-static void build_depth_table() {
-    const int R = 7;  // DEPTH_FIELD_RADIUS, render.hpp:7
-    std::vector<DepthOff> v;
-    for (int z = -R; z <= R; z++)
-        for (int y = -R; y <= R; y++)
-            for (int x = -R; x <= R; x++) {
-                if (x * x + y * y + z * z > R * R) continue;
-                int xd = x - (x > 0) + (x < 0), yd = y - (y > 0) + (y < 0), zd = z - (z > 0) + (z < 0);
-                // render.cpp:81: dist = -sqrt(int) through double sqrt, stored as float
-                float dist = (float)(-std::sqrt((double)(xd * xd + yd * yd + zd * zd)));
-                if (dist > (float)(-R + 1)) v.push_back(DepthOff{dist, (int8_t)x, (int8_t)y, (int8_t)z, 0});
-            }
-    std::stable_sort(v.begin(), v.end(), [](const DepthOff& a, const DepthOff& b) { return a.dist > b.dist; });
-    g_depth_table = v;
-    g_depth_count = (int)v.size();
-}
-
-static int ensure_depth_table() {
-    std::call_once(g_depth_once, build_depth_table);
-    // constant memory is per device: upload each time (cheap, 8 KB) to stay correct on any device
-    VRT_CUDA(cudaMemcpyToSymbol(c_depth_offs, g_depth_table.data(), g_depth_table.size() * sizeof(DepthOff)));
-    VRT_CUDA(cudaMemcpyToSymbol(g_depth_offs, g_depth_table.data(), g_depth_table.size() * sizeof(DepthOff)));
-    VRT_CUDA(cudaMemcpyToSymbol(c_depth_count, &g_depth_count, sizeof(int)));
-    return VRT_OK;
-}
-
-// fixDepthField (render.cpp:226-253) for every voxel of the box, or of the sphere
-// x*x+y*y+z*z < r2*r2 around (cx,cy,cz) when r2 > 0 (removeSphere's second loop,
-// level.cpp:43-55).  Neighbours outside the world count as not solid (the reference
-// reads voxels[-1] there).  Only air words are written and only solidity is read, so
-// voxels of one launch do not interact.
-__global__ void fix_depth_field_kernel(int32_t* words, Layout L, int x0, int y0, int z0, int nx,
-                                       int ny, int nz, int cx, int cy, int cz, int r2) {
-    uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (uint64_t)nx * ny * nz) return;
-    int x = x0 + (int)(t % nx), y = y0 + (int)((t / nx) % ny), z = z0 + (int)(t / ((uint64_t)nx * ny));
-    if (x < 0 || y < 0 || z < 0 || x >= L.W || y >= L.H || z >= L.W) return;
-    if (r2 > 0) {
-        int ox = x - cx, oy = y - cy, oz = z - cz;
-        if (ox * ox + oy * oy + oz * oz >= r2 * r2) return;
-    }
-    uint64_t idx = (uint64_t)x + (uint64_t)L.W * y + (uint64_t)L.W * L.H * z;
-    if (words[idx] >= 0) return;
-    float nearest = -6.0f;  // -DEPTH_FIELD_RADIUS + 1
-    const int n = c_depth_count;
-    for (int i = 0; i < n; i++) {
-        DepthOff o = c_depth_offs[i];
-        int qx = x + o.x, qy = y + o.y, qz = z + o.z;
-        if (qx < 0 || qy < 0 || qz < 0 || qx >= L.W || qy >= L.H || qz >= L.W) continue;
-        // plain load: this launch writes other air words of the same array
-        if (words[(uint64_t)qx + (uint64_t)L.W * qy + (uint64_t)L.W * L.H * qz] >= 0) {
-            nearest = o.dist <= -2.0f ? o.dist : 0.0f;
-            break;
-        }
-    }
-    if (nearest < 0.0f) words[idx] = __float_as_int(nearest);
-}
-
-// fix_depth_field_kernel with one warp per voxel, for edit-sized boxes: one thread per
-// voxel leaves most SMs idle there while each thread walks the offset table in turn.  The
-// lanes test 32 consecutive table offsets at a time and a ballot picks the first solid
-// one in table order -- the offset the one-thread loop stops at -- so the words written
-// are the same.
-__global__ void fix_depth_field_warp_kernel(int32_t* words, Layout L, int x0, int y0, int z0, int nx, int ny,
-                                            int nz, int cx, int cy, int cz, int r2) {
-    const uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // this warp's voxel
-    const int lane = threadIdx.x & 31;
-    if (t >= (uint64_t)nx * ny * nz) return;  // the returns before the ballot are warp-uniform
-    const int x = x0 + (int)(t % nx), y = y0 + (int)((t / nx) % ny), z = z0 + (int)(t / ((uint64_t)nx * ny));
-    if (x < 0 || y < 0 || z < 0 || x >= L.W || y >= L.H || z >= L.W) return;
-    if (r2 > 0) {
-        const int ox = x - cx, oy = y - cy, oz = z - cz;
-        if (ox * ox + oy * oy + oz * oz >= r2 * r2) return;
-    }
-    const uint64_t idx = (uint64_t)x + (uint64_t)L.W * y + (uint64_t)L.W * L.H * z;
-    if (words[idx] >= 0) return;
-    float nearest = -6.0f;  // -DEPTH_FIELD_RADIUS + 1
-    const int n = c_depth_count;
-    for (int base = 0; base < n; base += 32) {
-        const int i = base + lane;
-        bool solid = false;
-        if (i < n) {
-            const DepthOff o = g_depth_offs[i];
-            const int qx = x + o.x, qy = y + o.y, qz = z + o.z;
-            if (qx >= 0 && qy >= 0 && qz >= 0 && qx < L.W && qy < L.H && qz < L.W)
-                solid = words[(uint64_t)qx + (uint64_t)L.W * qy + (uint64_t)L.W * L.H * qz] >= 0;  // plain load
-        }
-        const unsigned hits = __ballot_sync(0xffffffffu, solid);
-        if (hits) {
-            const float d = g_depth_offs[base + __ffs(hits) - 1].dist;
-            nearest = d <= -2.0f ? d : 0.0f;
-            break;
-        }
-    }
-    if (lane == 0 && nearest < 0.0f) words[idx] = __float_as_int(nearest);
-}
-
-// Boxes of at most this many voxels take the warp-per-voxel kernel (the edit of a
-// radius-1024 sphere would otherwise launch 2^38 threads).
-constexpr uint64_t kWarpPerVoxelMax = 1ull << 22;
-
-static void launch_fix_depth_field(vrt_world* w, int x0, int y0, int z0, int nx, int ny, int nz, int cx, int cy, int cz,
-                                   int r2, cudaStream_t s) {
-    const uint64_t n = (uint64_t)nx * ny * nz;
-    if (n <= kWarpPerVoxelMax)
-        fix_depth_field_warp_kernel<<<blocks_for(n * 32, 256), 256, 0, s>>>(w->d_words, w->L, x0, y0, z0, nx, ny, nz,
-                                                                            cx, cy, cz, r2);
-    else
-        fix_depth_field_kernel<<<blocks_for(n, 256), 256, 0, s>>>(w->d_words, w->L, x0, y0, z0, nx, ny, nz, cx, cy,
-                                                                  cz, r2);
 }
 
 __global__ void probe_kernel(const int32_t* __restrict__ words, Layout L, const int32_t* __restrict__ xyz, int n,
@@ -872,12 +745,10 @@ int vrt_fix_depth_field_box(vrt_world* w, int32_t x0, int32_t y0, int32_t z0, in
     x0 = std::max(x0, 0); y0 = std::max(y0, 0); z0 = std::max(z0, 0);
     x1 = std::min(x1, w->L.W); y1 = std::min(y1, w->L.H); z1 = std::min(z1, w->L.W);
     if (x0 >= x1 || y0 >= y1 || z0 >= z1) return VRT_OK;
-    int st = ensure_depth_table();
-    if (st) return st;
-    launch_fix_depth_field(w, x0, y0, z0, x1 - x0, y1 - y0, z1 - z0, 0, 0, 0, 0, S(stream));
-    VRT_CUDA(cudaGetLastError());
+    // the depth field changes air words only, so the occupancy structures stay as they are
+    mark_words(w, x0, y0, z0, x1, y1, z1);
     w->has_depth_field = 1;
-    return refresh_masks_box(w, x0, y0, z0, x1, y1, z1, S(stream));
+    return launch_fix_depth_field(w, x0, y0, z0, x1, y1, z1, 0, 0, 0, 0, S(stream));
 }
 
 int vrt_remove_sphere(vrt_world* w, int32_t cx, int32_t cy, int32_t cz, int32_t radius, int32_t refresh_depth_field,
@@ -888,18 +759,16 @@ int vrt_remove_sphere(vrt_world* w, int32_t cx, int32_t cy, int32_t cz, int32_t 
         uint64_t n = (uint64_t)(2 * radius) * (2 * radius) * (2 * radius);
         remove_sphere_kernel<<<blocks_for(n, 256), 256, 0, S(stream)>>>(w->d_words, w->L, cx, cy, cz, radius);
         VRT_CUDA(cudaGetLastError());
-    }
-    int r2 = radius + (7 >> 1);  // DEPTH_FIELD_RADIUS >> 1, level.cpp:43
-    if (refresh_depth_field && r2 > 0) {
-        int st = ensure_depth_table();
+        // the masks first: the depth field reads solidity from them
+        int st = refresh_masks_box(w, cx - radius, cy - radius, cz - radius, cx + radius, cy + radius, cz + radius,
+                                   S(stream));
         if (st) return st;
-        const int n = 2 * r2;
-        launch_fix_depth_field(w, cx - r2, cy - r2, cz - r2, n, n, n, cx, cy, cz, r2, S(stream));
-        VRT_CUDA(cudaGetLastError());
-        w->has_depth_field = 1;
     }
-    int rb = std::max(radius, refresh_depth_field ? r2 : radius);
-    return refresh_masks_box(w, cx - rb, cy - rb, cz - rb, cx + rb, cy + rb, cz + rb, S(stream));
+    if (!refresh_depth_field) return VRT_OK;
+    const int r2 = radius + (7 >> 1);  // DEPTH_FIELD_RADIUS >> 1, level.cpp:43
+    mark_words(w, cx - r2, cy - r2, cz - r2, cx + r2, cy + r2, cz + r2);
+    w->has_depth_field = 1;
+    return launch_fix_depth_field(w, cx - r2, cy - r2, cz - r2, cx + r2, cy + r2, cz + r2, cx, cy, cz, r2, S(stream));
 }
 
 int vrt_world_init_reference(vrt_world* w, void* stream) {
