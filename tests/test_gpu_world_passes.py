@@ -4,7 +4,7 @@ the depth field's radius) and dense ones, against the oracle, word for word."""
 import numpy as np
 import pytest
 
-from helpers import make_world
+from helpers import expected_distances, expected_masks, make_world
 
 pytestmark = pytest.mark.gpu
 
@@ -50,3 +50,45 @@ def test_removed_spheres_refresh_the_depth_field(cuda, oracle, W, H):
         oracle.remove_sphere(ref, W, H, *c, r, 1)
         got = w.download(np.empty_like(ref))
         assert np.array_equal(got, ref), (c, r)
+
+
+def check_structures(w, words, W, H):
+    bricks, regions, supers = w.masks()
+    eb, er, es = expected_masks(words, W, H)
+    assert np.array_equal(bricks, eb) and np.array_equal(regions, er) and np.array_equal(supers, es)
+    bdir, rdist = w.distances()
+    ed, erd = expected_distances(words, W, H)
+    assert np.array_equal(bdir, ed) and np.array_equal(rdist, erd)
+
+
+@pytest.mark.parametrize("W,H", [(3, 130), (64, 64), (70, 47), (129, 20), (257, 65)])
+def test_structures_follow_uploads_and_edits(cuda, W, H):
+    """Masks of every level and both distance fields after whole and partial uploads from
+    host and device memory at odd offsets (bricks fill and empty in one pass), removed
+    spheres and placed voxels, against the model built from the words."""
+    rng = np.random.default_rng(W)
+    n = W * H * W
+    words = sparse_words(W, H, W, 0.0002)
+    w = make_world(words, W, H)
+    check_structures(w, words, W, H)
+    for k, density in enumerate((0.0001, 0.02, 0.0)):
+        first = int(rng.integers(0, n // 2))
+        part = sparse_words(W, H, 10 + k, density)[: int(rng.integers(1, n - first))]
+        if k == 1:
+            w.upload(part, first)
+        else:
+            pad = 1 + k  # a source address that is not 16-byte aligned
+            d = cuda.from_numpy(np.concatenate([np.zeros(pad, np.int32), part])).cuda()
+            w.upload_device(d.data_ptr() + 4 * pad, first, part.size)
+        words[first:first + part.size] = part
+        got = w.download(np.empty_like(words))
+        assert np.array_equal(got, words)
+        check_structures(w, words, W, H)
+        assert w.info().has_depth_field == int((words < -1).any())
+    w.place_voxel(W - 1, H - 1, 0, 0x01FFFFFF)
+    words[W - 1 + W * (H - 1)] = 0x01FFFFFF
+    w.remove_sphere(W // 2, H // 2, W // 2, 9, 0)
+    z, y, x = np.meshgrid(np.arange(W) - W // 2, np.arange(H) - H // 2, np.arange(W) - W // 2, indexing="ij")
+    words.reshape(W, H, W)[x * x + y * y + z * z < 81] = -1
+    assert np.array_equal(w.download(np.empty_like(words)), words)
+    check_structures(w, words, W, H)

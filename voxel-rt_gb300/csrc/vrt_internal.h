@@ -95,29 +95,43 @@ struct vrt_world {
     int z_dirty[6] = {0, 0, 0, 0, 0, 0};  // box [x0,x1)x[y0,y1)x[z0,z1) of words changed since the
                                     // copy was last brought up to date (empty: x0 >= x1)
     cudaEvent_t z_ready = nullptr;  // recorded after each copy update: renders on other streams wait on it
-    uint8_t* d_tmp_a = nullptr;     // scratch of the distance passes (8 * n_bricks each)
-    uint8_t* d_tmp_b = nullptr;
-    int* d_flag = nullptr;          // has-depth-field flag written by the mask kernels
+    uint64_t* d_stop_regions = nullptr;  // region masks of the stop masks
+    int* d_boxes = nullptr;         // the brick pass's record per CTA (8 ints: solid box, flag, 0)
     int* d_aabb = nullptr;          // bounding box of the solid voxels, brick-granular and
-                                    // never smaller than the truth: min x,y,z then max x,y,z
+                                    // never smaller than the truth: min x,y,z then max x,y,z;
+                                    // [6] the has-depth-field flag
     int h_aabb[6] = {0, 0, 0, -1, -1, -1};  // host copy passed to the render kernels; kept a
                                     // superset of the device box (read back after uploads)
     int has_depth_field = 0;        // host copy (as of the last sync)
     uint64_t device_bytes = 0;
     int device = 0;
+    int num_sms = 0;
 };
 
 namespace vrt {
-// Rebuild the masks of every brick overlapping words [first, first+count).
-int refresh_masks(vrt_world* w, uint64_t first, uint64_t count, cudaStream_t s);
-// Rebuild the masks of the voxel box [x0,x1)x[y0,y1)x[z0,z1) (clipped).
-int refresh_masks_box(vrt_world* w, int x0, int y0, int z0, int x1, int y1, int z1, cudaStream_t s);
-// fixDepthField (render.cpp:226-253) for the voxels of the box [x0,x1)x[y0,y1)x[z0,z1)
-// (clipped to the world); with r2 > 0 only for those of the sphere |v - c|^2 < r2^2
-// (removeSphere's second loop, level.cpp:43-55).  Reads solidity from the brick masks,
-// which have to be up to date.
-int launch_fix_depth_field(vrt_world* w, int x0, int y0, int z0, int x1, int y1, int z1, int cx, int cy, int cz,
-                           int r2, cudaStream_t s);
+// A change of a world's words and what follows from it (world_passes.cu).
+enum { kReadWords, kRemoveSphere, kPlaceVoxel, kCopyWords, kStopWords };
+struct WordChange {
+    int op;                 // kReadWords: the words changed already, or are to be looked at again
+    int64_t box[6];         // the words concerned: [x0,y0,z0, x1,y1,z1), clipped to the world; may be empty
+    const int32_t* src;     // kCopyWords: words [first, first + count) are copied from here
+    uint64_t first, count;
+    int x, y, z, r;         // kRemoveSphere: |v - c|^2 < r^2 becomes air; kPlaceVoxel: the voxel
+    int32_t word;           // kPlaceVoxel
+    bool reset_flag;        // whole-world boxes: the depth-field flag starts from 0
+    bool fix;               // then fixDepthField (render.cpp:226-253) over fix_box, and with
+    int64_t fix_box[6];     // fix_r > 0 only over its voxels with |v - c|^2 < fix_r^2 (removeSphere's
+    int fix_r;              // second loop, level.cpp:43-55)
+};
+// Change the words, and bring the masks, distances, solid box and flag up to date: at most two
+// launches.
+int change_words(vrt_world* w, const WordChange& c, cudaStream_t s);
+// Note that the words of the box changed: the stop masks and, there, the z-major copy follow.
+void mark_words(vrt_world* w, const int64_t box[6]);
+// CTAs of a brick pass per SM, at most
+constexpr int kBrickCtasPerSm = 6;
+// Rebuild the stop masks and their directed distances from the words.
+int refresh_stop_masks(vrt_world* w, cudaStream_t s);
 // Bring the stop masks and their directed distances up to date (allocated on first use),
 // and make stream s wait until they are: the rebuild may have run on another stream.
 int refresh_stop(vrt_world* w, cudaStream_t s);

@@ -1,10 +1,10 @@
 // Device-resident worlds: the voxel words (the reference's SSBO), the derived occupancy
 // hierarchy, and the edit kernels that replace the reference's CPU world code:
-//   removeSphere  level.cpp:30-56        -> remove_sphere_kernel + mask refresh + depth refresh
-//   fixDepthField render.cpp:226-253     -> fix_depth_field_kernel (world_passes.cu)
-//   placeVoxel    render.cpp:256-262     -> place_voxel_kernel
+//   removeSphere  level.cpp:30-56        -> change_words (world_passes.cu)
+//   fixDepthField render.cpp:226-253     -> change_words
+//   placeVoxel    render.cpp:256-262     -> change_words
 //   initVoxels    level.cpp:82-138       -> init_reference_layers_kernel + init_reference_trees_kernel
-//   updateGeometry/updatePartialGeometry render.cpp:199-223 -> vrt_world_upload (+ mask refresh)
+//   updateGeometry/updatePartialGeometry render.cpp:199-223 -> vrt_world_upload -> change_words
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -36,224 +36,7 @@ Layout make_layout(int W, int H) {
     return L;
 }
 
-// ------------------------------------------------------------------ mask kernels
-
-// One thread per brick of the brick box [b0, b1): OR of (word >= 0) over its 4x4x4
-// voxels; any word < -1 raises the depth-field flag.
-__global__ void brick_mask_kernel(const int32_t* __restrict__ words, uint64_t* __restrict__ bricks, int* flag,
-                                  int* aabb, Layout L, int bx0, int by0, int bz0, int nbx, int nby, int nbz) {
-    uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    uint64_t total = (uint64_t)nbx * nby * nbz;
-    if (t >= total) return;
-    int bx = bx0 + (int)(t % nbx);
-    int by = by0 + (int)((t / nbx) % nby);
-    int bz = bz0 + (int)(t / ((uint64_t)nbx * nby));
-    uint64_t m = 0;
-    bool depth = false;
-    const int x0 = bx * 4;
-    const bool vec = (x0 + 4 <= L.W) && ((L.W & 3) == 0);
-    for (int dz = 0; dz < 4; dz++) {
-        int z = bz * 4 + dz;
-        if (z >= L.W) break;
-        for (int dy = 0; dy < 4; dy++) {
-            int y = by * 4 + dy;
-            if (y >= L.H) break;
-            const int32_t* row = words + ((uint64_t)z * L.H + y) * L.W;
-            int v[4];
-            if (vec) {
-                int4 q = __ldg(reinterpret_cast<const int4*>(row + x0));
-                v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
-            } else {
-                for (int dx = 0; dx < 4; dx++) v[dx] = (x0 + dx < L.W) ? __ldg(row + x0 + dx) : -1;
-            }
-            for (int dx = 0; dx < 4; dx++) {
-                if (v[dx] >= 0) m |= 1ull << (dx + 4 * dy + 16 * dz);
-                depth |= (v[dx] < -1);
-            }
-        }
-    }
-    bricks[brick_index(L, bx, by, bz)] = m;
-    if (depth) atomicOr(flag, 1);
-    // grow the solid bounding box by this brick (one atomic per warp and bound)
-    const unsigned mask = __activemask();
-    int v[6];
-    if (m) {
-        v[0] = 4 * bx; v[1] = 4 * by; v[2] = 4 * bz;
-        v[3] = 4 * bx + 3; v[4] = 4 * by + 3; v[5] = 4 * bz + 3;
-    } else {
-        v[0] = v[1] = v[2] = INT_MAX;
-        v[3] = v[4] = v[5] = INT_MIN;
-    }
-    for (int i = 0; i < 3; i++) v[i] = __reduce_min_sync(mask, v[i]);
-    for (int i = 3; i < 6; i++) v[i] = __reduce_max_sync(mask, v[i]);
-    if ((threadIdx.x & 31) == (__ffs(mask) - 1) && v[0] != INT_MAX) {
-        for (int i = 0; i < 3; i++) atomicMin(aabb + i, v[i]);
-        for (int i = 3; i < 6; i++) atomicMax(aabb + i, v[i]);
-    }
-}
-
-__global__ void reset_aabb_kernel(int* aabb) {
-    if (threadIdx.x < 3) aabb[threadIdx.x] = INT_MAX;
-    else if (threadIdx.x < 6) aabb[threadIdx.x] = INT_MIN;
-}
-
-// One thread per node of the parent box: bit i set when child i is non-zero.
-// children are stored as 64 consecutive uint64 per parent (region-major / super-major).
-__global__ void parent_mask_kernel(const uint64_t* __restrict__ child, uint64_t* __restrict__ parent,
-                                   int px0, int py0, int pz0, int npx, int npy, int npz, Layout L, int level) {
-    uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    uint64_t total = (uint64_t)npx * npy * npz;
-    if (t >= total) return;
-    int px = px0 + (int)(t % npx);
-    int py = py0 + (int)((t / npx) % npy);
-    int pz = pz0 + (int)(t / ((uint64_t)npx * npy));
-    uint64_t slot = level == 1 ? region_index(L, px, py, pz) : super_index(L, px, py, pz);
-    uint64_t m = 0;
-    if (level == 1) {  // the region's 4x4x4 bricks: 16 rows of 4 consecutive slots
-        for (int lz = 0; lz < 4; lz++)
-            for (int ly = 0; ly < 4; ly++) {
-                const uint64_t* row = child + brick_index(L, 4 * px, 4 * py + ly, 4 * pz + lz);
-                for (int lx = 0; lx < 4; lx++) m |= (uint64_t)(row[lx] != 0) << (lx + 4 * ly + 16 * lz);
-            }
-    } else {  // a super block's 64 regions are consecutive
-        const uint64_t* c = child + slot * 64;
-        for (int i = 0; i < 64; i += 2) {
-            ulonglong2 q = *reinterpret_cast<const ulonglong2*>(c + i);
-            m |= (uint64_t)(q.x != 0) << i;
-            m |= (uint64_t)(q.y != 0) << (i + 1);
-        }
-    }
-    parent[slot] = m;
-}
-
 static inline unsigned blocks_for(uint64_t n, int threads) { return (unsigned)((n + threads - 1) / threads); }
-
-// One 1-D pass of the capped Chebyshev distance transform over the region grid:
-//   out(p) = min over |k| <= cap of max(|k|, in(p + k e_axis)),
-// where in() of the first pass is 0 for a non-empty region and cap+1 for an empty one, and
-// regions outside the padded grid are empty.  Three passes (x, y, z) give the L-inf distance.
-__global__ void cheb_pass_kernel(const uint64_t* __restrict__ occ, const uint8_t* __restrict__ in,
-                                 uint8_t* __restrict__ out, Layout L, int axis, int first) {
-    const int DX = L.RWp, DY = L.RHp;
-    uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (uint64_t)DX * DY * DX) return;
-    const int x = (int)(t % DX), y = (int)((t / DX) % DY), z = (int)(t / ((uint64_t)DX * DY));
-    const int cap = kDistCap;
-    int best = cap + 1;
-    for (int k = -cap; k <= cap; k++) {
-        int qx = x + (axis == 0 ? k : 0), qy = y + (axis == 1 ? k : 0), qz = z + (axis == 2 ? k : 0);
-        if (qx < 0 || qy < 0 || qz < 0 || qx >= DX || qy >= DY || qz >= DX) continue;
-        const int v = first ? (occ[region_index(L, qx, qy, qz)] != 0 ? 0 : cap + 1) : in[region_linear(L, qx, qy, qz)];
-        int a = k < 0 ? -k : k;
-        best = min(best, max(a, v));
-    }
-    out[region_linear(L, x, y, z)] = (uint8_t)min(best, cap);
-}
-
-// One axis pass of the directed brick distances, all eight octants at once (one byte
-// each): out_o(b) = min over j in [0, cap] of max(j, in_o(b + sgn_o * j * e_axis)), where
-// sgn_o is + for octants with bit `axis` set.  The first pass reads occupancy (0 for a
-// non-empty brick, cap otherwise).  Bytes are processed four at a time with the SIMD
-// byte min/max intrinsics; values never exceed the cap, which stands for "cap or more".
-__global__ void dir_pass_kernel(const uint64_t* __restrict__ occ, const uint64_t* __restrict__ in,
-                                uint64_t* __restrict__ out, Layout L, int axis, int x0, int y0, int z0, int nx,
-                                int ny, int nz, int first) {
-    uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (uint64_t)nx * ny * nz) return;
-    const int x = x0 + (int)(t % nx), y = y0 + (int)((t / nx) % ny), z = z0 + (int)(t / ((uint64_t)nx * ny));
-    const int c = axis == 0 ? x : (axis == 1 ? y : z);
-    const int D = axis == 1 ? L.BHp : L.BWp;
-    const int64_t stride = axis == 0 ? 1 : (axis == 1 ? (int64_t)L.BWp : (int64_t)L.BWp * L.BHp);
-    const int64_t self = (int64_t)brick_index(L, x, y, z);
-    const uint32_t capb = 0x01010101u * kDistCap;
-    uint64_t res[2];
-    for (int d = 0; d < 2; d++) {
-        const int sg = d == 0 ? 1 : -1;
-        uint32_t lo = capb, hi = capb;
-        for (int j = 0; j <= kDistCap; j++) {
-            const int q = c + sg * j;
-            if (q < 0 || q >= D) break;
-            const int64_t qi = self + sg * j * stride;
-            const uint64_t v = first ? (occ[qi] ? 0ull : ((uint64_t)capb << 32 | capb)) : in[qi];
-            const uint32_t jj = 0x01010101u * (uint32_t)j;
-            lo = __vminu4(lo, __vmaxu4((uint32_t)v, jj));
-            hi = __vminu4(hi, __vmaxu4((uint32_t)(v >> 32), jj));
-            if (__vcmpleu4(lo, jj) == 0xFFFFFFFFu && __vcmpleu4(hi, jj) == 0xFFFFFFFFu) break;  // nothing drops below j
-        }
-        res[d] = (uint64_t)hi << 32 | lo;
-    }
-    const uint64_t plus = axis == 0 ? 0xFF00FF00FF00FF00ull : (axis == 1 ? 0xFFFF0000FFFF0000ull : 0xFFFFFFFF00000000ull);
-    out[self] = (res[0] & plus) | (res[1] & ~plus);
-}
-
-// One thread per brick of the whole grid: bit x+4y+16z set when the voxel's word is not
-// -1, i.e. the cells where the shader's loop stops to hit (word >= 0) or to jump (a
-// depth-field word, fshader.glsl:114-121).  Voxels outside the world are clear.
-__global__ void stop_mask_kernel(const int32_t* __restrict__ words, uint64_t* __restrict__ stop, Layout L) {
-    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= L.n_bricks) return;
-    const int bx = (int)(t % L.BWp), by = (int)((t / L.BWp) % L.BHp), bz = (int)(t / ((uint64_t)L.BWp * L.BHp));
-    uint64_t m = 0;
-    for (int dz = 0; dz < 4; dz++) {
-        const int z = bz * 4 + dz;
-        if (z >= L.W) break;
-        for (int dy = 0; dy < 4; dy++) {
-            const int y = by * 4 + dy;
-            if (y >= L.H) break;
-            const int32_t* row = words + ((uint64_t)z * L.H + y) * L.W;
-            for (int dx = 0; dx < 4; dx++) {
-                const int x = bx * 4 + dx;
-                if (x < L.W && __ldg(row + x) != -1) m |= 1ull << (dx + 4 * dy + 16 * dz);
-            }
-        }
-    }
-    stop[t] = m;  // t is the linear brick slot bx + BWp*(by + BHp*bz)
-}
-
-static int dir_passes(vrt_world* w, const uint64_t* occ, uint8_t* dst8, int bx0, int by0, int bz0, int bx1, int by1,
-                      int bz1, cudaStream_t s) {
-    const Layout& L = w->L;
-    const int cap = kDistCap;
-    auto clampbox = [&](int& a0, int& a1, int lim) { a0 = std::max(a0, 0); a1 = std::min(a1, lim); };
-    int X0 = bx0, X1 = bx1, Y0 = by0, Y1 = by1, Z0 = bz0, Z1 = bz1;
-    clampbox(X0, X1, L.BWp); clampbox(Y0, Y1, L.BHp); clampbox(Z0, Z1, L.BWp);
-    if (X0 >= X1 || Y0 >= Y1 || Z0 >= Z1) return VRT_OK;
-    int ya0 = Y0 - cap, ya1 = Y1 + cap, za0 = Z0 - cap, za1 = Z1 + cap;
-    clampbox(ya0, ya1, L.BHp); clampbox(za0, za1, L.BWp);
-    uint64_t* ta = reinterpret_cast<uint64_t*>(w->d_tmp_a);
-    uint64_t* tb = reinterpret_cast<uint64_t*>(w->d_tmp_b);
-    uint64_t n = (uint64_t)(X1 - X0) * (ya1 - ya0) * (za1 - za0);
-    dir_pass_kernel<<<blocks_for(n, 256), 256, 0, s>>>(occ, nullptr, ta, L, 0, X0, ya0, za0, X1 - X0, ya1 - ya0,
-                                                       za1 - za0, 1);
-    n = (uint64_t)(X1 - X0) * (Y1 - Y0) * (za1 - za0);
-    dir_pass_kernel<<<blocks_for(n, 256), 256, 0, s>>>(occ, ta, tb, L, 1, X0, Y0, za0, X1 - X0, Y1 - Y0, za1 - za0,
-                                                       0);
-    n = (uint64_t)(X1 - X0) * (Y1 - Y0) * (Z1 - Z0);
-    dir_pass_kernel<<<blocks_for(n, 256), 256, 0, s>>>(occ, tb, reinterpret_cast<uint64_t*>(dst8), L, 2, X0, Y0, Z0,
-                                                       X1 - X0, Y1 - Y0, Z1 - Z0, 0);
-    VRT_CUDA(cudaGetLastError());
-    return VRT_OK;
-}
-
-static int region_passes(vrt_world* w, cudaStream_t s) {
-    const Layout& L = w->L;
-    const uint64_t n = (uint64_t)L.RWp * L.RHp * L.RWp;
-    cheb_pass_kernel<<<blocks_for(n, 256), 256, 0, s>>>(w->d_regions, nullptr, w->d_tmp_a, L, 0, 1);
-    cheb_pass_kernel<<<blocks_for(n, 256), 256, 0, s>>>(w->d_regions, w->d_tmp_a, w->d_tmp_b, L, 1, 0);
-    cheb_pass_kernel<<<blocks_for(n, 256), 256, 0, s>>>(w->d_regions, w->d_tmp_b, w->d_rdist, L, 2, 0);
-    VRT_CUDA(cudaGetLastError());
-    return VRT_OK;
-}
-
-// Directed distances of every brick within kDistCap bricks of the changed brick box, and
-// the distances of all regions (a few thousand to a few hundred thousand bytes).
-static int refresh_distances(vrt_world* w, int bx0, int by0, int bz0, int bx1, int by1, int bz1, cudaStream_t s) {
-    const int cap = kDistCap;
-    int st = dir_passes(w, w->d_bricks, w->d_bdir, bx0 - cap, by0 - cap, bz0 - cap, bx1 + cap, by1 + cap, bz1 + cap,
-                        s);
-    if (st) return st;
-    return region_passes(w, s);
-}
 
 int refresh_stop(vrt_world* w, cudaStream_t s) {
     if (!w->stop_stale) {
@@ -264,43 +47,48 @@ int refresh_stop(vrt_world* w, cudaStream_t s) {
     if (!w->d_stop) {
         cudaError_t e = cudaMalloc(&w->d_stop, L.n_bricks * 8);
         if (e == cudaSuccess) e = cudaMalloc(&w->d_sdir, L.n_bricks * 8);
+        if (e == cudaSuccess) e = cudaMalloc(&w->d_stop_regions, L.n_regions * 8);
+        if (e == cudaSuccess) e = cudaMemsetAsync(w->d_stop, 0, L.n_bricks * 8, s);
+        if (e == cudaSuccess) e = cudaMemsetAsync(w->d_stop_regions, 0, L.n_regions * 8, s);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&w->stop_ready, cudaEventDisableTiming);
         if (e != cudaSuccess) {
             cudaGetLastError();
             cudaFree(w->d_stop);
             cudaFree(w->d_sdir);
+            cudaFree(w->d_stop_regions);
             if (w->stop_ready) cudaEventDestroy(w->stop_ready);
             w->d_stop = nullptr;
             w->d_sdir = nullptr;
+            w->d_stop_regions = nullptr;
             w->stop_ready = nullptr;
             return set_error(VRT_ENOMEM, "stop masks: %s", cudaGetErrorString(e));
         }
-        w->device_bytes += L.n_bricks * 16;
+        w->device_bytes += L.n_bricks * 16 + L.n_regions * 8;
     }
-    stop_mask_kernel<<<blocks_for(L.n_bricks, 256), 256, 0, s>>>(w->d_words, w->d_stop, L);
-    VRT_CUDA(cudaGetLastError());
-    const int st = dir_passes(w, w->d_stop, w->d_sdir, 0, 0, 0, L.BWp, L.BHp, L.BWp, s);
+    const int st = refresh_stop_masks(w, s);
     if (st) return st;
     VRT_CUDA(cudaEventRecord(w->stop_ready, s));
     w->stop_stale = false;
     return VRT_OK;
 }
 
-// The words of the box [x0,x1)x[y0,y1)x[z0,z1) changed (clipped to the world): the stop
-// masks and, there, the z-major copy must follow.
-static void mark_words(vrt_world* w, int x0, int y0, int z0, int x1, int y1, int z1) {
-    x0 = std::max(x0, 0); y0 = std::max(y0, 0); z0 = std::max(z0, 0);
-    x1 = std::min(x1, w->L.W); y1 = std::min(y1, w->L.H); z1 = std::min(z1, w->L.W);
-    if (x0 >= x1 || y0 >= y1 || z0 >= z1) return;
+void mark_words(vrt_world* w, const int64_t v[6]) {
+    const int dim[3] = {w->L.W, w->L.H, w->L.W};
+    int lo[3], hi[3];
+    for (int a = 0; a < 3; a++) {
+        const int64_t l = std::max<int64_t>(v[a], 0), h = std::min<int64_t>(v[3 + a], dim[a]);
+        if (l >= h) return;
+        lo[a] = (int)l;
+        hi[a] = (int)h;
+    }
     w->stop_stale = true;
     if (!w->d_words_z) return;
     int* b = w->z_dirty;
-    if (b[0] >= b[3]) {
-        b[0] = x0; b[1] = y0; b[2] = z0; b[3] = x1; b[4] = y1; b[5] = z1;
-        return;
+    const bool empty = b[0] >= b[3];
+    for (int a = 0; a < 3; a++) {
+        b[a] = empty ? lo[a] : std::min(b[a], lo[a]);
+        b[3 + a] = empty ? hi[a] : std::max(b[3 + a], hi[a]);
     }
-    b[0] = std::min(b[0], x0); b[1] = std::min(b[1], y0); b[2] = std::min(b[2], z0);
-    b[3] = std::max(b[3], x1); b[4] = std::max(b[4], y1); b[5] = std::max(b[5], z1);
 }
 
 // Whole-world copy with x and z swapped, through 32x32 tiles of the (x, z) plane of each y
@@ -363,73 +151,37 @@ int refresh_words_z(vrt_world* w, cudaStream_t s) {
     return VRT_OK;
 }
 
-int refresh_masks_box(vrt_world* w, int x0, int y0, int z0, int x1, int y1, int z1, cudaStream_t s) {
-    const Layout& L = w->L;
-    x0 = std::max(x0, 0); y0 = std::max(y0, 0); z0 = std::max(z0, 0);
-    x1 = std::min(x1, L.W); y1 = std::min(y1, L.H); z1 = std::min(z1, L.W);
-    if (x0 >= x1 || y0 >= y1 || z0 >= z1) return VRT_OK;
-    mark_words(w, x0, y0, z0, x1, y1, z1);
-    int bx0 = x0 >> 2, by0 = y0 >> 2, bz0 = z0 >> 2;
-    int bx1 = (x1 + 3) >> 2, by1 = (y1 + 3) >> 2, bz1 = (z1 + 3) >> 2;
-    uint64_t nb = (uint64_t)(bx1 - bx0) * (by1 - by0) * (bz1 - bz0);
-    // a refresh of the whole world recomputes the solid bounding box; a partial one only grows it
-    if (x0 == 0 && y0 == 0 && z0 == 0 && x1 == L.W && y1 == L.H && z1 == L.W) reset_aabb_kernel<<<1, 32, 0, s>>>(w->d_aabb);
-    brick_mask_kernel<<<blocks_for(nb, 256), 256, 0, s>>>(w->d_words, w->d_bricks, w->d_flag, w->d_aabb, L, bx0, by0,
-                                                           bz0, bx1 - bx0, by1 - by0, bz1 - bz0);
-    int rx0 = bx0 >> 2, ry0 = by0 >> 2, rz0 = bz0 >> 2;
-    int rx1 = (bx1 + 3) >> 2, ry1 = (by1 + 3) >> 2, rz1 = (bz1 + 3) >> 2;
-    uint64_t nr = (uint64_t)(rx1 - rx0) * (ry1 - ry0) * (rz1 - rz0);
-    parent_mask_kernel<<<blocks_for(nr, 256), 256, 0, s>>>(w->d_bricks, w->d_regions, rx0, ry0, rz0, rx1 - rx0,
-                                                           ry1 - ry0, rz1 - rz0, L, 1);
-    int sx0 = rx0 >> 2, sy0 = ry0 >> 2, sz0 = rz0 >> 2;
-    int sx1 = (rx1 + 3) >> 2, sy1 = (ry1 + 3) >> 2, sz1 = (rz1 + 3) >> 2;
-    uint64_t ns = (uint64_t)(sx1 - sx0) * (sy1 - sy0) * (sz1 - sz0);
-    parent_mask_kernel<<<blocks_for(ns, 256), 256, 0, s>>>(w->d_regions, w->d_supers, sx0, sy0, sz0, sx1 - sx0,
-                                                           sy1 - sy0, sz1 - sz0, L, 2);
-    VRT_CUDA(cudaGetLastError());
-    return refresh_distances(w, bx0, by0, bz0, bx1, by1, bz1, s);
+// The box of the words [first, first + count): planes, rows or part of a row.
+static void words_box(const Layout& L, uint64_t first, uint64_t count, int64_t v[6]) {
+    const uint64_t last = first + count - 1, plane = (uint64_t)L.W * L.H;
+    const int64_t z0 = first / plane, z1 = last / plane;
+    const int64_t y0 = first % plane / L.W, y1 = last % plane / L.W;
+    const int64_t x0 = first % L.W, x1 = last % L.W;
+    const bool rows = z0 != z1, cells = !rows && y0 == y1;
+    v[0] = cells ? x0 : 0;
+    v[1] = rows ? 0 : y0;
+    v[2] = z0;
+    v[3] = cells ? x1 + 1 : L.W;
+    v[4] = rows ? L.H : y1 + 1;
+    v[5] = z1 + 1;
 }
 
-int refresh_masks(vrt_world* w, uint64_t first, uint64_t count, cudaStream_t s) {
-    if (count == 0) return VRT_OK;
-    const Layout& L = w->L;
-    uint64_t last = first + count - 1;
-    uint64_t plane = (uint64_t)L.W * L.H;
-    int z0 = (int)(first / plane), z1 = (int)(last / plane);
-    if (z0 != z1) return refresh_masks_box(w, 0, 0, z0, L.W, L.H, z1 + 1, s);
-    int y0 = (int)((first % plane) / L.W), y1 = (int)((last % plane) / L.W);
-    if (y0 != y1) return refresh_masks_box(w, 0, y0, z0, L.W, y1 + 1, z0 + 1, s);
-    int x0 = (int)(first % L.W), x1 = (int)(last % L.W);
-    return refresh_masks_box(w, x0, y0, z0, x1 + 1, y0 + 1, z0 + 1, s);
+static WordChange whole_world(const Layout& L) {
+    WordChange c{};
+    c.op = kReadWords;
+    c.box[3] = L.W; c.box[4] = L.H; c.box[5] = L.W;
+    return c;
 }
 
-// Copy the device solid bounding box to the host copy the render launches pass on
-// (synchronises the stream).
-static int read_aabb(vrt_world* w, cudaStream_t s) {
-    int bb[8];
-    VRT_CUDA(cudaMemcpyAsync(bb, w->d_aabb, sizeof(bb), cudaMemcpyDeviceToHost, s));
+// Copy the solid bounding box and the depth-field flag to the host copies the render
+// launches go by (synchronises the stream).
+static int read_state(vrt_world* w, int& flag, cudaStream_t s) {
+    int st[8];
+    VRT_CUDA(cudaMemcpyAsync(st, w->d_aabb, sizeof(st), cudaMemcpyDeviceToHost, s));
     VRT_CUDA(cudaStreamSynchronize(s));
-    for (int i = 0; i < 6; i++) w->h_aabb[i] = bb[i];
+    for (int i = 0; i < 6; i++) w->h_aabb[i] = st[i];
+    flag = st[6];
     return VRT_OK;
-}
-
-// ------------------------------------------------------------------ edits
-
-// removeSphere's first loop (level.cpp:31-42): voxels with offsets in [-r,r)^3,
-// x*x+y*y+z*z < r*r and inside the world become air.
-__global__ void remove_sphere_kernel(int32_t* __restrict__ words, Layout L, int cx, int cy, int cz, int r) {
-    int n = 2 * r;
-    uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (uint64_t)n * n * n) return;
-    int x = (int)(t % n) - r, y = (int)((t / n) % n) - r, z = (int)(t / ((uint64_t)n * n)) - r;
-    int ax = x + cx, ay = y + cy, az = z + cz;
-    if (ax < L.W && ay < L.H && az < L.W && ax >= 0 && ay >= 0 && az >= 0 && x * x + y * y + z * z < r * r)
-        words[(uint64_t)ax + (uint64_t)L.W * ay + (uint64_t)L.W * L.H * az] = -1;
-}
-
-__global__ void place_voxel_kernel(int32_t* words, Layout L, int x, int y, int z, int32_t v) {
-    if (x >= 0 && y >= 0 && z >= 0 && x < L.W && y < L.H && z < L.W)
-        words[(uint64_t)x + (uint64_t)L.W * y + (uint64_t)L.W * L.H * z] = v;
 }
 
 __global__ void probe_kernel(const int32_t* __restrict__ words, Layout L, const int32_t* __restrict__ xyz, int n,
@@ -523,8 +275,10 @@ int vrt_world_create(int32_t width, int32_t height, vrt_world** out) {
     vrt_world* w = new vrt_world();
     w->L = L;
     cudaGetDevice(&w->device);
-    uint64_t bytes = w->L.n_words * 4 + (w->L.n_bricks + w->L.n_regions + w->L.n_supers) * 8 + 24 * w->L.n_bricks +
-                     (uint64_t)w->L.RWp * w->L.RHp * w->L.RWp + 256;
+    cudaDeviceGetAttribute(&w->num_sms, cudaDevAttrMultiProcessorCount, w->device);
+    const uint64_t box_bytes = (uint64_t)w->num_sms * kBrickCtasPerSm * 8 * sizeof(int);
+    uint64_t bytes = w->L.n_words * 4 + (w->L.n_bricks + w->L.n_regions + w->L.n_supers) * 8 + 8 * w->L.n_bricks +
+                     (uint64_t)w->L.RWp * w->L.RHp * w->L.RWp + box_bytes + 256;
     cudaError_t e = cudaMalloc(&w->d_words, w->L.n_words * 4);
     if (e == cudaSuccess) e = cudaMalloc(&w->d_bricks, w->L.n_bricks * 8);
     if (e == cudaSuccess) e = cudaMalloc(&w->d_regions, w->L.n_regions * 8);
@@ -532,9 +286,7 @@ int vrt_world_create(int32_t width, int32_t height, vrt_world** out) {
     const uint64_t rbytes = ((uint64_t)w->L.RWp * w->L.RHp * w->L.RWp + 15) & ~(uint64_t)15;  // staged as uint4
     if (e == cudaSuccess) e = cudaMalloc(&w->d_rdist, rbytes);
     if (e == cudaSuccess) e = cudaMalloc(&w->d_bdir, w->L.n_bricks * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&w->d_tmp_a, w->L.n_bricks * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&w->d_tmp_b, w->L.n_bricks * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&w->d_flag, sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc(&w->d_boxes, box_bytes);
     if (e == cudaSuccess) e = cudaMalloc(&w->d_aabb, 8 * sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(w->d_words, 0xFF, w->L.n_words * 4);  // air = -1 (render.cpp:349-351)
     if (e == cudaSuccess) e = cudaMemset(w->d_bricks, 0, w->L.n_bricks * 8);
@@ -542,8 +294,7 @@ int vrt_world_create(int32_t width, int32_t height, vrt_world** out) {
     if (e == cudaSuccess) e = cudaMemset(w->d_supers, 0, w->L.n_supers * 8);
     if (e == cudaSuccess) e = cudaMemset(w->d_bdir, kDistCap, w->L.n_bricks * 8);  // an all-air world
     if (e == cudaSuccess) e = cudaMemset(w->d_rdist, kDistCap, rbytes);
-    if (e == cudaSuccess) e = cudaMemset(w->d_flag, 0, sizeof(int));
-    if (e == cudaSuccess) {  // an all-air world: empty box (min > max)
+    if (e == cudaSuccess) {  // an all-air world: empty box (min > max), no depth-field word
         const int empty[8] = {INT_MAX, INT_MAX, INT_MAX, INT_MIN, INT_MIN, INT_MIN, 0, 0};
         e = cudaMemcpy(w->d_aabb, empty, sizeof(empty), cudaMemcpyHostToDevice);
         for (int i = 0; i < 6; i++) w->h_aabb[i] = empty[i];
@@ -573,9 +324,8 @@ int vrt_world_destroy(vrt_world* w) {
     if (w->stop_ready) cudaEventDestroy(w->stop_ready);
     cudaFree(w->d_words_z);
     if (w->z_ready) cudaEventDestroy(w->z_ready);
-    cudaFree(w->d_tmp_a);
-    cudaFree(w->d_tmp_b);
-    cudaFree(w->d_flag);
+    cudaFree(w->d_stop_regions);
+    cudaFree(w->d_boxes);
     cudaFree(w->d_aabb);
     delete w;
     return VRT_OK;
@@ -601,15 +351,25 @@ static int upload_common(vrt_world* w, const int32_t* src, uint64_t first, uint6
         return set_error(VRT_ERANGE, "words [%llu, %llu) beyond the world's %llu", (unsigned long long)first,
                          (unsigned long long)(first + count), (unsigned long long)w->L.n_words);
     if (count == 0) return VRT_OK;
-    VRT_CUDA(cudaMemcpyAsync(w->d_words + first, src, count * 4, kind, S(stream)));
-    int st = refresh_masks(w, first, count, S(stream));
+    WordChange c{};
+    words_box(w->L, first, count, c.box);
+    if (kind == cudaMemcpyDeviceToDevice) {  // copied by the pass that makes the masks
+        c.op = kCopyWords;
+        c.src = src;
+        c.first = first;
+        c.count = count;
+    } else {
+        c.op = kReadWords;
+        VRT_CUDA(cudaMemcpyAsync(w->d_words + first, src, count * 4, kind, S(stream)));
+    }
+    int st = change_words(w, c, S(stream));
     if (st) return st;
     // the kernel choice depends on the depth-field flag: read it back now
     int flag = 0;
-    VRT_CUDA(cudaMemcpyAsync(&flag, w->d_flag, sizeof(int), cudaMemcpyDeviceToHost, S(stream)));
-    VRT_CUDA(cudaStreamSynchronize(S(stream)));
+    st = read_state(w, flag, S(stream));
+    if (st) return st;
     w->has_depth_field |= flag;
-    return read_aabb(w, S(stream));
+    return VRT_OK;
 }
 
 int vrt_world_upload(vrt_world* w, const int32_t* host_words, uint64_t first, uint64_t count, void* stream) {
@@ -653,18 +413,19 @@ int vrt_world_download_distances(const vrt_world* w, uint8_t* brick_dir, uint8_t
     return VRT_OK;
 }
 
-// The flag is raised by the brick kernel whenever it sees a word < -1 and never lowered
-// by it; a full-world refresh after clearing gives the exact current state.
+// The brick pass raises the flag whenever it sees a word < -1 and never lowers it; a pass
+// over the whole world that starts it from 0 gives the exact current state.
 int vrt_world_sync_flags(vrt_world* w, void* stream) {
     if (!w) return set_error(VRT_EINVAL, "NULL world");
-    VRT_CUDA(cudaMemsetAsync(w->d_flag, 0, sizeof(int), S(stream)));
-    int st = refresh_masks_box(w, 0, 0, 0, w->L.W, w->L.H, w->L.W, S(stream));
+    WordChange c = whole_world(w->L);
+    c.reset_flag = true;
+    int st = change_words(w, c, S(stream));
     if (st) return st;
     int flag = 0;
-    VRT_CUDA(cudaMemcpyAsync(&flag, w->d_flag, sizeof(int), cudaMemcpyDeviceToHost, S(stream)));
-    VRT_CUDA(cudaStreamSynchronize(S(stream)));
+    st = read_state(w, flag, S(stream));
+    if (st) return st;
     w->has_depth_field = flag;
-    return read_aabb(w, S(stream));
+    return VRT_OK;
 }
 
 int vrt_world_probe(const vrt_world* w, const int32_t* d_xyz, int32_t n, int32_t* d_words, void* stream) {
@@ -726,8 +487,13 @@ int vrt_world_load(const char* path, vrt_world** out, void* stream) {
 int vrt_place_voxel(vrt_world* w, int32_t x, int32_t y, int32_t z, int32_t word, void* stream) {
     if (!w) return set_error(VRT_EINVAL, "NULL world");
     if (x < 0 || y < 0 || z < 0 || x >= w->L.W || y >= w->L.H || z >= w->L.W) return VRT_OK;  // render.cpp:259
-    place_voxel_kernel<<<1, 1, 0, S(stream)>>>(w->d_words, w->L, x, y, z, word);
-    VRT_CUDA(cudaGetLastError());
+    WordChange ch{};
+    ch.op = kPlaceVoxel;
+    ch.x = x; ch.y = y; ch.z = z; ch.word = word;
+    const int64_t box[6] = {x, y, z, x + 1, y + 1, z + 1};
+    std::memcpy(ch.box, box, sizeof(box));
+    const int st = change_words(w, ch, S(stream));
+    if (st) return st;
     if (word < -1) w->has_depth_field = 1;
     if (word >= 0) {  // grow the host copy of the solid box by the voxel's brick
         const int c[3] = {x & ~3, y & ~3, z & ~3};
@@ -736,39 +502,46 @@ int vrt_place_voxel(vrt_world* w, int32_t x, int32_t y, int32_t z, int32_t word,
             w->h_aabb[3 + i] = std::max(w->h_aabb[3 + i], c[i] + 3);
         }
     }
-    return refresh_masks_box(w, x, y, z, x + 1, y + 1, z + 1, S(stream));
+    return VRT_OK;
 }
 
 int vrt_fix_depth_field_box(vrt_world* w, int32_t x0, int32_t y0, int32_t z0, int32_t x1, int32_t y1, int32_t z1,
                             void* stream) {
     if (!w) return set_error(VRT_EINVAL, "NULL world");
-    x0 = std::max(x0, 0); y0 = std::max(y0, 0); z0 = std::max(z0, 0);
-    x1 = std::min(x1, w->L.W); y1 = std::min(y1, w->L.H); z1 = std::min(z1, w->L.W);
-    if (x0 >= x1 || y0 >= y1 || z0 >= z1) return VRT_OK;
     // the depth field changes air words only, so the occupancy structures stay as they are
-    mark_words(w, x0, y0, z0, x1, y1, z1);
+    WordChange c{};
+    const int64_t box[6] = {x0, y0, z0, x1, y1, z1};
+    std::memcpy(c.fix_box, box, sizeof(box));
+    c.fix = true;
+    const int dim[3] = {w->L.W, w->L.H, w->L.W};
+    for (int a = 0; a < 3; a++)
+        if (std::max<int64_t>(box[a], 0) >= std::min<int64_t>(box[3 + a], dim[a])) return VRT_OK;
     w->has_depth_field = 1;
-    return launch_fix_depth_field(w, x0, y0, z0, x1, y1, z1, 0, 0, 0, 0, S(stream));
+    return change_words(w, c, S(stream));
 }
 
 int vrt_remove_sphere(vrt_world* w, int32_t cx, int32_t cy, int32_t cz, int32_t radius, int32_t refresh_depth_field,
                       void* stream) {
     if (!w) return set_error(VRT_EINVAL, "NULL world");
     if (radius < 0 || radius > 1024) return set_error(VRT_ERANGE, "radius %d outside [0, 1024]", radius);
-    if (radius > 0) {
-        uint64_t n = (uint64_t)(2 * radius) * (2 * radius) * (2 * radius);
-        remove_sphere_kernel<<<blocks_for(n, 256), 256, 0, S(stream)>>>(w->d_words, w->L, cx, cy, cz, radius);
-        VRT_CUDA(cudaGetLastError());
-        // the masks first: the depth field reads solidity from them
-        int st = refresh_masks_box(w, cx - radius, cy - radius, cz - radius, cx + radius, cy + radius, cz + radius,
-                                   S(stream));
-        if (st) return st;
+    const int64_t at[3] = {cx, cy, cz};
+    WordChange c{};
+    c.op = kRemoveSphere;
+    c.x = cx; c.y = cy; c.z = cz; c.r = radius;
+    for (int a = 0; a < 3; a++) {
+        c.box[a] = at[a] - radius;
+        c.box[3 + a] = at[a] + radius;
     }
-    if (!refresh_depth_field) return VRT_OK;
-    const int r2 = radius + (7 >> 1);  // DEPTH_FIELD_RADIUS >> 1, level.cpp:43
-    mark_words(w, cx - r2, cy - r2, cz - r2, cx + r2, cy + r2, cz + r2);
-    w->has_depth_field = 1;
-    return launch_fix_depth_field(w, cx - r2, cy - r2, cz - r2, cx + r2, cy + r2, cz + r2, cx, cy, cz, r2, S(stream));
+    if (refresh_depth_field) {
+        c.fix = true;
+        c.fix_r = radius + (7 >> 1);  // DEPTH_FIELD_RADIUS >> 1, level.cpp:43
+        for (int a = 0; a < 3; a++) {
+            c.fix_box[a] = at[a] - c.fix_r;
+            c.fix_box[3 + a] = at[a] + c.fix_r;
+        }
+        w->has_depth_field = 1;
+    }
+    return change_words(w, c, S(stream));
 }
 
 int vrt_world_init_reference(vrt_world* w, void* stream) {
@@ -786,11 +559,13 @@ int vrt_world_init_reference(vrt_world* w, void* stream) {
         init_reference_trees_kernel<<<grid, 256, 0, S(stream)>>>(w->d_words, L, trees_x);
         VRT_CUDA(cudaGetLastError());
     }
-    VRT_CUDA(cudaMemsetAsync(w->d_flag, 0, sizeof(int), S(stream)));
+    WordChange c = whole_world(L);
+    c.reset_flag = true;
     w->has_depth_field = 0;
-    int st = refresh_masks_box(w, 0, 0, 0, L.W, L.H, L.W, S(stream));
+    int flag = 0;
+    int st = change_words(w, c, S(stream));
     if (st) return st;
-    return read_aabb(w, S(stream));
+    return read_state(w, flag, S(stream));
 }
 
 }  // extern "C"

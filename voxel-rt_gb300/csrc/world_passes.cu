@@ -1,13 +1,25 @@
-// Bit-parallel passes over the occupancy masks: the depth field (fixDepthField,
-// render.cpp:226-253).
+// The passes behind every change of a world's words, in two launches:
+//   brick_pass_kernel  changes the words (removeSphere, placeVoxel, an upload from device
+//                      memory, or nothing), and rebuilds the brick masks of the box in the same
+//                      pass, with the region and super masks' bits, the solid bounding box
+//                      and the depth-field flag;
+//   node_pass_kernel   everything that follows from them, as independent tiles of one launch:
+//                      the directed brick distances, the region distances and the depth
+//                      field (fixDepthField, render.cpp:226-253).
 //
-// A row of 32 voxels along x is one 32-bit word here.  The masks already hold a bit per
-// voxel, 4 bits of a row in each brick, so a tile of rows with its halo is put together in
-// shared memory from the few KB of masks it spans, and the neighbourhood work of 32
-// voxels is done by one instruction.
+// The node pass is bit-parallel: a row of 32 nodes along x is one 32-bit word.  The masks
+// already hold a bit per voxel (brick masks) and per brick (region masks), 4 bits of a row in
+// each 64-bit mask, so a tile of rows with its halo is put together in shared memory from the
+// few KB of masks that it spans, and the neighbourhood work of 32 nodes is done by one
+// instruction.
+//
+// Both are latency chains for an edit (4.5 and 8.6 us, a few dozen CTAs), where ten launches
+// of a few microseconds each took 88 us for removeSphere(8) in the 512 x 256 x 512 world, 12.6
+// now, host included.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <utility>
@@ -15,6 +27,49 @@
 #include "vrt_internal.h"
 
 namespace vrt {
+
+struct BrickPass {
+    int32_t* words;
+    const int32_t* src;          // kCopyWords: words [first, first + count) come from here
+    uint64_t first, count;
+    uint64_t* bricks;
+    uint64_t* regions;
+    uint64_t* supers;            // may be NULL (stop masks)
+    int* boxes;                  // one record per CTA: solid box (min x,y,z, max x,y,z), depth flag, 0
+    Layout L;
+    int bx0, by0, bz0, bx1;      // the bricks' box (its ends in y and z follow from ny and tasks)
+    int g0;                      // first group of 8 bricks along x
+    unsigned ng, ny, tasks;      // groups along x, bricks along y, groups in all
+    int x, y, z, r;              // kRemoveSphere: centre and radius; kPlaceVoxel: the voxel
+    int32_t word;                // kPlaceVoxel
+};
+
+constexpr int kFixLevels = 36;
+
+struct FixPass {
+    int32_t* words;
+    const uint64_t* bricks;
+    Layout L;
+    int x0, y0, z0, x1, y1, z1;  // the voxels to refresh, within the world
+    int cx, cy, cz, r2;          // r2 > 0: of those, the ones inside this sphere
+    int tx0, ty0, tz0, ntx, nty; // the tiles that cover the box
+    int32_t word[kFixLevels + 1];
+};
+
+struct NodePass {
+    const uint64_t* regions;
+    uint32_t* bdir;              // directed distances, 4 octants to a word (the -z ones first)
+    const uint64_t* supers;
+    uint8_t* rdist;
+    int* aabb;                   // solid box, then the depth-field flag
+    const int* boxes;
+    Layout L;
+    int n_fix, n_dir, n_reg, n_boxes;            // tiles of each kind; records to merge
+    int dx0, dy0, dz0, ndx, ndy;                 // distance tiles of 32 x 8 x 8 bricks
+    int rx0, ry0, rz0, nrx, nry;                 // and of 32 x 8 x 8 regions
+    int reset_box, reset_flag;
+    FixPass fix;
+};
 
 // ------------------------------------------------------------------ depth field
 //
@@ -41,7 +96,6 @@ constexpr int kFixPitch = 48;
 constexpr int kFixPlane = kFixRows * kFixPitch;
 constexpr int kFixK = 6;               // D_1 .. D_6 (|x| = 7 alone gives s = 36)
 constexpr int kFixNodes = 12 * 8 * 8;  // bricks spanned: 8 + 2 x 2 in x, 4 + 2 x 2 in y and z
-constexpr int kFixLevels = 36;
 
 struct FixSmem {
     uint64_t nodes[kFixNodes];
@@ -104,16 +158,6 @@ __device__ __forceinline__ void fix_levels(const uint32_t* d, uint32_t& found, u
         fix_levels<S + 1>(d, found, bit);
     }
 }
-
-struct FixPass {
-    int32_t* words;
-    const uint64_t* bricks;
-    Layout L;
-    int x0, y0, z0, x1, y1, z1;  // the voxels to refresh, within the world
-    int cx, cy, cz, r2;          // r2 > 0: of those, the ones inside this sphere
-    int tx0, ty0, tz0, ntx, nty; // the tiles that cover the box
-    int32_t word[kFixLevels + 1];
-};
 
 // One 32 x 16 x 16 tile by 256 threads, one row each.  Only the air voxels of P.box (and of
 // the sphere, if there is one) are written; only solidity is read, which no thread changes.
@@ -199,20 +243,528 @@ __device__ void fix_tile(const FixPass& P, int tile, FixSmem& s) {
     }
 }
 
-__global__ void __launch_bounds__(256) fix_depth_field_kernel(const __grid_constant__ FixPass P) {
-    __shared__ FixSmem s;
-    fix_tile(P, blockIdx.x, s);
+// ------------------------------------------------------------------ directed brick distances
+//
+// D(b) = the largest r <= 15 for which the cube of r^3 bricks from b into the octant is empty.
+// With E_r = "that cube is empty" as a bit per brick, E_1 is the complement of the occupancy,
+// and for a + c <= 2a the cube of side a + c is the union of the cubes of side a at the eight
+// corners {0, c}^3.  So E_2, E_4 and E_8 follow from each other, every other E_r is an AND of
+// eight shifted copies of one of them, and D is the number of r with E_r set.  The AND over x
+// is one shift of the row word, over y and z it is four rows.  (Three passes, one per axis, of
+// up to 16 byte minima per brick and octant took 92 us for the 512 x 96 x 512 level, and
+// three more for the regions 19 us; this whole launch takes 19 us, bound by its instructions.)
+//
+// One tile: 32 x 8 x 8 bricks and the four octants of one z direction.  Rows are held as
+// 64-bit windows from 16 bricks before the tile, so no carry between words is needed: a
+// window end spoils at most 14 bits, which end before the tile's own.  Smaller tiles in y and
+// z would read more halo (14 rows each), larger ones leave an edit's few tiles too long.
+
+constexpr int kDirRows = 22;  // 8 + 14 rows along the octant's y and z
+constexpr int kDirYY = 36;    // both y directions
+constexpr int kDirNodes = 16 * 10 * 6;
+
+struct alignas(16) DirSmem {
+    uint64_t nodes[kDirNodes];  // region masks; later the distance bit planes
+    uint64_t e1[kDirRows * kDirYY];
+    ulonglong2 e2[2][21 * 21];  // [y direction]: .x toward +x, .y toward -x; later the output
+    ulonglong2 e4[2][19 * 19];
+    ulonglong2 e8[2][15 * 15];
+};
+
+// The 64-bit row window at row (py, pz) of 16 x 10 x n masks held in shared memory.
+__device__ __forceinline__ uint64_t row_window(const uint32_t* n32, int py, int pz) {
+    const uint32_t* n = n32 + 2 * ((py >> 2) * 16 + (pz >> 2) * 160) + ((pz & 3) >> 1);
+    const int shift = 4 * (py & 3) + 16 * (pz & 1);
+    uint64_t w = 0;
+#pragma unroll
+    for (int j = 0; j < 16; j++) w |= (uint64_t)(n[2 * j] >> shift & 15) << (4 * j);
+    return w;
 }
 
-int launch_fix_depth_field(vrt_world* w, int x0, int y0, int z0, int x1, int y1, int z1, int cx, int cy, int cz,
-                           int r2, cudaStream_t s) {
-    FixPass P{};
+__device__ __forceinline__ ulonglong2 and4(const ulonglong2* e, int pitch, int o) {
+    const ulonglong2 a = e[0], b = e[o], c = e[o * pitch], d = e[o * pitch + o];
+    return make_ulonglong2(a.x & b.x & c.x & d.x, a.y & b.y & c.y & d.y);
+}
+
+// E_(a+o) of one row and x direction (word 0: +x, word 1: -x) from E_a of side-a cubes.
+template <int PITCH, int O>
+__device__ __forceinline__ uint32_t corners(const ulonglong2* e, int word, bool plus) {
+    const uint64_t* q = reinterpret_cast<const uint64_t*>(e) + word;
+    const uint64_t v = q[0] & q[2 * O] & q[2 * O * PITCH] & q[2 * (O * PITCH + O)];
+    return (uint32_t)((v & (plus ? v >> O : v << O)) >> 16);
+}
+
+// bit i of x -> bit 0 of byte i, for the low 4 bits
+__device__ __forceinline__ uint32_t spread4(uint32_t x) { return (x * 0x00204081u) & 0x01010101u; }
+
+// 4 nodes' values, one per byte, from the bit planes at bit position sh
+__device__ __forceinline__ uint32_t plane_bytes(uint4 p, int sh) {
+    return spread4(p.x >> sh & 15) | spread4(p.y >> sh & 15) << 1 | spread4(p.z >> sh & 15) << 2 |
+           spread4(p.w >> sh & 15) << 3;
+}
+
+// r is the value of the nodes in `now`
+__device__ __forceinline__ void add_planes(uint4& p, int r, uint32_t now) {
+    if (r & 1) p.x |= now;
+    if (r & 2) p.y |= now;
+    if (r & 4) p.z |= now;
+    if (r & 8) p.w |= now;
+}
+
+__device__ void dir_tile(const NodePass& P, int tile, DirSmem& s) {
+    const Layout& L = P.L;
+    const int zs = tile & 1;  // 1: toward +z
+    tile >>= 1;
+    const int x0 = (P.dx0 + tile % P.ndx) * 32, y0 = (P.dy0 + tile / P.ndx % P.ndy) * 8;
+    const int z0 = (P.dz0 + tile / (P.ndx * P.ndy)) * 8;
+    const int t = threadIdx.x;
+
+    // the regions the tile and its halo span; beyond the grid everything is empty
+    const int rx0 = x0 / 4 - 4, ry0 = y0 / 4 - 4, rz0 = zs ? z0 / 4 : z0 / 4 - 4;
+    for (int i = t; i < kDirNodes; i += 256) {
+        const int rx = rx0 + (i & 15), ry = ry0 + (i >> 4) % 10, rz = rz0 + i / 160;
+        uint64_t m = 0;
+        if (rx >= 0 && ry >= 0 && rz >= 0 && rx < L.RWp && ry < L.RHp && rz < L.RWp)
+            m = P.regions[region_index(L, rx, ry, rz)];
+        s.nodes[i] = m;
+    }
+    __syncthreads();
+    // E_1: rows yy = y - (y0 - 14), and lz along the z direction (0..7 the tile's own)
+    const uint32_t* n32 = reinterpret_cast<const uint32_t*>(s.nodes);
+    for (int i = t; i < kDirRows * kDirYY; i += 256) {
+        const int lz = i / kDirYY;
+        s.e1[i] = ~row_window(n32, i % kDirYY + 2, zs ? lz : 23 - lz);
+    }
+    __syncthreads();
+    for (int i = t; i < 2 * 21 * 21; i += 256) {
+        const int ys = i / 441, r = i % 441, ly = r % 21, lz = r / 21;
+        const int yy = ys ? 14 + ly : 21 - ly, step = ys ? 1 : -1;
+        const uint64_t* e = s.e1 + lz * kDirYY + yy;
+        const uint64_t v = e[0] & e[step] & e[kDirYY] & e[kDirYY + step];
+        s.e2[ys][r] = make_ulonglong2(v & v >> 1, v & v << 1);
+    }
+    __syncthreads();
+    for (int i = t; i < 2 * 19 * 19; i += 256) {
+        const int ys = i / 361, r = i % 361;
+        const ulonglong2 v = and4(&s.e2[ys][r % 19 + r / 19 * 21], 21, 2);
+        s.e4[ys][r] = make_ulonglong2(v.x & v.x >> 2, v.y & v.y << 2);
+    }
+    __syncthreads();
+    for (int i = t; i < 2 * 15 * 15; i += 256) {
+        const int ys = i / 225, r = i % 225;
+        const ulonglong2 v = and4(&s.e4[ys][r % 15 + r / 15 * 19], 19, 4);
+        s.e8[ys][r] = make_ulonglong2(v.x & v.x >> 4, v.y & v.y << 4);
+    }
+    __syncthreads();
+    // One of the tile's 64 rows, and one of the four octants, per thread
+    const int ya = t & 7, za = t >> 3 & 7, xs = t >> 6 & 1, ys = t >> 7;
+    uint4 p = make_uint4(0, 0, 0, 0);
+    {
+        const int ly = ys ? ya : 7 - ya, lz = zs ? za : 7 - za;
+        const ulonglong2* e2 = &s.e2[ys][lz * 21 + ly];
+        const ulonglong2* e4 = &s.e4[ys][lz * 19 + ly];
+        const ulonglong2* e8 = &s.e8[ys][lz * 15 + ly];
+        const int word = xs ? 0 : 1;
+        const bool plus = xs != 0;
+        uint32_t cur = 0xffffffffu;
+        auto level = [&](int r, uint32_t e) {  // E_r: the nodes that end here have r - 1
+            add_planes(p, r - 1, cur & ~e);
+            cur = e;
+        };
+        level(1, (uint32_t)(s.e1[lz * kDirYY + (ys ? 14 + ly : 21 - ly)] >> 16));
+        level(2, corners<21, 0>(e2, word, plus));
+        level(3, corners<21, 1>(e2, word, plus));
+        level(4, corners<19, 0>(e4, word, plus));
+        level(5, corners<19, 1>(e4, word, plus));
+        level(6, corners<19, 2>(e4, word, plus));
+        level(7, corners<19, 3>(e4, word, plus));
+        level(8, corners<15, 0>(e8, word, plus));
+        level(9, corners<15, 1>(e8, word, plus));
+        level(10, corners<15, 2>(e8, word, plus));
+        level(11, corners<15, 3>(e8, word, plus));
+        level(12, corners<15, 4>(e8, word, plus));
+        level(13, corners<15, 5>(e8, word, plus));
+        level(14, corners<15, 6>(e8, word, plus));
+        level(15, corners<15, 7>(e8, word, plus));
+        add_planes(p, kDistCap, cur);
+    }
+    uint4* planes = reinterpret_cast<uint4*>(s.nodes);  // [octant of this z direction][row]
+    planes[(xs + 2 * ys) * 64 + (t & 63)] = p;
+    __syncthreads();
+    // planes -> one byte per octant: 8 bricks of one row per thread, four octants to a word
+    uint32_t* out = reinterpret_cast<uint32_t*>(s.e2);  // 64 rows x 32 bricks
+    {
+        const int row = t >> 2, seg = t & 3;
+#pragma unroll
+        for (int g = 0; g < 2; g++) {
+            const int sh = 8 * seg + 4 * g;
+            const uint32_t a0 = plane_bytes(planes[row], sh), a1 = plane_bytes(planes[64 + row], sh);
+            const uint32_t a2 = plane_bytes(planes[128 + row], sh), a3 = plane_bytes(planes[192 + row], sh);
+            const uint32_t l0 = __byte_perm(a0, a1, 0x5140), l1 = __byte_perm(a2, a3, 0x5140);
+            const uint32_t h0 = __byte_perm(a0, a1, 0x7362), h1 = __byte_perm(a2, a3, 0x7362);
+            *reinterpret_cast<uint4*>(out + 32 * row + sh) =
+                make_uint4(__byte_perm(l0, l1, 0x5410), __byte_perm(l0, l1, 0x7632), __byte_perm(h0, h1, 0x5410),
+                           __byte_perm(h0, h1, 0x7632));
+        }
+    }
+    __syncthreads();
+    const int lane = t & 31;
+    if (x0 + lane < L.BWp)
+        for (int row = t >> 5; row < 64; row += 8)  // BHp and BWp are multiples of 16: y and z lie in the grid
+            P.bdir[2 * brick_index(L, x0 + lane, y0 + (row & 7), z0 + (row >> 3)) + zs] = out[32 * row + lane];
+}
+
+// ------------------------------------------------------------------ region distances
+//
+// The same for the centred distances of the regions: D(r) = the number of k in [0, 15) for
+// which the cube of side 2k + 1 around r is empty, from E_1, E_2, E_4, E_8 and E_16 of cubes
+// that start at a node and reach toward +.  One tile: 32 x 8 x 8 regions.
+
+constexpr int kRegNodes = 16 * 10 * 10;
+
+struct alignas(16) RegSmem {
+    uint64_t e1[36 * 36];
+    union {
+        uint64_t nodes[kRegNodes];  // done with when E_1 is
+        struct {
+            uint64_t e2[35 * 35], e4[33 * 33], e8[29 * 29], e16[21 * 21];
+        };
+    };
+    uint32_t planes[64][4];
+};
+
+template <int PITCH, int O>
+__device__ __forceinline__ uint64_t cube_from(const uint64_t* e) {
+    const uint64_t v = e[0] & e[O] & e[O * PITCH] & e[O * PITCH + O];
+    return v & v >> O;
+}
+
+// Whether the cube of radius K around the row's nodes is empty; (ly, lz) the row in the tile.
+template <int K>
+__device__ __forceinline__ uint32_t centred(const RegSmem& s, int ly, int lz) {
+    const int y = ly + 14 - K, z = lz + 14 - K;
+    uint64_t v;
+    if constexpr (K == 0) v = s.e1[z * 36 + y];
+    else if constexpr (K < 2) v = cube_from<35, 2 * K + 1 - 2>(s.e2 + z * 35 + y);
+    else if constexpr (K < 4) v = cube_from<33, 2 * K + 1 - 4>(s.e4 + z * 33 + y);
+    else if constexpr (K < 8) v = cube_from<29, 2 * K + 1 - 8>(s.e8 + z * 29 + y);
+    else v = cube_from<21, 2 * K + 1 - 16>(s.e16 + z * 21 + y);
+    return (uint32_t)(v >> (16 - K));
+}
+
+// The distances K0 .. K0 + 3 of a row
+template <int K0>
+__device__ __forceinline__ uint4 centred_planes(const RegSmem& s, int ly, int lz) {
+    uint4 p = make_uint4(0, 0, 0, 0);
+    uint32_t prev = 0xffffffffu;
+    if constexpr (K0 > 0) prev = centred<K0 - 1>(s, ly, lz);
+    const uint32_t a = centred<K0>(s, ly, lz), b = centred<K0 + 1>(s, ly, lz), c = centred<K0 + 2>(s, ly, lz);
+    uint32_t d = 0;  // 15: "15 or more"
+    if constexpr (K0 + 3 < kDistCap) d = centred<K0 + 3>(s, ly, lz);
+    add_planes(p, K0, prev & ~a);
+    add_planes(p, K0 + 1, a & ~b);
+    add_planes(p, K0 + 2, b & ~c);
+    add_planes(p, K0 + 3, c & ~d);
+    return p;
+}
+
+template <int N, int PREV, int STEP>
+__device__ __forceinline__ void cube_level(uint64_t* out, const uint64_t* in) {
+    for (int i = threadIdx.x; i < N * N; i += 256) out[i] = cube_from<PREV, STEP>(in + i / N * PREV + i % N);
+    __syncthreads();
+}
+
+__device__ void region_tile(const NodePass& P, int tile, RegSmem& s) {
+    const Layout& L = P.L;
+    const int x0 = (P.rx0 + tile % P.nrx) * 32, y0 = (P.ry0 + tile / P.nrx % P.nry) * 8;
+    const int z0 = (P.rz0 + tile / (P.nrx * P.nry)) * 8;
+    const int t = threadIdx.x;
+    // the super blocks the tile and its halo span: 16 x 10 x 10; beyond the grid all is empty
+    const int sx0 = x0 / 4 - 4, sy0 = y0 / 4 - 4, sz0 = z0 / 4 - 4;
+    for (int i = t; i < kRegNodes; i += 256) {
+        const int sx = sx0 + (i & 15), sy = sy0 + (i >> 4) % 10, sz = sz0 + i / 160;
+        uint64_t m = 0;
+        if (sx >= 0 && sy >= 0 && sz >= 0 && sx < L.SW && sy < L.SH && sz < L.SW)
+            m = P.supers[super_index(L, sx, sy, sz)];
+        s.nodes[i] = m;
+    }
+    __syncthreads();
+    const uint32_t* n32 = reinterpret_cast<const uint32_t*>(s.nodes);
+    for (int i = t; i < 36 * 36; i += 256) s.e1[i] = ~row_window(n32, i % 36 + 2, i / 36 + 2);
+    (&s.planes[0][0])[t] = 0;
+    __syncthreads();
+    cube_level<35, 36, 1>(s.e2, s.e1);
+    cube_level<33, 35, 2>(s.e4, s.e2);
+    cube_level<29, 33, 4>(s.e8, s.e4);
+    cube_level<21, 29, 8>(s.e16, s.e8);
+    const int row = t & 63, ly = row & 7, lz = row >> 3;
+    const int part = t >> 6;  // four distances of the row each; warp-uniform
+    const uint4 p = part == 0 ? centred_planes<0>(s, ly, lz)
+                              : (part == 1 ? centred_planes<4>(s, ly, lz)
+                                           : (part == 2 ? centred_planes<8>(s, ly, lz) : centred_planes<12>(s, ly, lz)));
+    atomicOr(&s.planes[row][0], p.x);
+    atomicOr(&s.planes[row][1], p.y);
+    atomicOr(&s.planes[row][2], p.z);
+    atomicOr(&s.planes[row][3], p.w);
+    __syncthreads();
+    const int r2 = t >> 2, y = y0 + (r2 & 7), z = z0 + (r2 >> 3);
+    const uint4 q = *reinterpret_cast<const uint4*>(s.planes[r2]);
+    for (int g = 0; g < 2; g++) {
+        const int sh = 8 * (t & 3) + 4 * g;  // RWp is a multiple of 4: all four regions or none
+        if (x0 + sh < L.RWp && y < L.RHp && z < L.RWp)
+            *reinterpret_cast<uint32_t*>(P.rdist + region_linear(L, x0 + sh, y, z)) = plane_bytes(q, sh);
+    }
+}
+
+// The solid bounding box and the depth-field flag: the brick pass left one record per CTA.
+__device__ void merge_boxes(const NodePass& P, int* box) {
+    const int t = threadIdx.x;
+    if (t < 7) box[t] = t < 3 ? (P.reset_box ? INT_MAX : P.aabb[t])
+                              : (t < 6 ? (P.reset_box ? INT_MIN : P.aabb[t]) : (P.reset_flag ? 0 : P.aabb[6]));
+    __syncthreads();
+    int v[7] = {INT_MAX, INT_MAX, INT_MAX, INT_MIN, INT_MIN, INT_MIN, 0};
+    for (int i = t; i < P.n_boxes; i += 256) {
+        const int4 a = *reinterpret_cast<const int4*>(P.boxes + 8 * i), b = *reinterpret_cast<const int4*>(P.boxes + 8 * i + 4);
+        v[0] = min(v[0], a.x); v[1] = min(v[1], a.y); v[2] = min(v[2], a.z);
+        v[3] = max(v[3], a.w); v[4] = max(v[4], b.x); v[5] = max(v[5], b.y); v[6] |= b.z;
+    }
+    for (int k = 0; k < 3; k++) atomicMin(box + k, v[k]);
+    for (int k = 3; k < 6; k++) atomicMax(box + k, v[k]);
+    atomicOr(box + 6, v[6]);
+    __syncthreads();
+    if (t < 7) P.aabb[t] = box[t];
+}
+
+// ------------------------------------------------------------------ launches
+
+union NodeSmem {
+    DirSmem dir;
+    RegSmem reg;
+    FixSmem fix;
+    int box[8];
+};
+
+// The kinds of work lie one after the other in the grid, the longest first.  All of them only
+// read what the brick pass wrote, and write different arrays.
+__global__ void __launch_bounds__(256) node_pass_kernel(const __grid_constant__ NodePass P) {
+    __shared__ NodeSmem s;
+    int b = blockIdx.x;
+    if (b < P.n_fix) return fix_tile(P.fix, b, s.fix);
+    b -= P.n_fix;
+    if (b < P.n_dir) return dir_tile(P, b, s.dir);
+    b -= P.n_dir;
+    if (b < P.n_reg) return region_tile(P, b, s.reg);
+    merge_boxes(P, s.box);
+}
+
+// ------------------------------------------------------------------ brick pass
+//
+// A warp takes 8 bricks in a row along x: lane (b, q) the four rows at z = q of brick b, one
+// 16-byte load each, so that a load instruction covers four whole 128-byte lines.  The words
+// are read once and written only where they change; the masks come from the same registers.
+// Bound by the words' HBM reads: the 512 x 96 x 512 level takes 25 us (4 TB/s), where the masks
+// of the three levels took 58 us in three launches.  An upload from device memory copies and
+// masks in this one pass.  CTAs loop over their bricks and keep the bounding box in registers, which leaves one record
+// per CTA instead of six atomics per warp.
+
+template <int OP>
+__global__ void __launch_bounds__(256, 4) brick_pass_kernel(const __grid_constant__ BrickPass P) {
+    const Layout& L = P.L;
+    const int lane = threadIdx.x & 31, b = lane >> 2, q = lane & 3;
+    const bool vec = (L.W & 3) == 0;
+    int bx_lo = INT_MAX, by_lo = INT_MAX, bz_lo = INT_MAX, bx_hi = INT_MIN, by_hi = INT_MIN, bz_hi = INT_MIN;
+    bool depth = false;
+    for (unsigned task = blockIdx.x * 8 + (threadIdx.x >> 5); task < P.tasks; task += gridDim.x * 8) {
+        const int by = P.by0 + (int)(task / P.ng % P.ny), bz = P.bz0 + (int)(task / P.ng / P.ny);
+        const int bx = 8 * (P.g0 + (int)(task % P.ng)) + b;
+        const bool in = bx >= P.bx0 && bx < P.bx1;
+        const int x0 = 4 * bx, z = 4 * bz + q;
+        const uint64_t slot = brick_index(L, bx, by, bz);
+        uint64_t old = 0;
+        if (in && q == 0) old = P.bricks[slot];
+        int v[4][4];
+#pragma unroll
+        for (int dy = 0; dy < 4; dy++) {
+            const int y = 4 * by + dy;
+            const uint64_t at = ((uint64_t)z * L.H + y) * L.W + x0;
+            v[dy][0] = v[dy][1] = v[dy][2] = v[dy][3] = -1;
+            if (!(in && y < L.H && z < L.W)) continue;
+            if (vec) {
+                const int32_t* from = P.words + at;
+                if (OP == kCopyWords && at >= P.first && at + 4 <= P.first + P.count) {
+                    const int32_t* src = P.src + (at - P.first);
+                    if (((uintptr_t)src & 15) == 0) {
+                        from = src;
+                    } else {
+                        for (int e = 0; e < 4; e++) v[dy][e] = src[e];
+                        from = nullptr;
+                    }
+                }
+                if (from) {
+                    const int4 w = *reinterpret_cast<const int4*>(from);
+                    v[dy][0] = w.x; v[dy][1] = w.y; v[dy][2] = w.z; v[dy][3] = w.w;
+                }
+            } else {
+                for (int e = 0; e < 4; e++)
+                    if (x0 + e < L.W) v[dy][e] = P.words[at + e];
+            }
+        }
+        uint32_t chunk = 0;  // the 16 voxels at z = q, bit x + 4y
+#pragma unroll
+        for (int dy = 0; dy < 4; dy++) {
+            const int y = 4 * by + dy;
+            const bool row = in && y < L.H && z < L.W;
+            if (OP != kReadWords && OP != kStopWords && row) {
+                const uint64_t at = ((uint64_t)z * L.H + y) * L.W + x0;
+                bool changed[4];
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    changed[e] = false;
+                    if (OP == kRemoveSphere) {
+                        const int ox = x0 + e - P.x, oy = y - P.y, oz = z - P.z;
+                        if (v[dy][e] != -1 && ox * ox + oy * oy + oz * oz < P.r * P.r) {
+                            v[dy][e] = -1;
+                            changed[e] = true;
+                        }
+                    } else if (OP == kPlaceVoxel) {
+                        if (x0 + e == P.x && y == P.y && z == P.z) {
+                            v[dy][e] = P.word;
+                            changed[e] = true;
+                        }
+                    } else {
+                        const uint64_t i = at + e;
+                        if (x0 + e < L.W && i >= P.first && i < P.first + P.count) {
+                            if (!(vec && at >= P.first && at + 4 <= P.first + P.count)) v[dy][e] = P.src[i - P.first];
+                            changed[e] = true;
+                        }
+                    }
+                }
+                if (vec && (changed[0] | changed[1] | changed[2] | changed[3])) {
+                    *reinterpret_cast<int4*>(P.words + at) = make_int4(v[dy][0], v[dy][1], v[dy][2], v[dy][3]);
+                } else if (!vec) {
+                    for (int e = 0; e < 4; e++)
+                        if (changed[e] && x0 + e < L.W) P.words[at + e] = v[dy][e];
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                if (OP == kStopWords ? v[dy][e] != -1 : v[dy][e] >= 0) chunk |= 1u << (4 * dy + e);
+                depth |= v[dy][e] < -1;
+            }
+        }
+        uint32_t half = chunk << (16 * (q & 1));
+        half |= __shfl_xor_sync(0xffffffffu, half, 1);
+        const uint32_t other = __shfl_xor_sync(0xffffffffu, half, 2);
+        const uint64_t m = (uint64_t)other << 32 | half;  // right in lanes q = 0
+        if (in && q == 0) {
+            if (m != old) P.bricks[slot] = m;
+            if ((m != 0) != (old != 0)) {  // the brick's own bit of its region
+                unsigned long long* r = reinterpret_cast<unsigned long long*>(
+                    P.regions + region_index(L, bx >> 2, by >> 2, bz >> 2));
+                const unsigned long long bit = 1ull << ((bx & 3) + 4 * (by & 3) + 16 * (bz & 3));
+                // The region's own bit in its super block flips whenever the region's mask becomes
+                // or stops being 0.  Flips of one region by several warps may arrive in any order:
+                // their number alone decides the bit, which sets and clears would not.
+                const unsigned long long was = m ? atomicOr(r, bit) : atomicAnd(r, ~bit);
+                if (was == (m ? 0 : bit) && P.supers)
+                    atomicXor(reinterpret_cast<unsigned long long*>(P.supers + super_index(L, bx >> 4, by >> 4, bz >> 4)),
+                              1ull << ((bx >> 2 & 3) + 4 * (by >> 2 & 3) + 16 * (bz >> 2 & 3)));
+            }
+        }
+        const unsigned solid = __ballot_sync(0xffffffffu, in && q == 0 && m != 0);
+        if (solid) {
+            const int first = bx - b;  // the warp's first brick
+            bx_lo = min(bx_lo, first + (__ffs(solid) - 1) / 4);
+            bx_hi = max(bx_hi, first + (31 - __clz(solid)) / 4);
+            by_lo = min(by_lo, by); by_hi = max(by_hi, by);
+            bz_lo = min(bz_lo, bz); bz_hi = max(bz_hi, bz);
+        }
+    }
+    if (OP == kStopWords) return;
+    __shared__ int box[8];
+    if (threadIdx.x < 8) box[threadIdx.x] = threadIdx.x < 3 ? INT_MAX : (threadIdx.x < 6 ? INT_MIN : 0);
+    __syncthreads();
+    if (__any_sync(0xffffffffu, depth) && lane == 0) box[6] = 1;
+    if (lane == 0 && bx_lo != INT_MAX) {
+        atomicMin(box, 4 * bx_lo); atomicMin(box + 1, 4 * by_lo); atomicMin(box + 2, 4 * bz_lo);
+        atomicMax(box + 3, 4 * bx_hi + 3); atomicMax(box + 4, 4 * by_hi + 3); atomicMax(box + 5, 4 * bz_hi + 3);
+    }
+    __syncthreads();
+    if (threadIdx.x < 8) P.boxes[8 * blockIdx.x + threadIdx.x] = box[threadIdx.x];
+}
+
+// The brick box [b0, b1) of a voxel box, clipped to the world; false when it is empty.
+static bool brick_box(const Layout& L, const int64_t v[6], int b[6]) {
+    const int dim[3] = {L.W, L.H, L.W};
+    for (int a = 0; a < 3; a++) {
+        const int64_t lo = std::max<int64_t>(v[a], 0), hi = std::min<int64_t>(v[3 + a], dim[a]);
+        if (lo >= hi) return false;
+        b[a] = (int)(lo >> 2);
+        b[3 + a] = (int)((hi + 3) >> 2);
+    }
+    return true;
+}
+
+template <int OP>
+static int run_brick_pass(BrickPass& P, int num_sms, cudaStream_t s, int* blocks) {
+    // Whole worlds: 6 CTAs of 8 warps per SM keep 3 KB of loads per warp in flight
+    const unsigned need = (P.tasks + 7) / 8;
+    *blocks = (int)std::min<unsigned>(need, (unsigned)num_sms * kBrickCtasPerSm);
+    brick_pass_kernel<OP><<<*blocks, 256, 0, s>>>(P);
+    VRT_CUDA(cudaGetLastError());
+    return VRT_OK;
+}
+
+static BrickPass brick_pass_of(vrt_world* w, const int b[6]) {
+    BrickPass P{};
+    P.words = w->d_words;
+    P.bricks = w->d_bricks;
+    P.regions = w->d_regions;
+    P.supers = w->d_supers;
+    P.boxes = w->d_boxes;
+    P.L = w->L;
+    P.bx0 = b[0]; P.by0 = b[1]; P.bz0 = b[2]; P.bx1 = b[3];
+    P.g0 = b[0] >> 3;
+    P.ng = (unsigned)(((b[3] + 7) >> 3) - P.g0);
+    P.ny = (unsigned)(b[4] - b[1]);
+    P.tasks = P.ng * P.ny * (unsigned)(b[5] - b[2]);
+    return P;
+}
+
+// Distance tiles of every brick (region) within kDistCap of the changed box.
+static void node_tiles(NodePass& P, const int b[6]) {
+    const Layout& L = P.L;
+    int lo[3], hi[3], rlo[3], rhi[3];
+    const int bdim[3] = {L.BWp, L.BHp, L.BWp}, rdim[3] = {L.RWp, L.RHp, L.RWp};
+    for (int a = 0; a < 3; a++) {
+        lo[a] = std::max(b[a] - kDistCap, 0);
+        hi[a] = std::min(b[3 + a] + kDistCap, bdim[a]);
+        rlo[a] = std::max((b[a] >> 2) - kDistCap, 0);
+        rhi[a] = std::min(((b[3 + a] + 3) >> 2) + kDistCap, rdim[a]);
+    }
+    P.dx0 = lo[0] >> 5; P.ndx = ((hi[0] + 31) >> 5) - P.dx0;
+    P.dy0 = lo[1] >> 3; P.ndy = ((hi[1] + 7) >> 3) - P.dy0;
+    P.dz0 = lo[2] >> 3; P.n_dir = 2 * P.ndx * P.ndy * (((hi[2] + 7) >> 3) - P.dz0);
+    P.rx0 = rlo[0] >> 5; P.nrx = ((rhi[0] + 31) >> 5) - P.rx0;
+    P.ry0 = rlo[1] >> 3; P.nry = ((rhi[1] + 7) >> 3) - P.ry0;
+    P.rz0 = rlo[2] >> 3; P.n_reg = P.nrx * P.nry * (((rhi[2] + 7) >> 3) - P.rz0);
+}
+
+static bool fix_tiles(NodePass& N, vrt_world* w, const int64_t v[6], int cx, int cy, int cz, int r2) {
+    FixPass& P = N.fix;
+    const int dim[3] = {w->L.W, w->L.H, w->L.W};
+    int lo[3], hi[3];
+    for (int a = 0; a < 3; a++) {
+        const int64_t l = std::max<int64_t>(v[a], 0), h = std::min<int64_t>(v[3 + a], dim[a]);
+        if (l >= h) return false;
+        lo[a] = (int)l;
+        hi[a] = (int)h;
+    }
     P.words = w->d_words;
     P.bricks = w->d_bricks;
     P.L = w->L;
-    P.x0 = std::max(x0, 0); P.y0 = std::max(y0, 0); P.z0 = std::max(z0, 0);
-    P.x1 = std::min(x1, w->L.W); P.y1 = std::min(y1, w->L.H); P.z1 = std::min(z1, w->L.W);
-    if (P.x0 >= P.x1 || P.y0 >= P.y1 || P.z0 >= P.z1) return VRT_OK;
+    P.x0 = lo[0]; P.y0 = lo[1]; P.z0 = lo[2];
+    P.x1 = hi[0]; P.y1 = hi[1]; P.z1 = hi[2];
     P.cx = cx; P.cy = cy; P.cz = cz; P.r2 = r2;
     for (int i = 0; i <= kFixLevels; i++) {
         // render.cpp:81: -sqrt(int) through double sqrt, stored as float; nothing found: the
@@ -223,10 +775,68 @@ int launch_fix_depth_field(vrt_world* w, int x0, int y0, int z0, int x1, int y1,
     P.tx0 = P.x0 / kFixX; P.ty0 = P.y0 / kFixY; P.tz0 = P.z0 / kFixZ;
     P.ntx = (P.x1 - 1) / kFixX - P.tx0 + 1;
     P.nty = (P.y1 - 1) / kFixY - P.ty0 + 1;
-    const int ntz = (P.z1 - 1) / kFixZ - P.tz0 + 1;
-    fix_depth_field_kernel<<<P.ntx * P.nty * ntz, 256, 0, s>>>(P);
+    N.n_fix = P.ntx * P.nty * ((P.z1 - 1) / kFixZ - P.tz0 + 1);
+    return true;
+}
+
+static int run_node_pass(const NodePass& P, cudaStream_t s) {
+    const int blocks = P.n_fix + P.n_dir + P.n_reg + (P.n_boxes > 0 ? 1 : 0);
+    if (blocks > 0) node_pass_kernel<<<blocks, 256, 0, s>>>(P);
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;
+}
+
+int change_words(vrt_world* w, const WordChange& c, cudaStream_t s) {
+    const Layout& L = w->L;
+    NodePass N{};
+    N.L = L;
+    N.regions = w->d_regions;
+    N.bdir = reinterpret_cast<uint32_t*>(w->d_bdir);
+    N.supers = w->d_supers;
+    N.rdist = w->d_rdist;
+    N.aabb = w->d_aabb;
+    N.boxes = w->d_boxes;
+    int b[6];
+    if (brick_box(L, c.box, b)) {
+        mark_words(w, c.box);
+        BrickPass P = brick_pass_of(w, b);
+        P.src = c.src; P.first = c.first; P.count = c.count;
+        P.x = c.x; P.y = c.y; P.z = c.z; P.r = c.r; P.word = c.word;
+        int st = VRT_OK;
+        switch (c.op) {
+            case kReadWords: st = run_brick_pass<kReadWords>(P, w->num_sms, s, &N.n_boxes); break;
+            case kRemoveSphere: st = run_brick_pass<kRemoveSphere>(P, w->num_sms, s, &N.n_boxes); break;
+            case kPlaceVoxel: st = run_brick_pass<kPlaceVoxel>(P, w->num_sms, s, &N.n_boxes); break;
+            default: st = run_brick_pass<kCopyWords>(P, w->num_sms, s, &N.n_boxes); break;
+        }
+        if (st) return st;
+        node_tiles(N, b);
+        // a pass over the whole world knows the solid bounding box; a partial one only grows it
+        N.reset_box = b[0] == 0 && b[1] == 0 && b[2] == 0 && 4 * b[3] >= L.W && 4 * b[4] >= L.H && 4 * b[5] >= L.W;
+        N.reset_flag = c.reset_flag;
+    }
+    if (c.fix && fix_tiles(N, w, c.fix_box, c.x, c.y, c.z, c.fix_r)) mark_words(w, c.fix_box);
+    return run_node_pass(N, s);
+}
+
+int refresh_stop_masks(vrt_world* w, cudaStream_t s) {
+    const Layout& L = w->L;
+    const int64_t v[6] = {0, 0, 0, L.W, L.H, L.W};
+    int b[6], blocks = 0;
+    brick_box(L, v, b);
+    BrickPass P = brick_pass_of(w, b);
+    P.bricks = w->d_stop;
+    P.regions = w->d_stop_regions;
+    P.supers = nullptr;
+    const int st = run_brick_pass<kStopWords>(P, w->num_sms, s, &blocks);
+    if (st) return st;
+    NodePass N{};
+    N.L = L;
+    node_tiles(N, b);
+    N.regions = w->d_stop_regions;
+    N.bdir = reinterpret_cast<uint32_t*>(w->d_sdir);
+    N.n_reg = 0;
+    return run_node_pass(N, s);
 }
 
 }  // namespace vrt
