@@ -3,8 +3,8 @@
 // render_word_kernel  one thread per pixel; every DDA step reads the 4-byte voxel word,
 //                     follows depth-field jumps (fshader.glsl:114-121).  Exact on every
 //                     world, including worlds built by fixDepthField.  Steps along z read
-//                     a z-major copy of the words; depth-field worlds prefetch ahead along
-//                     each ray; tiles run heaviest first by the last frame's costs.
+//                     a z-major copy of the words; tiles run heaviest first by the last
+//                     frame's costs.
 // render_mask_kernel  persistent warps over ray tiles; traversal reads the 64-ary
 //                     occupancy hierarchy (64^3 -> 16^3 -> 4^3 -> voxel, one uint64
 //                     per node) and keeps the current brick's 64 voxel bits in
@@ -29,6 +29,40 @@
 
 namespace vrt {
 
+// The pixels of an image's tiles, without integer divisions: 80 of the instructions that each
+// warp spent before its first ray.  A quotient by a constant n is a multiplication by
+// ceil(2^k / n), exact for the few bits of a thread's index, and at most 1 too large for a
+// tile's (tiles < 2^32: the error is below tile / 2^32).
+struct TileMap {
+    int tw, th;        // pixels of a tile, one thread each (tw * th <= 128)
+    int tiles_x;       // tiles in a row of the image
+    uint32_t tw_mul;   // ceil(2^16 / tw)
+    uint32_t row_mul;  // ceil(2^32 / tiles_x), or 0 for tiles_x = 1
+    float inv_w, inv_h;  // 1 / width and 1 / height, rounded to nearest: primary_dir's divisions
+    __device__ __forceinline__ void pixel(int tile, int thread, int& px, int& py) const {
+        int row = row_mul ? (int)__umulhi((uint32_t)tile, row_mul) : tile;
+        int col = tile - row * tiles_x;
+        if (col < 0) {
+            row--;
+            col += tiles_x;
+        }
+        const int ty = (int)((uint32_t)thread * tw_mul >> 16);
+        px = col * tw + (thread - ty * tw);
+        py = row * th + ty;
+    }
+};
+static TileMap tile_map(int width, int height, int tw, int th) {
+    TileMap m;
+    m.tw = tw;
+    m.th = th;
+    m.tiles_x = (width + tw - 1) / tw;
+    m.tw_mul = (65536u + tw - 1) / tw;
+    m.row_mul = m.tiles_x == 1 ? 0 : (uint32_t)(((1ull << 32) + m.tiles_x - 1) / m.tiles_x);
+    m.inv_w = 1.0f / (float)width;
+    m.inv_h = 1.0f / (float)height;
+    return m;
+}
+
 // ====================================================================== word kernel
 
 struct WordParams {
@@ -39,7 +73,8 @@ struct WordParams {
     unsigned long long* stats;
     int bb[6];   // solid bounding box: min x,y,z, max x,y,z (never smaller than the truth)
     int exact;   // 1: every DDA iteration of the shader runs (step counts asked for)
-    int tw, th;  // pixel tile of a CTA (tw * th threads)
+    TileMap map;  // pixel tiles of a CTA each
+    const int32_t* words;    // x + W*y + W*H*z
     const int32_t* words_z;  // the same words with x and z swapped: z + W*y + W*H*x
     // The tile order (see tile_class): the last frame's tiles by cost class, or NULL (CTA
     // (x, y) renders tile (x, y)); this frame's classes, appended to; the counts zeroed for
@@ -102,6 +137,7 @@ __device__ __forceinline__ uint32_t pack_color_tab(const vrt_uniforms& u, bool h
 // inactive light (a coordinate < 0, :167) never is one.
 __device__ __forceinline__ unsigned warp_light_candidates(const vrt_uniforms& u, bool lit, V3 hp) {
     const unsigned full = 0xffffffffu;
+    if (!__any_sync(full, lit)) return 0;  // a warp of sky
     const int x0 = __reduce_min_sync(full, lit ? (int)floorf(hp.x) : INT_MAX);
     const int y0 = __reduce_min_sync(full, lit ? (int)floorf(hp.y) : INT_MAX);
     const int z0 = __reduce_min_sync(full, lit ? (int)floorf(hp.z) : INT_MAX);
@@ -121,6 +157,37 @@ __device__ __forceinline__ unsigned warp_light_candidates(const vrt_uniforms& u,
     return __ballot_sync(full, c);
 }
 
+// t = t + d (round to nearest) where p holds, else t unchanged: one predicated PTX add,
+// which the compiler cannot turn into a branch or a select.
+__device__ __forceinline__ void pred_fadd(float& t, float d, bool p) {
+    asm("{.reg .pred q; setp.ne.b32 q, %1, 0; @q add.rn.f32 %0, %0, %2;}" : "+f"(t) : "r"((int)p), "f"(d));
+}
+
+// The cell of a position and its intersects, fshader.glsl:69-79 and :117-120:
+// t = (float(cell + (s > 0)) - start) / dir.  inv = frcp of dir's components; fast: they lie
+// in div_by's range.
+__device__ __forceinline__ void enter_cell(RaySetup& r, V3 start, V3 dir, V3 inv, bool fast) {
+    if (fast && fminf(fminf(start.x, start.y), start.z) >= kDivMinA &&
+        fmaxf(fmaxf(start.x, start.y), start.z) < 4194304.0f) {
+        // int(x) and float(int(x)) of 0 <= x < 2^22 from x + 2^23 rounded toward zero, on
+        // the FMA pipe instead of six conversions at an eighth of its rate
+        const float mx = __fadd_rz(start.x, 8388608.0f), my = __fadd_rz(start.y, 8388608.0f),
+                    mz = __fadd_rz(start.z, 8388608.0f);
+        r.cx = __float_as_int(mx) - 0x4B000000;
+        r.cy = __float_as_int(my) - 0x4B000000;
+        r.cz = __float_as_int(mz) - 0x4B000000;
+        // the next cell's bound: (mx - 2^23) + 1 or + 0 is mx - (2^23 - 1) or mx - 2^23, both exact
+        r.tx = div_by(fsub(fsub(mx, r.sx > 0 ? 8388607.0f : 8388608.0f), start.x), dir.x, inv.x);
+        r.ty = div_by(fsub(fsub(my, r.sy > 0 ? 8388607.0f : 8388608.0f), start.y), dir.y, inv.y);
+        r.tz = div_by(fsub(fsub(mz, r.sz > 0 ? 8388607.0f : 8388608.0f), start.z), dir.z, inv.z);
+    } else {
+        r.cx = f2i(start.x); r.cy = f2i(start.y); r.cz = f2i(start.z);
+        r.tx = fdiv(fsub((float)(r.cx + (r.sx > 0)), start.x), dir.x);
+        r.ty = fdiv(fsub((float)(r.cy + (r.sy > 0)), start.y), dir.y);
+        r.tz = fdiv(fsub((float)(r.cz + (r.sz > 0)), start.z), dir.z);
+    }
+}
+
 struct WordRay {
     int32_t hit;   // voxel index or -1
     float cd;      // currDist at the hit
@@ -128,11 +195,6 @@ struct WordRay {
     V3 start;      // start position after depth-field jumps (hitPos uses it)
     int steps;
 };
-
-// How far ahead along its line a ray of the word kernel prefetches, in cell lengths.
-constexpr float WORD_AHEAD = 24.0f;
-
-__device__ __forceinline__ void prefetch_l1(const int32_t* a) { asm volatile("prefetch.global.L1 [%0];" ::"l"(a)); }
 
 // castRay, fshader.glsl:59-129, over the voxel words.  A cell outside the world ends the
 // ray, getVoxelIndex == -1 (:123-125).  Inexact launches also end a ray that cannot hit
@@ -142,18 +204,29 @@ __device__ __forceinline__ void prefetch_l1(const int32_t* a) { asm volatile("pr
 // true.  (Only y: in terrain worlds the solid box spans x and z, and two registers per
 // ray are what this latency-bound kernel can spare.)
 //
-// AHEAD: each iteration also prefetches, into L1, the words of the cell WORD_AHEAD cell
-// lengths further along the ray's line, in both copies.  Every cell the ray visits lies on
-// that line (a depth-field jump moves the start along it), so the long rays that end a
-// frame find their words in L1 instead of waiting on one miss per step.  A prefetch reads
-// nothing into a register, so results are unchanged.
-template <bool AHEAD>
-__device__ WordRay cast_word(const int32_t* __restrict__ words, const Layout& L, const WordParams& p, V3 start,
-                             V3 dir, int dist, int maxSteps) {
+// What bounds it: instruction issue (72 % of the slots while an SM is busy), 52 M warp
+// instructions for an 800x600 frame of the level with three lights.  An iteration is about 40
+// instructions, a jump 45 more, a ray's set-up and shading 400.  The jump's three IEEE
+// divisions as div_by, the intersect adds left to the iterations that do not jump, and no
+// prefetch of the words ahead (24 instructions in each iteration, once worth it for its long
+// dependent chain): that frame 77.7 -> 66.6 us, the app's first frame 67.2 -> 60.3 us (of
+// which the divisions alone are nothing and the prefetch 8 us).  Tried without gain: 8x4 tiles
+// of the words instead of the second copy (96 us on the app's first frame), both copies' loads
+// predicated (75.7), 5 to 8 CTAs per SM by fewer registers (67.0-69.3), one warp per CTA (63.6
+// against 60.3 us with 16x8 tiles).
+__device__ WordRay cast_word(const Layout& L, const WordParams& p, V3 start, V3 dir, int dist, int maxSteps) {
     WordRay o;
     o.hit = -1; o.cd = 0.0f; o.axis = 2; o.s = 0; o.steps = 0;
     RaySetup r;
-    ray_setup(start, dir, r);
+    // The divisions by the ray's direction, here and at each jump: see div_by.
+    const V3 inv{frcp(dir.x), frcp(dir.y), frcp(dir.z)};
+    const bool fast = fminf(fminf(fabsf(dir.x), fabsf(dir.y)), fabsf(dir.z)) >= kDivMinB &&
+                      fmaxf(fmaxf(fabsf(dir.x), fabsf(dir.y)), fabsf(dir.z)) <= kDivMaxB;
+    r.sx = isign(dir.x); r.sy = isign(dir.y); r.sz = isign(dir.z);
+    r.dx = frcp(fabsf(fadd(dir.x, 0.000001f)));
+    r.dy = frcp(fabsf(fadd(dir.y, 0.000001f)));
+    r.dz = frcp(fabsf(fadd(dir.z, 0.000001f)));
+    enter_cell(r, start, dir, inv, fast);
     int lo_y = 0, span_y = L.H;
     if (!p.exact) {
         if (r.sy > 0) {
@@ -163,96 +236,88 @@ __device__ WordRay cast_word(const int32_t* __restrict__ words, const Layout& L,
             span_y = L.H - lo_y;
         }
     }
-    float cd = 0.0f, travelled = 0.0f;
-    const float fdist = (float)dist, fcap = (float)maxSteps;
-    int axis = 2, s = 0;
-    while (travelled < fdist && travelled < fcap) {
+    float travelled = 0.0f;
+    const float lim = fminf((float)dist, (float)maxSteps);
+    const int W = L.W, WH = L.W * L.H;
+    while (travelled < lim) {
         o.steps++;
         travelled = fadd(travelled, 1.0f);
-        {
-            // The shader's axis choice (strict <, ties to z), as selects: its neighbouring
-            // pixels step different axes, and three divergent branches per step cost this
-            // latency-bound loop more than the selects (0.089 -> 0.083 ms on the reference
-            // scene).
-            const bool bx = (r.tx < r.ty) & (r.tx < r.tz);
-            const bool by = (r.ty < r.tx) & (r.ty < r.tz);  // false whenever bx holds, NaN included
-            cd = bx ? r.tx : (by ? r.ty : r.tz);
-            const float tn = fadd(cd, bx ? r.dx : (by ? r.dy : r.dz));
-            axis = bx ? 0 : (by ? 1 : 2);
-            s = bx ? r.sx : (by ? r.sy : r.sz);
-            r.cx += bx ? r.sx : 0;
-            r.cy += by ? r.sy : 0;
-            r.cz += (bx | by) ? 0 : r.sz;
-            r.tx = bx ? tn : r.tx;
-            r.ty = by ? tn : r.ty;
-            r.tz = (bx | by) ? r.tz : tn;
-        }
-        if ((unsigned)r.cx >= (unsigned)L.W || (unsigned)(r.cy - lo_y) >= (unsigned)span_y ||
-            (unsigned)r.cz >= (unsigned)L.W)
-            break;  // getVoxelIndex == -1, or no solid voxel ahead
-        if (AHEAD) {  // the cell clamped to the world, so the address is always inside both copies
-            const float t = cd + WORD_AHEAD;
-            const int ax = min(max(__float2int_rz(__fmaf_rn(dir.x, t, start.x)), 0), L.W - 1);
-            const int ay = min(max(__float2int_rz(__fmaf_rn(dir.y, t, start.y)), 0), L.H - 1);
-            const int az = min(max(__float2int_rz(__fmaf_rn(dir.z, t, start.z)), 0), L.W - 1);
-            prefetch_l1(words + (ax + L.W * ay + L.W * L.H * az));
-            prefetch_l1(p.words_z + (az + L.W * ay + L.W * L.H * ax));
-        }
+        // The shader's axis choice (strict <, ties to z); each axis' move is predicated, not a
+        // divergent branch.
+        const bool bx = (r.tx < r.ty) & (r.tx < r.tz);
+        const bool by = (r.ty < r.tx) & (r.ty < r.tz);  // false whenever bx holds, NaN included
+        const bool bz = !(bx | by);
+        if (bx) r.cx += r.sx;
+        if (by) r.cy += r.sy;
+        if (bz) r.cz += r.sz;
+        // Outside the world (getVoxelIndex == -1), or no solid voxel ahead: the ray ends as at a
+        // solid voxel (word 0), without a hit.
+        const bool in = ((unsigned)r.cx < (unsigned)L.W) & ((unsigned)(r.cy - lo_y) < (unsigned)span_y) &
+                        ((unsigned)r.cz < (unsigned)L.W);
         // A step along z reads the copy in which z is the fastest index: a run of z steps then
         // reads consecutive words instead of one cache line per step (W*H words apart).  That
         // run is the longest ray of the reference's own frame: the shader's x == y tie sends a
         // ray along z for hundreds of steps, which set the frame's length.
-        const int32_t* q = axis == 2 ? p.words_z + (r.cz + L.W * r.cy + L.W * L.H * r.cx)
-                                     : words + (r.cx + L.W * r.cy + L.W * L.H * r.cz);
-        const int32_t v = __ldg(q);
-        if (v >= 0) {
-            o.hit = r.cx + L.W * r.cy + L.W * L.H * r.cz;
-            break;
-        } else if (v != -1) {  // depth-field jump
-            float toJump = -__int_as_float(v);
+        int32_t v = 0;
+        if (in) v = __ldg((bz ? p.words_z : p.words) + ((bz ? r.cz : r.cx) + W * r.cy + WH * (bz ? r.cx : r.cz)));
+        const bool plain = v == -1;
+        if (!plain) {
+            const float cd = bx ? r.tx : (by ? r.ty : r.tz);
+            if (v >= 0) {
+                if (in) {
+                    o.hit = r.cx + W * r.cy + WH * r.cz;
+                    o.cd = cd;
+                    o.axis = bx ? 0 : (by ? 1 : 2);
+                    o.s = bx ? r.sx : (by ? r.sy : r.sz);
+                    o.start = start;
+                }
+                break;
+            }
+            // depth-field jump
+            const float toJump = -__int_as_float(v);
             travelled = fadd(travelled, toJump);
-            cd = fadd(cd, toJump);
-            start = add3(mul3s(dir, cd), start);
-            r.cx = f2i(start.x); r.cy = f2i(start.y); r.cz = f2i(start.z);
-            r.tx = fdiv(fsub((float)(r.cx + (r.sx > 0)), start.x), dir.x);
-            r.ty = fdiv(fsub((float)(r.cy + (r.sy > 0)), start.y), dir.y);
-            r.tz = fdiv(fsub((float)(r.cz + (r.sz > 0)), start.z), dir.z);
+            start = add3(mul3s(dir, fadd(cd, toJump)), start);
+            enter_cell(r, start, dir, inv, fast);
         }
+        pred_fadd(r.tx, r.dx, bx & plain);
+        pred_fadd(r.ty, r.dy, by & plain);
+        pred_fadd(r.tz, r.dz, bz & plain);
     }
-    o.cd = cd; o.axis = axis; o.s = s; o.start = start;
     return o;
 }
 
-// A minimum of 4 CTAs per SM gives the compiler up to 128 registers; it takes 77 (6 CTAs
-// per SM).  The reference frame, whose length is set by a few long chains of dependent
-// steps, ran 0.0806 against 0.0814 ms with the default bound (64 registers, 8 CTAs per SM).
-template <bool DEBUG, bool AHEAD>
+// A minimum of 4 CTAs per SM gives the compiler up to 128 registers; it takes 72 (7 CTAs
+// per SM).
+template <bool DEBUG>
 __global__ void __launch_bounds__(128, 4) render_word_kernel(const int32_t* __restrict__ words, Layout L,
                                                           const __grid_constant__ WordParams p) {
-    __shared__ int s_cost, s_tile;
-    if (threadIdx.x == 0) {
-        const int b = (int)(blockIdx.x + gridDim.x * blockIdx.y);
+    __shared__ int s_cost, s_done, s_tile;
+    if (threadIdx.x < 32) {
+        const int b = (int)(blockIdx.x + gridDim.x * blockIdx.y), lane = threadIdx.x;
         int tile = b;
         if (p.class_count_in) {  // the b-th tile of the last frame's classes, heaviest class first
-            int base = 0;
-            for (int c = kTileClasses - 1; c >= 0; c--) {
-                const int n = __ldg(p.class_count_in + c);
-                if (b < base + n) {
-                    tile = __ldg(p.class_list_in + c * p.tiles + (b - base));
-                    break;
-                }
-                base += n;
+            const int c = kTileClasses - 1 - lane;  // lane l: class 15 - l, and how many lie before it
+            const int n = lane < kTileClasses ? __ldg(p.class_count_in + c) : 0;
+            int end = n;
+            for (int o = 1; o < kTileClasses; o *= 2) {
+                const int u = __shfl_up_sync(0xffffffffu, end, o);
+                if (lane >= o) end += u;
             }
+            if (b < end && b >= end - n) tile = __ldg(p.class_list_in + c * p.tiles + (b - (end - n)));
+            const unsigned found = __ballot_sync(0xffffffffu, b < end && b >= end - n);
+            tile = __shfl_sync(0xffffffffu, tile, found ? __ffs(found) - 1 : 0);
         }
-        if (b == 0 && p.class_count_clear)
-            for (int c = 0; c < kTileClasses; c++) p.class_count_clear[c] = 0;
-        s_tile = tile;
-        s_cost = 0;
+        if (b == 0 && p.class_count_clear && lane < kTileClasses) p.class_count_clear[lane] = 0;
+        if (lane == 0) {
+            s_tile = tile;
+            s_cost = 0;
+            s_done = 0;
+        }
     }
     __syncthreads();
     const int tile = s_tile;
-    const int px = (tile % (int)gridDim.x) * p.tw + (int)threadIdx.x % p.tw;
-    const int py = (tile / (int)gridDim.x) * p.th + (int)threadIdx.x / p.tw;
+    int px, py;
+    p.map.pixel(tile, (int)threadIdx.x, px, py);
     const bool valid = px < p.width && py < p.height;
     PixelResult res{};
     const vrt_uniforms& u = p.u;
@@ -261,8 +326,8 @@ __global__ void __launch_bounds__(128, 4) render_word_kernel(const int32_t* __re
     WordRay pr;
     pr.hit = -1; pr.cd = 0.f; pr.axis = 2; pr.s = 0; pr.start = cam; pr.steps = 0;
     if (valid) {
-        rd = primary_dir(u, px, py, p.width, p.height);
-        pr = cast_word<AHEAD>(words, L, p, cam, rd, u.maxSteps, u.maxSteps);
+        rd = primary_dir(u, px, py, p.width, p.height, p.map.inv_w, p.map.inv_h);
+        pr = cast_word(L, p, cam, rd, u.maxSteps, u.maxSteps);
     }
     const bool lit = valid && pr.hit >= 0 && u.viewDepthField != 1;
     const V3 hp = lit ? add3(mul3s(rd, pr.cd), pr.start) : V3{0.f, 0.f, 0.f};
@@ -279,7 +344,7 @@ __global__ void __launch_bounds__(128, 4) render_word_kernel(const int32_t* __re
             V3 hn = axis_normal(pr.axis, pr.s);
             V3 lp{u.lightPos[0], u.lightPos[1], u.lightPos[2]};
             V3 toLight = norm3(sub3(lp, hp));
-            WordRay sr = cast_word<AHEAD>(words, L, p, add3(hp, mul3s(toLight, 0.001f)), toLight, u.maxSteps, u.maxSteps);
+            WordRay sr = cast_word(L, p, add3(hp, mul3s(toLight, 0.001f)), toLight, u.maxSteps, u.maxSteps);
             res.steps += sr.steps;
             res.cast |= 1u;
             if (sr.hit < 0) {
@@ -311,7 +376,7 @@ __global__ void __launch_bounds__(128, 4) render_word_kernel(const int32_t* __re
                 float ld = len3(dl);
                 if (ld <= R) {
                     V3 tl = norm3(dl);
-                    WordRay lr = cast_word<AHEAD>(words, L, p, add3(hp, mul3s(tl, 0.001f)), tl, f2i(fadd(ld, 1.0f)),
+                    WordRay lr = cast_word(L, p, add3(hp, mul3s(tl, 0.001f)), tl, f2i(fadd(ld, 1.0f)),
                                            u.maxSteps);
                     res.steps += lr.steps;
                     res.cast |= 2u << i;
@@ -336,11 +401,15 @@ __global__ void __launch_bounds__(128, 4) render_word_kernel(const int32_t* __re
         else reinterpret_cast<uint32_t*>(p.rgba)[(uint64_t)py * p.width + px] = res.rgba;
     }
     const int wmax = __reduce_max_sync(0xffffffffu, valid ? res.steps : 0);
-    if ((threadIdx.x & 31) == 0) atomicMax(&s_cost, wmax);
-    __syncthreads();
-    if (threadIdx.x == 0 && p.class_list_out) {
-        const int c = tile_class(s_cost);
-        p.class_list_out[c * p.tiles + atomicAdd(p.class_count_out + c, 1)] = tile;
+    // The CTA's last warp to end appends the tile; nobody waits for it.
+    if ((threadIdx.x & 31) == 0 && p.class_list_out) {
+        atomicMax(&s_cost, wmax);
+        __threadfence_block();
+        if (atomicAdd(&s_done, 1) == (int)blockDim.x / 32 - 1) {
+            __threadfence_block();
+            const int c = tile_class(atomicMax(&s_cost, 0));
+            p.class_list_out[c * p.tiles + atomicAdd(p.class_count_out + c, 1)] = tile;
+        }
     }
     if (p.stats) {
         unsigned rays = valid ? 1u + __popc(res.cast) : 0u;
@@ -366,9 +435,8 @@ __global__ void __launch_bounds__(128, 4) render_word_kernel(const int32_t* __re
 struct ViewDev {
     vrt_uniforms u;
     int width, height;
-    int tiles_x;
+    TileMap map;
     int tile_begin;  // first global tile of this view
-    int tile_w, tile_h;
     int refill_min;  // lanes parked before a warp runs its slow phase (tile's view decides)
     int exact;       // 1: step every ray to its end (step counts asked for); 0: end rays that cannot hit
     uint8_t* rgba;
@@ -555,7 +623,7 @@ __global__ void __launch_bounds__(kThreads, MINB) render_mask_kernel(const __gri
                     const float cd = r.la == 0 ? r.tx : (r.la == 1 ? r.ty : r.tz);
                     hit = r.cx + P.L.W * r.cy + P.L.W * P.L.H * r.cz;
                     const int px = pix % V.width, py = pix / V.width;
-                    V3 rd = primary_dir(u, px, py, V.width, V.height);
+                    V3 rd = primary_dir(u, px, py, V.width, V.height, V.map.inv_w, V.map.inv_h);
                     hp = add3(mul3s(rd, cd), V3{u.camPos[0], u.camPos[1], u.camPos[2]});
                     const int s = r.la == 0 ? r.sx : (r.la == 1 ? r.sy : r.sz);
                     LSU(F_HN) = (uint32_t)(r.la | ((s + 1) << 2));
@@ -685,14 +753,14 @@ __global__ void __launch_bounds__(kThreads, MINB) render_mask_kernel(const __gri
                 const ViewDev& V = view_of(P, v);
                 const int lt_idx = (int)t - V.tile_begin;
                 q_vid = v;
-                q_tw = V.tile_w;
-                q_x0 = (lt_idx % V.tiles_x) * V.tile_w;
-                q_y0 = (lt_idx / V.tiles_x) * V.tile_h;
+                q_tw = V.map.tw;
+                q_x0 = (lt_idx % V.map.tiles_x) * V.map.tw;
+                q_y0 = (lt_idx / V.map.tiles_x) * V.map.th;
                 q_w = V.width;
                 q_h = V.height;
                 q_thr = V.refill_min;
                 q_pos = 0;
-                q_size = V.tile_w * V.tile_h;
+                q_size = V.map.tw * V.map.th;
             }
             const int rank = __popc(need & lt);
             const int take = min(__popc(need), q_size - q_pos);
@@ -709,7 +777,7 @@ __global__ void __launch_bounds__(kThreads, MINB) render_mask_kernel(const __gri
                     LSF(F_HPX) = 0.f; LSF(F_HPY) = 0.f; LSF(F_HPZ) = 0.f;
                     LSU(F_HN) = 2u | (1u << 2);
                     o = V3{u.camPos[0], u.camPos[1], u.camPos[2]};
-                    d = primary_dir(u, px, py, q_w, q_h);
+                    d = primary_dir(u, px, py, q_w, q_h, view_of(P, q_vid).map.inv_w, view_of(P, q_vid).map.inv_h);
                     n = u.maxSteps;
                     want = true;
                     phase = PH_PRIMARY;
@@ -809,12 +877,6 @@ __device__ __forceinline__ void set_axis(int c, int s, int lo, int hi, int kmax,
     const int ee = s > 0 ? hi : lo - 1;
     k = min(s != 0 ? s * (ee - c) - 1 : INT_MAX, kmax);
     e = s * k + c;
-}
-
-// t = t + d (round to nearest) where p holds, else t unchanged: one predicated PTX add,
-// which the compiler cannot turn into a branch or a select.
-__device__ __forceinline__ void pred_fadd(float& t, float d, bool p) {
-    asm("{.reg .pred q; setp.ne.b32 q, %1, 0; @q add.rn.f32 %0, %0, %2;}" : "+f"(t) : "r"((int)p), "f"(d));
 }
 
 // Per-octant alive ranges of a launch, one (lo, span) pair per octant and axis: a cell
@@ -1141,8 +1203,8 @@ __global__ void __launch_bounds__(128, 7) render_tiles_kernel(const __grid_const
     const int tile = (int)blockIdx.x + P.tile0;
     const ViewDev& V = view_of(P, view_of_tile(P, tile));
     const int lt = tile - V.tile_begin;
-    const int px = (lt % V.tiles_x) * V.tile_w + (int)threadIdx.x % V.tile_w;
-    const int py = (lt / V.tiles_x) * V.tile_h + (int)threadIdx.x / V.tile_w;
+    int px, py;
+    V.map.pixel(lt, (int)threadIdx.x, px, py);
     const bool valid = px < V.width && py < V.height;
     PixelResult res{};
     unsigned refills = 0;
@@ -1155,7 +1217,7 @@ __global__ void __launch_bounds__(128, 7) render_tiles_kernel(const __grid_const
     int pr = T_MISS;
     V3 from = cam, from2;  // the start a hit position is measured from (moved by depth-field jumps)
     if (valid) {
-        rd = primary_dir(u, px, py, V.width, V.height);
+        rd = primary_dir(u, px, py, V.width, V.height, V.map.inv_w, V.map.inv_h);
         pr = cast_box<DF, DEBUG>(P, alive, clip_k, cam, rd, u.maxSteps, u.maxSteps, cd, axis, sgn, steps, hit, refills, from);
         res.primary_steps = steps;
     }
@@ -1459,10 +1521,8 @@ static void fill_view(ViewDev& v, const vrt_uniforms& u, int width, int height, 
     v.u = u;
     v.width = width;
     v.height = height;
-    v.tile_w = t.tile_w;
-    v.tile_h = t.tile_h;
+    v.map = tile_map(width, height, t.tile_w, t.tile_h);
     v.refill_min = t.refill_min;
-    v.tiles_x = (width + t.tile_w - 1) / t.tile_w;
     v.tile_begin = tile_begin;
     v.rgba = rgba;
     if (dbg) v.dbg = *dbg;
@@ -1617,33 +1677,24 @@ int vrt_render(vrt_renderer* r, const vrt_world* w, const vrt_uniforms* u, int32
         std::memcpy(p.bb, w->h_aabb, sizeof(p.bb));
         p.exact = (opts && opts->exact_steps) || u->viewDepthField == 1 || (dbg && (dbg->steps || dbg->primary_steps));
         // 16x8 pixels per CTA unless the options name another tile (a multiple of 32 threads, at most 128)
-        p.tw = opts && opts->tile_w > 0 && opts->tile_h > 0 ? opts->tile_w : 16;
-        p.th = opts && opts->tile_w > 0 && opts->tile_h > 0 ? opts->tile_h : 8;
-        const int threads = p.tw * p.th;
+        const int tw = opts && opts->tile_w > 0 && opts->tile_h > 0 ? opts->tile_w : 16;
+        const int th = opts && opts->tile_w > 0 && opts->tile_h > 0 ? opts->tile_h : 8;
+        const int threads = tw * th;
         if (threads % 32 != 0 || threads > 128)
-            return set_error(VRT_EINVAL, "pixel tile %dx%d: tile_w*tile_h must be a multiple of 32 up to 128", p.tw,
-                             p.th);
-        dim3 grid((width + p.tw - 1) / p.tw, (height + p.th - 1) / p.th);
+            return set_error(VRT_EINVAL, "pixel tile %dx%d: tile_w*tile_h must be a multiple of 32 up to 128", tw, th);
+        p.map = tile_map(width, height, tw, th);
+        dim3 grid((width + tw - 1) / tw, (height + th - 1) / th);
         // the z-major copy of the words is a cache of them, brought up to date here
         st = refresh_words_z(const_cast<vrt_world*>(w), S(stream));
         if (st) return st;
+        p.words = w->d_words;
         p.words_z = w->d_words_z;
         st = word_tile_order(r, grid, S(stream), &p);
         if (st) return st;
         const bool debug = dbg && (dbg->hit_index || dbg->cast_mask || dbg->occ_mask || dbg->steps ||
                                    dbg->primary_steps || dbg->shade);
-        // Depth-field worlds prefetch ahead: their frames end on long rays near the surface
-        // (0.115 -> 0.101 ms on the reference scene).  Other worlds' frames are many short
-        // rays, for which the prefetch is only extra instructions (0.250 -> 0.285 ms for this
-        // kernel on a 1080p terrain frame).
-        const bool ahead = w->has_depth_field != 0;
-        if (debug) {
-            if (ahead) render_word_kernel<true, true><<<grid, threads, 0, S(stream)>>>(w->d_words, w->L, p);
-            else render_word_kernel<true, false><<<grid, threads, 0, S(stream)>>>(w->d_words, w->L, p);
-        } else {
-            if (ahead) render_word_kernel<false, true><<<grid, threads, 0, S(stream)>>>(w->d_words, w->L, p);
-            else render_word_kernel<false, false><<<grid, threads, 0, S(stream)>>>(w->d_words, w->L, p);
-        }
+        if (debug) render_word_kernel<true><<<grid, threads, 0, S(stream)>>>(w->d_words, w->L, p);
+        else render_word_kernel<false><<<grid, threads, 0, S(stream)>>>(w->d_words, w->L, p);
         const cudaError_t le = cudaGetLastError();
         if (le != cudaSuccess) {
             r->tile_gx = r->tile_gy = 0;  // the classes of this frame were not written
@@ -1754,7 +1805,7 @@ int vrt_render_to_host(vrt_renderer* r, const vrt_world* w, const vrt_uniforms* 
     if (st) return st;
     ViewDev v;
     fill_view(v, *u, width, height, r->d_staging, nullptr, nullptr, t, 0);
-    const int tiles_x = v.tiles_x, tiles_y = (height + t.tile_h - 1) / t.tile_h;
+    const int tiles_x = v.map.tiles_x, tiles_y = (height + t.tile_h - 1) / t.tile_h;
     const int total = tiles_x * tiles_y;
     const size_t row_bytes = (size_t)width * 4;
     // Each band renders on its own stream, with no order among the bands: the launches run
