@@ -110,9 +110,10 @@ struct vrt_world {
 
 namespace vrt {
 // A change of a world's words and what follows from it (world_passes.cu).
-enum { kReadWords, kRemoveSphere, kPlaceVoxel, kCopyWords, kStopWords };
+enum { kReadWords, kRemoveSphere, kPlaceVoxel, kCopyWords, kInitLevel, kStopWords };
 struct WordChange {
-    int op;                 // kReadWords: the words changed already, or are to be looked at again
+    int op;                 // kReadWords: the words changed already, or are to be looked at again;
+                            // kInitLevel: the reference's level (initVoxels, level.cpp:82-138)
     int64_t box[6];         // the words concerned: [x0,y0,z0, x1,y1,z1), clipped to the world; may be empty
     const int32_t* src;     // kCopyWords: words [first, first + count) are copied from here
     uint64_t first, count;
@@ -129,7 +130,7 @@ int change_words(vrt_world* w, const WordChange& c, cudaStream_t s);
 // Note that the words of the box changed: the stop masks and, there, the z-major copy follow.
 void mark_words(vrt_world* w, const int64_t box[6]);
 // CTAs of a brick pass per SM, at most
-constexpr int kBrickCtasPerSm = 6;
+constexpr int kBrickCtasPerSm = 4;
 // Rebuild the stop masks and their directed distances from the words.
 int refresh_stop_masks(vrt_world* w, cudaStream_t s);
 // Bring the stop masks and their directed distances up to date (allocated on first use),

@@ -3,7 +3,7 @@
 //   removeSphere  level.cpp:30-56        -> change_words (world_passes.cu)
 //   fixDepthField render.cpp:226-253     -> change_words
 //   placeVoxel    render.cpp:256-262     -> change_words
-//   initVoxels    level.cpp:82-138       -> init_reference_layers_kernel + init_reference_trees_kernel
+//   initVoxels    level.cpp:82-138       -> change_words
 //   updateGeometry/updatePartialGeometry render.cpp:199-223 -> vrt_world_upload -> change_words
 #include <cuda_runtime.h>
 
@@ -191,67 +191,6 @@ __global__ void probe_kernel(const int32_t* __restrict__ words, Layout L, const 
     const int x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
     const bool in = x >= 0 && y >= 0 && z >= 0 && x < L.W && y < L.H && z < L.W;
     out[i] = in ? words[(uint64_t)x + (uint64_t)L.W * y + (uint64_t)L.W * L.H * z] : -1;
-}
-
-// ------------------------------------------------------------------ initVoxels
-
-// level.cpp:85-128: stone/dirt/grass layers, then the holes that placeBush/placeTrunk
-// punch near the origin by calling destroyVoxel with relative coordinates
-// (level.cpp:11,64): (0,0..5,0) from the trunks and the x,y,z >= 0 part of the radius-6
-// ball from the bushes.  Both are applied after the layers, as in the reference.
-__global__ void init_reference_layers_kernel(int32_t* __restrict__ words, Layout L, int any_tree) {
-    uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= L.n_words) return;
-    int x = (int)(t % L.W), y = (int)((t / L.W) % L.H), z = (int)(t / ((uint64_t)L.W * L.H));
-    int cv = 5 * ((x + y + z) % 3);
-    int v = -1;
-    if (y <= 25) v = ((90 + cv) << 16) | ((90 + cv) << 8) | (90 + cv);
-    else if (y <= 33) v = ((120 + cv) << 16) | ((100 + cv) << 8);
-    else if (y <= 36) v = (10 << 16) | ((130 + cv) << 8) | 10;
-    if (any_tree) {
-        if (x == 0 && z == 0 && y < 6) v = -1;
-        if (x < 6 && y < 6 && z < 6 && x * x + y * y + z * z < 36) v = -1;
-    }
-    words[t] = v;
-}
-
-// One tree per blockIdx.y: trunk (placeTrunk, level.cpp:59-79) then bush (placeBush,
-// level.cpp:4-27) over the tree's bounding box [-6,6)^3 around the bush centre, which
-// contains the trunk; the bush is written last, so it wins where the two overlap.
-// Trees are 30 x 25 voxels apart and never overlap each other.
-__global__ void init_reference_trees_kernel(int32_t* __restrict__ words, Layout L, int trees_x) {
-    int tree = blockIdx.y;
-    int tx = 30 * (1 + tree % trees_x);       // x % 30 == 0, x in [10, W-10)
-    int tz = 25 * (1 + tree / trees_x);       // z % 25 == 0, z in [10, W-10)
-    int bush_x = tx + tz % 7, bush_y = 46, bush_z = tz;      // level.cpp:134
-    int trunk_x = tx + 1 + tz % 7, trunk_y = 36, trunk_z = tz; // level.cpp:133
-    // box around the bush centre: x in [bush_x-6, bush_x+6) covers the trunk (x offsets [-2,1) from bush_x+1)
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int bw = 12, bh = 16;  // y from 36 (trunk base) to 52 (bush top)
-    if (t >= bw * bh * bw) return;
-    int ax = bush_x - 6 + t % bw;
-    int ay = 36 + (t / bw) % bh;
-    int az = bush_z - 6 + t / (bw * bh);
-    if (ax < 0 || ay < 0 || az < 0 || ax >= L.W || ay >= L.H || az >= L.W) return;
-    int v = 0;
-    bool write = false;
-    {   // placeTrunk(ivec3(trunk_x, 36, tz), ivec3(128,100,15), 6): x,z in [-2,1), y in [0,6)
-        int x = ax - trunk_x, y = ay - trunk_y, z = az - trunk_z;
-        if (x >= -2 && x < 1 && z >= -2 && z < 1 && y >= 0 && y < 6) {
-            int r = 128 - ((x + z) % 2) * 10, g = 100 - ((x + z) % 2) * 10;
-            v = (((r << 8) + g) << 8) + 15;
-            write = true;
-        }
-    }
-    {   // placeBush(ivec3(bush_x, 46, tz), ivec3(15,128,15), 6): offsets in [-6,6)^3, |o|^2 < 36
-        int x = ax - bush_x, y = ay - bush_y, z = az - bush_z;
-        if (x >= -6 && x < 6 && y >= -6 && y < 6 && z >= -6 && z < 6 && x * x + y * y + z * z < 36) {
-            int g = 128 - ((x + y + z) % 3) * 20;
-            v = (((15 << 8) + g) << 8) + 15;
-            write = true;
-        }
-    }
-    if (write) words[(uint64_t)ax + (uint64_t)L.W * ay + (uint64_t)L.W * L.H * az] = v;
 }
 
 }  // namespace vrt
@@ -546,20 +485,8 @@ int vrt_remove_sphere(vrt_world* w, int32_t cx, int32_t cy, int32_t cz, int32_t 
 
 int vrt_world_init_reference(vrt_world* w, void* stream) {
     if (!w) return set_error(VRT_EINVAL, "NULL world");
-    const Layout& L = w->L;
-    // trees at x % 30 == 0 and z % 25 == 0 for x, z in [10, W-10) (level.cpp:130-137)
-    int trees_x = 0, trees_z = 0;
-    for (int x = 10; x < L.W - 10; x++) trees_x += (x % 30 == 0);
-    for (int z = 10; z < L.W - 10; z++) trees_z += (z % 25 == 0);
-    init_reference_layers_kernel<<<blocks_for(L.n_words, 256), 256, 0, S(stream)>>>(w->d_words, L,
-                                                                                    trees_x * trees_z > 0);
-    VRT_CUDA(cudaGetLastError());
-    if (trees_x * trees_z > 0) {
-        dim3 grid(blocks_for(12 * 16 * 12, 256), trees_x * trees_z);
-        init_reference_trees_kernel<<<grid, 256, 0, S(stream)>>>(w->d_words, L, trees_x);
-        VRT_CUDA(cudaGetLastError());
-    }
-    WordChange c = whole_world(L);
+    WordChange c = whole_world(w->L);
+    c.op = kInitLevel;
     c.reset_flag = true;
     w->has_depth_field = 0;
     int flag = 0;

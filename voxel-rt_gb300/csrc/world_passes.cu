@@ -1,6 +1,6 @@
 // The passes behind every change of a world's words, in two launches:
 //   brick_pass_kernel  changes the words (removeSphere, placeVoxel, an upload from device
-//                      memory, or nothing), and rebuilds the brick masks of the box in the same
+//                      memory, the reference's level, or nothing), and rebuilds the brick masks of the box in the same
 //                      pass, with the region and super masks' bits, the solid bounding box
 //                      and the depth-field flag;
 //   node_pass_kernel   everything that follows from them, as independent tiles of one launch:
@@ -142,9 +142,12 @@ __device__ __forceinline__ uint32_t fix_or(const uint32_t* d, std::integer_seque
 }
 
 // Add level S (and the levels after it) to a row: found = voxels whose smallest s is known.
+// Now and then the warp looks whether every air voxel of its rows has been found.
 template <int S>
-__device__ __forceinline__ void fix_levels(const uint32_t* d, uint32_t& found, uint32_t (&bit)[6]) {
+__device__ __forceinline__ void fix_levels(const uint32_t* d, uint32_t air, uint32_t& found, uint32_t (&bit)[6]) {
     if constexpr (S < kFixLevels) {
+        if constexpr (S == 5 || S == 10 || S == 17 || S == 26)
+            if (!__any_sync(0xffffffffu, (air & ~found) != 0)) return;
         if constexpr (FixTable<S>::L.n > 0) {
             const uint32_t now = fix_or<S>(d, std::make_integer_sequence<int, FixTable<S>::L.n>{}) & ~found;
             found |= now;
@@ -155,7 +158,7 @@ __device__ __forceinline__ void fix_levels(const uint32_t* d, uint32_t& found, u
             if (S & 16) bit[4] |= now;
             if (S & 32) bit[5] |= now;
         }
-        fix_levels<S + 1>(d, found, bit);
+        fix_levels<S + 1>(d, air, found, bit);
     }
 }
 
@@ -216,7 +219,8 @@ __device__ void fix_tile(const FixPass& P, int tile, FixSmem& s) {
             }
         }
         __syncthreads();
-        if (air) fix_levels<3>(s.d + ((t >> 4) + kFixHalo) * kFixPitch + (t & 15) + kFixHalo, found, bit);
+        if (__any_sync(0xffffffffu, air != 0))
+            fix_levels<3>(s.d + ((t >> 4) + kFixHalo) * kFixPitch + (t & 15) + kFixHalo, air, found, bit);
     }
     // s <= 3 was recorded as 3: those voxels keep their word
     const uint32_t keep = found & ~(bit[2] | bit[3] | bit[4] | bit[5]);
@@ -225,21 +229,37 @@ __device__ void fix_tile(const FixPass& P, int tile, FixSmem& s) {
     s.out[6][t] = air & ~keep;
     __syncthreads();
 
-    // write: a warp per row, a lane per voxel
-    const int lane = t & 31;
-    for (int row = t >> 5; row < kFixY * kFixZ; row += 8) {
-        const uint32_t wr = s.out[6][row];
-        if (!(wr >> lane & 1)) continue;
-        const int ry = y0 + (row & 15), rz = z0 + (row >> 4), rx = x0 + lane;
-        if (P.r2 > 0) {
-            const int ox = rx - P.cx, oy = ry - P.cy, oz = rz - P.cz;
-            if (ox * ox + oy * oy + oz * oz >= P.r2 * P.r2) continue;
-        }
-        int sq = 0;
+    // write: four voxels of a row per thread, one 16-byte store where all four change
+    const bool vec = (L.W & 3) == 0;
+    const int seg = 4 * (t & 7);
+    for (int row = t >> 3; row < kFixY * kFixZ; row += 32) {
+        uint32_t wr = s.out[6][row] >> seg & 15;
+        if (!wr) continue;
+        const int ry = y0 + (row & 15), rz = z0 + (row >> 4), rx = x0 + seg;
+        uint32_t b[6];
 #pragma unroll
-        for (int k = 0; k < 6; k++) sq |= (int)(s.out[k][row] >> lane & 1) << k;
-        // every recorded s is at least 3, so 0 says that no solid voxel was found
-        P.words[(uint64_t)rx + (uint64_t)L.W * ry + (uint64_t)L.W * L.H * rz] = s.word[sq ? sq : kFixLevels];
+        for (int k = 0; k < 6; k++) b[k] = s.out[k][row] >> seg;
+        int32_t v[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            int sq = 0;
+#pragma unroll
+            for (int k = 0; k < 6; k++) sq |= (int)(b[k] >> e & 1) << k;
+            // every recorded s is at least 3, so 0 says that no solid voxel was found
+            v[e] = s.word[sq ? sq : kFixLevels];
+            if (P.r2 > 0) {
+                const int ox = rx + e - P.cx, oy = ry - P.cy, oz = rz - P.cz;
+                if (ox * ox + oy * oy + oz * oz >= P.r2 * P.r2) wr &= ~(1u << e);
+            }
+        }
+        int32_t* q = P.words + ((uint64_t)rx + (uint64_t)L.W * ry + (uint64_t)L.W * L.H * rz);
+        if (vec && wr == 15) {
+            *reinterpret_cast<int4*>(q) = make_int4(v[0], v[1], v[2], v[3]);
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+                if (wr >> e & 1) q[e] = v[e];
+        }
     }
 }
 
@@ -557,15 +577,64 @@ __global__ void __launch_bounds__(256) node_pass_kernel(const __grid_constant__ 
     merge_boxes(P, s.box);
 }
 
+// The depth field alone (fixDepthField over a box): without the distance tiles' 80 registers
+// a fourth CTA fits on each SM.
+__global__ void __launch_bounds__(256, 4) fix_depth_field_kernel(const __grid_constant__ FixPass P) {
+    __shared__ FixSmem s;
+    fix_tile(P, blockIdx.x, s);
+}
+
 // ------------------------------------------------------------------ brick pass
 //
 // A warp takes 8 bricks in a row along x: lane (b, q) the four rows at z = q of brick b, one
 // 16-byte load each, so that a load instruction covers four whole 128-byte lines.  The words
 // are read once and written only where they change; the masks come from the same registers.
+// The reference's level is made in this pass too: 33 us, bound by its stores and the trees'
+// arithmetic, where layers, trees and masks took 131 us in three launches.
 // Bound by the words' HBM reads: the 512 x 96 x 512 level takes 25 us (4 TB/s), where the masks
 // of the three levels took 58 us in three launches.  An upload from device memory copies and
 // masks in this one pass.  CTAs loop over their bricks and keep the bounding box in registers, which leaves one record
 // per CTA instead of six atomics per warp.
+
+// Four voxels of the reference's level (initVoxels, level.cpp:82-138) along x: stone, dirt
+// and grass layers (:85-128), then the holes that placeBush and placeTrunk punch near the
+// origin by calling destroyVoxel with relative coordinates (:11, :64) -- (0, 0..5, 0) from the
+// trunks and the x, y, z >= 0 part of the radius-6 ball from the bushes -- and a tree at every
+// x % 30 == 0, z % 25 == 0 of [10, W - 10) (:130-137): trunk, then bush, which wins where
+// both are.  Trees are 30 x 25 voxels apart and 12 wide, so at most one reaches a voxel.
+// (y is the same for a whole warp, so the layers' branches do not diverge.)
+__device__ __forceinline__ void level_row(int (&v)[4], int x0, int y, int z, int W) {
+    const bool any_tree = W - 10 > 30;  // the first ones stand at x = 30 and z = 25
+    if (y <= 36) {
+        // 5 * ((x + y + z) % 3) on top of every channel of stone, red and green of dirt, green of grass
+        const int base = y <= 25 ? 0x5A5A5A : (y <= 33 ? 0x786400 : 0x0A820A);
+        const int step = y <= 25 ? 0x050505 : (y <= 33 ? 0x050500 : 0x000500);
+        const int m = (x0 + y + z) % 3, n = m == 2 ? 0 : m + 1, o = n == 2 ? 0 : n + 1;
+        v[0] = v[3] = base + m * step;
+        v[1] = base + n * step;
+        v[2] = base + o * step;
+        if (any_tree && y < 6 && x0 < 6 && z < 6)
+            for (int e = 0; e < 4; e++)
+                if ((x0 + e == 0 && z == 0) || (x0 + e < 6 && (x0 + e) * (x0 + e) + y * y + z * z < 36)) v[e] = -1;
+    }
+    if (any_tree && y >= 36 && y < 52) {
+        const int tz = (z + 6) / 25 * 25, lean = tz % 7, oz = z - tz;  // level.cpp:133-134
+        if (tz == 0 || tz >= W - 10 || oz >= 6) return;
+        for (int e = 0; e < 4; e++) {
+            const int tx = (x0 + e - lean + 6) / 30 * 30;
+            const int ox = x0 + e - lean - tx;  // from the bush's centre, (tx + tz % 7, 46, tz)
+            if (tx <= 0 || tx >= W - 10 || ox >= 6) continue;
+            // placeTrunk(ivec3(bush x + 1, 36, tz), ivec3(128,100,15), 6): x, z in [-2,1), y in [0,6)
+            const int ux = ox - 1, uy = y - 36, oy = y - 46;
+            if (ux >= -2 && ux < 1 && oz >= -2 && oz < 1 && uy < 6) {
+                const int d = (ux + oz) % 2 * 10;
+                v[e] = ((((128 - d) << 8) + 100 - d) << 8) + 15;
+            }
+            // placeBush(ivec3(bush x, 46, tz), ivec3(15,128,15), 6): offsets in [-6,6)^3, |o|^2 < 36
+            if (oy >= -6 && ox * ox + oy * oy + oz * oz < 36) v[e] = (((15 << 8) + 128 - (ox + oy + oz) % 3 * 20) << 8) + 15;
+        }
+    }
+}
 
 template <int OP>
 __global__ void __launch_bounds__(256, 4) brick_pass_kernel(const __grid_constant__ BrickPass P) {
@@ -589,6 +658,13 @@ __global__ void __launch_bounds__(256, 4) brick_pass_kernel(const __grid_constan
             const uint64_t at = ((uint64_t)z * L.H + y) * L.W + x0;
             v[dy][0] = v[dy][1] = v[dy][2] = v[dy][3] = -1;
             if (!(in && y < L.H && z < L.W)) continue;
+            if (OP == kInitLevel) {
+                level_row(v[dy], x0, y, z, L.W);
+                if (!vec)
+                    for (int e = 0; e < 4; e++)
+                        if (x0 + e >= L.W) v[dy][e] = -1;
+                continue;
+            }
             if (vec) {
                 const int32_t* from = P.words + at;
                 if (OP == kCopyWords && at >= P.first && at + 4 <= P.first + P.count) {
@@ -631,6 +707,8 @@ __global__ void __launch_bounds__(256, 4) brick_pass_kernel(const __grid_constan
                             v[dy][e] = P.word;
                             changed[e] = true;
                         }
+                    } else if (OP == kInitLevel) {
+                        changed[e] = x0 + e < L.W;
                     } else {
                         const uint64_t i = at + e;
                         if (x0 + e < L.W && i >= P.first && i < P.first + P.count) {
@@ -649,7 +727,7 @@ __global__ void __launch_bounds__(256, 4) brick_pass_kernel(const __grid_constan
 #pragma unroll
             for (int e = 0; e < 4; e++) {
                 if (OP == kStopWords ? v[dy][e] != -1 : v[dy][e] >= 0) chunk |= 1u << (4 * dy + e);
-                depth |= v[dy][e] < -1;
+                if (OP != kInitLevel) depth |= v[dy][e] < -1;
             }
         }
         uint32_t half = chunk << (16 * (q & 1));
@@ -707,7 +785,7 @@ static bool brick_box(const Layout& L, const int64_t v[6], int b[6]) {
 
 template <int OP>
 static int run_brick_pass(BrickPass& P, int num_sms, cudaStream_t s, int* blocks) {
-    // Whole worlds: 6 CTAs of 8 warps per SM keep 3 KB of loads per warp in flight
+    // Whole worlds: as many CTAs as fit at once, each looping over its share
     const unsigned need = (P.tasks + 7) / 8;
     *blocks = (int)std::min<unsigned>(need, (unsigned)num_sms * kBrickCtasPerSm);
     brick_pass_kernel<OP><<<*blocks, 256, 0, s>>>(P);
@@ -781,7 +859,8 @@ static bool fix_tiles(NodePass& N, vrt_world* w, const int64_t v[6], int cx, int
 
 static int run_node_pass(const NodePass& P, cudaStream_t s) {
     const int blocks = P.n_fix + P.n_dir + P.n_reg + (P.n_boxes > 0 ? 1 : 0);
-    if (blocks > 0) node_pass_kernel<<<blocks, 256, 0, s>>>(P);
+    if (blocks > 0 && blocks == P.n_fix) fix_depth_field_kernel<<<blocks, 256, 0, s>>>(P.fix);
+    else if (blocks > 0) node_pass_kernel<<<blocks, 256, 0, s>>>(P);
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;
 }
@@ -806,6 +885,7 @@ int change_words(vrt_world* w, const WordChange& c, cudaStream_t s) {
         switch (c.op) {
             case kReadWords: st = run_brick_pass<kReadWords>(P, w->num_sms, s, &N.n_boxes); break;
             case kRemoveSphere: st = run_brick_pass<kRemoveSphere>(P, w->num_sms, s, &N.n_boxes); break;
+            case kInitLevel: st = run_brick_pass<kInitLevel>(P, w->num_sms, s, &N.n_boxes); break;
             case kPlaceVoxel: st = run_brick_pass<kPlaceVoxel>(P, w->num_sms, s, &N.n_boxes); break;
             default: st = run_brick_pass<kCopyWords>(P, w->num_sms, s, &N.n_boxes); break;
         }
