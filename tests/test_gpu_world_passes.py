@@ -4,7 +4,8 @@ the depth field's radius) and dense ones, against the oracle, word for word."""
 import numpy as np
 import pytest
 
-from helpers import expected_distances, expected_masks, make_world
+import vrt
+from helpers import assert_same_frame, expected_distances, expected_masks, gpu_render, make_world
 
 pytestmark = pytest.mark.gpu
 
@@ -92,3 +93,37 @@ def test_structures_follow_uploads_and_edits(cuda, W, H):
     words.reshape(W, H, W)[x * x + y * y + z * z < 81] = -1
     assert np.array_equal(w.download(np.empty_like(words)), words)
     check_structures(w, words, W, H)
+
+
+@pytest.mark.parametrize("W,H", [(37, 33), (64, 48)])
+def test_frames_after_edits_that_write_the_z_major_copy(cuda, oracle, W, H):
+    """Small edits change the word kernel's z-major copy with the words; uploads and large
+    spheres leave it to the next frame.  In any order between two frames, each frame equals
+    the oracle's on the words of that moment."""
+    words = sparse_words(W, H, W, 0.2)
+    w = make_world(words, W, H)
+    w.fix_depth_field()
+    u = vrt.default_uniforms()
+    u.camPos[:] = [2.5, H - 2.25, 3.5]
+    u.rotateMatrix[:] = vrt.rotate_matrix(0.4, 0.6)
+    u.lightPos[:] = [W / 2, 300.0, W / 3]
+    u.aspectRatio = 1.5
+    rng = np.random.default_rng(3)
+
+    def small():
+        w.remove_sphere(*[int(rng.integers(0, n)) for n in (W, H, W)], 4, 1)
+
+    def voxel():
+        w.place_voxel(int(rng.integers(0, W)), int(rng.integers(0, H)), int(rng.integers(0, W)), 0x01FF8000)
+
+    def slab():
+        w.upload(sparse_words(W, H, 5, 0.3)[: 2 * W * H + 7], first=5 * W * H + 3)
+
+    def large():
+        w.remove_sphere(W, H, W, 22, 1)
+
+    for edits in ((), (small, voxel), (slab, small), (small, slab, voxel), (large, small), (voxel, large)):
+        for e in edits:
+            e()
+        now = w.download(np.empty(W * H * W, np.int32))
+        assert_same_frame(oracle.render(now, W, H, u, 60, 40), gpu_render(w, u, 60, 40, kernel=vrt.KERNEL_WORD))

@@ -127,8 +127,9 @@ struct WordChange {
 // Change the words, and bring the masks, distances, solid box and flag up to date: at most two
 // launches.
 int change_words(vrt_world* w, const WordChange& c, cudaStream_t s);
-// Note that the words of the box changed: the stop masks and, there, the z-major copy follow.
-void mark_words(vrt_world* w, const int64_t box[6]);
+// Note that the words of the box changed: the stop masks follow, and there the z-major copy
+// if it has not been changed with them.
+void mark_words(vrt_world* w, const int64_t box[6], bool z_copy);
 // CTAs of a brick pass per SM, at most
 constexpr int kBrickCtasPerSm = 4;
 // Rebuild the stop masks and their directed distances from the words.
