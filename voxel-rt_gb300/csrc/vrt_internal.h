@@ -106,6 +106,7 @@ struct vrt_world {
     uint64_t device_bytes = 0;
     int device = 0;
     int num_sms = 0;
+    bool reads_pageable = false;    // kernels read pageable host memory through the host's page tables
 };
 
 namespace vrt {
