@@ -1464,7 +1464,8 @@ static int launch_mask(vrt_renderer* r, const vrt_world* w, const ViewDev* h_vie
 
 // Tile kernel launch over the views' tile space (1 view: h_views[0] as a parameter).
 static int launch_tiles(const vrt_world* w, const ViewDev* h_views, int nviews, int total_tiles,
-                        const ViewDev* d_views, int threads, cudaStream_t s, int tile0 = 0, int ntiles = -1) {
+                        const ViewDev* d_views, int threads, cudaStream_t s, int tile0 = 0, int ntiles = -1,
+                        bool count_lookups = true) {
     MaskParams P;
     std::memset(&P, 0, sizeof(P));
     P.words = w->d_words;
@@ -1486,12 +1487,13 @@ static int launch_tiles(const vrt_world* w, const ViewDev* h_views, int nviews, 
         P.cl[3 + a] = exact ? dims[a] : std::min(dims[a], std::max(P.bb[3 + a] + 1, P.cl[a]));
     }
     // DEBUG launches store side outputs and count box lookups: any view with a debug output
-    // or counters
+    // or counters (whoever reads no more of the counters than rays, hits and pixels can do
+    // without the lookups: count_lookups)
     bool debug = false;
     for (int i = 0; i < nviews; i++) {
         const vrt_debug_out& d = h_views[i].dbg;
         debug |= d.hit_index || d.cast_mask || d.occ_mask || d.steps || d.primary_steps || d.shade ||
-                 h_views[i].stats != nullptr;
+                 (count_lookups && h_views[i].stats != nullptr);
     }
     const bool df = w->has_depth_field != 0;
     if (df) {
@@ -1893,13 +1895,14 @@ static int batch_tuning(const vrt_render_opts* opts, Tuning* t, bool* tiles) {
 }
 
 static int launch_batch(vrt_renderer* r, const vrt_world* w, const ViewDev* hv, int count, int total,
-                        const Tuning& t, bool tiles, const ViewDev* d_views, unsigned* d_counter, cudaStream_t s) {
-    if (tiles) return launch_tiles(w, hv, count, total, d_views, t.tile_w * t.tile_h, s);
+                        const Tuning& t, bool tiles, const ViewDev* d_views, unsigned* d_counter, cudaStream_t s,
+                        bool count_lookups = true) {
+    if (tiles) return launch_tiles(w, hv, count, total, d_views, t.tile_w * t.tile_h, s, 0, -1, count_lookups);
     return launch_mask(r, w, hv, count, total, t, d_views, d_counter, s);
 }
 
-int vrt_render_batch(vrt_renderer* r, const vrt_view* views, int32_t count, const vrt_render_opts* opts,
-                     void* stream) {
+static int render_batch(vrt_renderer* r, const vrt_view* views, int32_t count, const vrt_render_opts* opts,
+                        void* stream, bool count_lookups) {
     if (!r) return set_error(VRT_EINVAL, "NULL renderer");
     Tuning t;
     bool tiles = true;
@@ -1916,7 +1919,12 @@ int vrt_render_batch(vrt_renderer* r, const vrt_view* views, int32_t count, cons
         // pageable source: the copy is staged before the call returns, so hv may go
         VRT_CUDA(cudaMemcpyAsync(r->d_views, hv.data(), sizeof(ViewDev) * count, cudaMemcpyHostToDevice, S(stream)));
     }
-    return launch_batch(r, w, hv.data(), count, total, t, tiles, r->d_views, r->d_counter, S(stream));
+    return launch_batch(r, w, hv.data(), count, total, t, tiles, r->d_views, r->d_counter, S(stream), count_lookups);
+}
+
+int vrt_render_batch(vrt_renderer* r, const vrt_view* views, int32_t count, const vrt_render_opts* opts,
+                     void* stream) {
+    return render_batch(r, views, count, opts, stream, true);
 }
 
 int vrt_batch_graph_create(vrt_renderer* r, const vrt_view* views, int32_t count, const vrt_render_opts* opts,
@@ -2011,6 +2019,10 @@ int vrt_probe_l2_read_gbs(uint64_t bytes, int32_t iters, double* gbs_out) {
 }
 
 }  // extern "C"
+
+int vrt::render_batch_rays(vrt_renderer* r, const vrt_view* views, int32_t count, void* stream) {
+    return render_batch(r, views, count, nullptr, stream, false);
+}
 
 // ====================================================================== batch without allocation
 

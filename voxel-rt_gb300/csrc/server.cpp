@@ -264,7 +264,7 @@ static int launch_renders(vrt_server* s, int si, std::vector<Queued>& batch) {
     }
     if (we.has_edit) VRT_CUDA(cudaStreamWaitEvent(sl.stream, we.edit_event, 0));
     VRT_CUDA(cudaMemsetAsync(sl.d_stats, 0, sizeof(uint64_t) * VRT_STAT_COUNT * batch.size(), sl.stream));
-    st = vrt_render_batch(sl.renderer, views.data(), (int)views.size(), nullptr, sl.stream);
+    st = render_batch_rays(sl.renderer, views.data(), (int)views.size(), sl.stream);
     if (st) {
         release_images(s, sl);
         return st;

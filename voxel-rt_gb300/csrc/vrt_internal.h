@@ -142,4 +142,7 @@ int refresh_stop(vrt_world* w, cudaStream_t s);
 // only the box changed since), and make stream s wait until it is: the update may have
 // run on another stream.
 int refresh_words_z(vrt_world* w, cudaStream_t s);
+// vrt_render_batch without the box-lookup counter: the launch that stores no side output
+// (63 registers, 8 CTAs per SM) instead of the one that does (69, 7 CTAs).
+int render_batch_rays(vrt_renderer* r, const vrt_view* views, int32_t count, void* stream);
 }  // namespace vrt
