@@ -165,7 +165,7 @@ __device__ __forceinline__ void pred_fadd(float& t, float d, bool p) {
 
 // The cell of a position and its intersects, fshader.glsl:69-79 and :117-120:
 // t = (float(cell + (s > 0)) - start) / dir.  inv = frcp of dir's components; fast: they lie
-// in div_by's range.
+// in div_by's range, and the ray's first start is no NaN (a jump's NaN shows in every component).
 __device__ __forceinline__ void enter_cell(RaySetup& r, V3 start, V3 dir, V3 inv, bool fast) {
     if (fast && fminf(fminf(start.x, start.y), start.z) >= kDivMinA &&
         fmaxf(fmaxf(start.x, start.y), start.z) < 4194304.0f) {
@@ -220,8 +220,8 @@ __device__ WordRay cast_word(const Layout& L, const WordParams& p, V3 start, V3 
     RaySetup r;
     // The divisions by the ray's direction, here and at each jump: see div_by.
     const V3 inv{frcp(dir.x), frcp(dir.y), frcp(dir.z)};
-    const bool fast = fminf(fminf(fabsf(dir.x), fabsf(dir.y)), fabsf(dir.z)) >= kDivMinB &&
-                      fmaxf(fmaxf(fabsf(dir.x), fabsf(dir.y)), fabsf(dir.z)) <= kDivMaxB;
+    const float lo = min3_nan(start.x, start.y, start.z);
+    const bool fast = all_within(dir, kDivMinB, kDivMaxB) & (lo == lo);
     r.sx = isign(dir.x); r.sy = isign(dir.y); r.sz = isign(dir.z);
     r.dx = frcp(fabsf(fadd(dir.x, 0.000001f)));
     r.dy = frcp(fabsf(fadd(dir.y, 0.000001f)));
@@ -453,6 +453,8 @@ struct MaskParams {
     int cl[6];             // tile kernel: boxes are clipped to [cl[0],cl[3]) x [cl[1],cl[4]) x [cl[2],cl[5])
     int tile0;             // tile kernel: the launch covers tiles [tile0, tile0 + gridDim.x)
     int one, four, sixteen;  // 1, 4, 16: multipliers the compiler cannot fold (see cast_box)
+    int4 clip_k[27];       // tile kernel: see enter_box_lean
+    int4 oct_k[16];        // tile kernel: see cast_lean
     Layout L;
     const ViewDev* views;  // nviews entries (device); NULL when nviews == 1 (v0 is used)
     int nviews;
@@ -537,8 +539,7 @@ __device__ __forceinline__ int refill(Ray& r, const MaskParams& P, const uint8_t
         const uint64_t bi = brick_index(L, bx, by, bz);
         m = __ldg(P.bricks + bi);
         const int oct = (r.sx > 0) | ((r.sy > 0) << 1) | ((r.sz > 0) << 2);
-        const int db = __ldg(P.bdir + bi * 8 + oct);
-        const int k = m ? 0 : max(db, 1) - 1;
+        const int k = __ldg(P.bdir + bi * 8 + oct) >> 2;  // 0 for a non-empty brick
         lox = (bx - k) << 2; loy = (by - k) << 2; loz = (bz - k) << 2;
         hix = (bx + k + 1) << 2; hiy = (by + k + 1) << 2; hiz = (bz + k + 1) << 2;
     }
@@ -927,8 +928,7 @@ __device__ __forceinline__ int enter_box(BoxRay& r, int cx, int cy, int cz, cons
     const uint32_t bidx = (uint32_t)bx + (uint32_t)L.BWp * ((uint32_t)by + (uint32_t)L.BHp * (uint32_t)bz);
     // the two loads are independent: issue them together, wait once
     const uint64_t m = __ldg(P.bricks + bidx);
-    const int db = __ldg(P.bdir + (bidx * 8u + oct));
-    const int k = m ? 0 : max(db, 1) - 1;
+    const int k = __ldg(P.bdir + (bidx * 8u + oct)) >> 2;  // 0 for a non-empty brick
     // clip to the world, and for inexact launches to the solid box too: a ray that
     // leaves the solid box along its direction of travel then ends at the next lookup.
     // (Multiplies by a kernel parameter equal to 4 rather than shifts: FMA pipe.)
@@ -974,8 +974,7 @@ __device__ __forceinline__ int enter_box_lean(BoxRay& r, int cx, int cy, int cz,
     const int bx = cx >> 2, by = cy >> 2, bz = cz >> 2;
     const uint32_t bidx = (uint32_t)bx + (uint32_t)L.BWp * ((uint32_t)by + (uint32_t)L.BHp * (uint32_t)bz);
     const uint64_t m = __ldg(P.bricks + bidx);
-    const int db = __ldg(P.bdir + (bidx * 8u + A.w));
-    const int kk4 = (max(db, 1) - 1) * P.four;  // a non-empty brick has distance 0: its own box
+    const int kk4 = __ldg(P.bdir + (bidx * 8u + A.w));  // 0 for a non-empty brick: its own box
     const int kmax = (int)__umulhi((unsigned)max(left, 0), 0x55555556u);  // floor(left / 3)
     r.kx = min(min((((r.sx > 0) ? ~cx : cx) & 3) + kk4, kcx), kmax);
     r.ky = min(min((((r.sy > 0) ? ~cy : cy) & 3) + kk4, kcy), kmax);
@@ -1001,13 +1000,11 @@ __device__ __forceinline__ int enter_box_lean(BoxRay& r, int cx, int cy, int cz,
 // float because the jumps make distTravelled fractional.  start_out receives the start
 // the hit position is measured from.
 template <bool DF, bool COUNT>
-__device__ __forceinline__ int cast_box(const MaskParams& P, const int2* alive, const int4* clip_k, V3 o, V3 d,
-                                        int n, int maxSteps,
+__device__ __forceinline__ int cast_box(const MaskParams& P, const int2* alive, const int4* clip_k,
+                                        const RaySetup& s, V3 o, V3 d, int n, int maxSteps,
                                         float& cd, int& axis, int& sgn, int& steps, int32_t& hit_index,
                                         unsigned& refills, V3& start_out) {
     start_out = o;
-    RaySetup s;
-    ray_setup(o, d, s);
     BoxRay r;
     r.tx = s.tx; r.ty = s.ty; r.tz = s.tz;
     r.dx = s.dx; r.dy = s.dy; r.dz = s.dz;
@@ -1164,6 +1161,142 @@ __device__ __forceinline__ int cast_box(const MaskParams& P, const int2* alive, 
     return result;
 }
 
+// cast_box for a ray that moves along every axis and whose set-up held only ordinary numbers
+// (ray_setup_lean): practically all of them.  Such a ray only moves forward, so it is walked
+// in coordinates mirrored where it moves backward: q = c, or M - 1 - c with M the padded size
+// of the axis, a multiple of 4, so that bricks stay aligned.  Every step adds 1 to q, the rest
+// of a brick is 3 - (q & 3), the far side of the clip box and the slot of a brick need no sign
+// and no select, and the first cell is checked by one subtraction per axis.
+// oct_k: per octant {far clip side of q per axis, the brick slot of q = 0}, then {near side of
+// the world in q per axis, 63 ^ the bit flips of the mirrored axes}, from the host.
+//
+// The frame is bound by its instructions (86 % of the issue slots): on a 1080p frame of 191 M
+// warp instructions, 3.7 M warp iterations took 22 each, 0.8 M lookups 80, and 65 K pixels'
+// and 130 K rays' frame work the rest.  Mirrored, with the rays' reciprocals and quotients as
+// rcp_near and div_by and the octants' constants from the host: 182 M, 203.6 -> 192.3 us; 4K
+// grazing 574 -> 550, 64 views 4008 -> 3792, every side output of 853x479 89.4 -> 83.3.
+// Three ways to step several axes at once while a whole warp is in empty boxes (74-88 % of
+// the iterations, 1.8-2.4 steps a trip) lost by 1 to 25 %: the votes that keep the warp
+// together cost more per lookup than the trips save.
+template <bool COUNT>
+__device__ __forceinline__ int cast_lean(const MaskParams& P, const int4* oct_k, const RaySetup& s, int n,
+                                         int maxSteps, float& cd, int& axis, int& sgn, int& steps,
+                                         int32_t& hit_index, unsigned& refills) {
+    const Layout& L = P.L;
+    float tx = s.tx, ty = s.ty, tz = s.tz;
+    const int n0 = max(0, min(n, maxSteps));
+    if (n0 == 0) return T_MISS;
+    const int one = P.one, four = P.four, sixteen = P.sixteen;
+    const int sx = s.sx, sy4 = s.sy * four, sz16 = s.sz * sixteen;  // the bit-index moves along x, y and z
+    const int by_step = s.sy * L.BWp, bz_step = s.sz * L.BWp * L.BHp;
+    const int oct = (sx > 0) | ((s.sy > 0) << 1) | ((s.sz > 0) << 2);
+    int ex = sx > 0 ? s.cx : 4 * L.BWp - 1 - s.cx;
+    int ey = s.sy > 0 ? s.cy : 4 * L.BHp - 1 - s.cy;
+    int ez = s.sz > 0 ? s.cz : 4 * L.BWp - 1 - s.cz;
+    int flip;
+    {   // the first cell lies before the near side of the world: getVoxelIndex == -1
+        const int4 near = oct_k[8 + oct];
+        flip = near.w;
+        const bool fx = (tx < ty) & (tx < tz), fy = (ty < tx) & (ty < tz);
+        if (((ex + fx - near.x) | (ey + fy - near.y) | (ez + !(fx | fy) - near.z)) < 0) {
+            steps += 1;
+            return T_MISS;
+        }
+    }
+    const int left0 = n0 - 1;
+    int lb = left0, left_end = left0;
+    int kx = 0, ky = 0, kz = 0;  // no box yet: the first step along any axis triggers a lookup
+    uint64_t m = 0;
+    int bi = 0, result = T_MISS;
+#pragma unroll 2
+    for (;;) {
+        const bool bx = (tx < ty) & (tx < tz);
+        const bool by = (ty < tx) & (ty < tz);
+        const bool bz = !(bx | by);
+        if (bx) kx = kx * one - 1;
+        if (by) ky = ky * one - 1;
+        if (bz) kz = kz * one - 1;
+        if (bx) bi = bi * one + sx;
+        if (by) bi = bi * one + sy4;
+        if (bz) bi = bi * one + sz16;
+        uint64_t mb;
+        asm("shr.b64 %0, %1, %2;" : "=l"(mb) : "l"(m), "r"(bi));
+        const bool hb = mb & 1;
+        if (((kx | ky | kz) < 0) | hb) {
+            const int left = lb + kx + ky + kz;
+            left_end = left;
+            const int qx = ex - kx, qy = ey - ky, qz = ez - kz;
+            result = T_HIT;
+            if ((kx | ky | kz) < 0) {
+                if (COUNT) refills++;
+                const int4 A = oct_k[oct];
+                const int cx = A.x - qx, cy = A.y - qy, cz = A.z - qz;  // steps before the far clip side
+                result = T_MISS;
+                if ((cx | cy | cz) >= 0) {
+                    const uint32_t slot = (uint32_t)(A.w + sx * (qx >> 2) + by_step * (qy >> 2) + bz_step * (qz >> 2));
+                    m = __ldg(P.bricks + slot);
+                    const int far4 = __ldg(P.bdir + (slot * 8u + oct));  // 4 cells per further brick of the cube
+                    // floor(left / 3); on the last iteration (left = -1) the box does not matter
+                    const int kmax = (int)__umulhi((unsigned)left, 0x55555556u);
+                    const int rx = ~qx & 3, ry = ~qy & 3, rz = ~qz & 3;
+                    kx = min(min(rx + far4, cx), kmax);
+                    ky = min(min(ry + far4, cy), kmax);
+                    kz = min(min(rz + far4, cz), kmax);
+                    ex = qx + kx; ey = qy + ky; ez = qz + kz;
+                    lb = left - (kx + ky + kz);
+                    bi = (rx + four * ry + sixteen * rz) ^ flip;
+                    result = ((m >> bi) & 1) ? T_HIT : T_LIVE;
+                }
+            }
+            if (result != T_LIVE) {
+                axis = bx ? 0 : (by ? 1 : 2);
+                cd = bx ? tx : (by ? ty : tz);
+                sgn = bx ? s.sx : (by ? s.sy : s.sz);
+                const int x = sx > 0 ? qx : 4 * L.BWp - 1 - qx, y = s.sy > 0 ? qy : 4 * L.BHp - 1 - qy,
+                          z = s.sz > 0 ? qz : 4 * L.BWp - 1 - qz;
+                hit_index = x + L.W * y + L.W * L.H * z;
+                break;
+            }
+            if (left < 0) { result = T_MISS; break; }  // entered a box on the last iteration
+        }
+        pred_fadd(tx, s.dx, bx);
+        pred_fadd(ty, s.dy, by);
+        pred_fadd(tz, s.dz, bz);
+    }
+    steps += left0 - left_end;  // left_end = left0 - 1 - (index of the breaking iteration)
+    return result;
+}
+
+// ray_setup of a ray whose direction lies in div_by's range along every axis and that starts
+// at 2^-60 <= o < 2^22 along each: the cell by a truncating add, reciprocals and quotients
+// without the IEEE routines' range tests.  False, with nothing usable in s, for any other ray.
+__device__ __forceinline__ bool ray_setup_lean(V3 o, V3 d, RaySetup& s) {
+    const V3 b{fadd(d.x, 0.000001f), fadd(d.y, 0.000001f), fadd(d.z, 0.000001f)};
+    const bool ok = all_within(d, kDivMinB, kDivMaxB) & all_within(b, kDivMinB, 2.5f) &
+                    (min3_nan(o.x, o.y, o.z) >= kDivMinA) & (max3_nan(o.x, o.y, o.z) < 4194304.0f);
+    s.sx = d.x > 0.0f ? 1 : -1; s.sy = d.y > 0.0f ? 1 : -1; s.sz = d.z > 0.0f ? 1 : -1;
+    s.dx = rcp_near(fabsf(b.x)); s.dy = rcp_near(fabsf(b.y)); s.dz = rcp_near(fabsf(b.z));
+    const float mx = __fadd_rz(o.x, 8388608.0f), my = __fadd_rz(o.y, 8388608.0f), mz = __fadd_rz(o.z, 8388608.0f);
+    s.cx = __float_as_int(mx) - 0x4B000000; s.cy = __float_as_int(my) - 0x4B000000; s.cz = __float_as_int(mz) - 0x4B000000;
+    s.tx = div_by(fsub(fsub(mx, s.sx > 0 ? 8388607.0f : 8388608.0f), o.x), d.x, rcp_near(d.x));
+    s.ty = div_by(fsub(fsub(my, s.sy > 0 ? 8388607.0f : 8388608.0f), o.y), d.y, rcp_near(d.y));
+    s.tz = div_by(fsub(fsub(mz, s.sz > 0 ? 8388607.0f : 8388608.0f), o.z), d.z, rcp_near(d.z));
+    return ok;
+}
+
+template <bool DF, bool COUNT>
+__device__ __forceinline__ int cast_ray(const MaskParams& P, const int2* alive, const int4* clip_k, const int4* oct_k,
+                                        V3 o, V3 d, int n, int maxSteps, float& cd, int& axis, int& sgn, int& steps,
+                                        int32_t& hit_index, unsigned& refills, V3& start_out) {
+    RaySetup s;
+    if (!DF && ray_setup_lean(o, d, s)) {
+        start_out = o;
+        return cast_lean<COUNT>(P, oct_k, s, n, maxSteps, cd, axis, sgn, steps, hit_index, refills);
+    }
+    ray_setup(o, d, s);
+    return cast_box<DF, COUNT>(P, alive, clip_k, s, o, d, n, maxSteps, cd, axis, sgn, steps, hit_index, refills, start_out);
+}
+
 __device__ __forceinline__ int view_of_tile(const MaskParams& P, int t) {
     if (P.nviews == 1) return 0;
     int lo = 0, hi = P.nviews - 1;
@@ -1188,16 +1321,14 @@ template <bool EXACT, bool DEBUG, bool DF>
 // 0.1727 ms under a minimum of 8 (64 registers), the stress camera 0.423 against 0.427 ms.
 __global__ void __launch_bounds__(128, 7) render_tiles_kernel(const __grid_constant__ MaskParams P) {
     __shared__ int2 alive[24];  // read by enter_box, i.e. only with depth-field words
-    __shared__ int4 clip_k[27];  // per sign code: the far-clip constants of enter_box_lean, and the octant
-    if (DF) fill_alive_ranges(alive, P, EXACT);
-    if (threadIdx.x < 27) {
-        const int t = threadIdx.x, sx = t % 3 - 1, sy = (t / 3) % 3 - 1, sz = t / 9 - 1;
-        int4 c;
-        c.x = sx > 0 ? P.cl[3] - 1 : (sx < 0 ? -P.cl[0] : INT_MAX);
-        c.y = sy > 0 ? P.cl[4] - 1 : (sy < 0 ? -P.cl[1] : INT_MAX);
-        c.z = sz > 0 ? P.cl[5] - 1 : (sz < 0 ? -P.cl[2] : INT_MAX);
-        c.w = (sx > 0) | ((sy > 0) << 1) | ((sz > 0) << 2);
-        clip_k[t] = c;
+    __shared__ int4 clip_s[27];  // enter_box's octants
+    __shared__ int4 oct_k[16];   // cast_lean's constants
+    const int4* clip_k = DF ? clip_s : P.clip_k;
+    if (DF) {
+        fill_alive_ranges(alive, P, EXACT);
+        if (threadIdx.x < 27) clip_s[threadIdx.x] = P.clip_k[threadIdx.x];
+    } else if (threadIdx.x < 16) {
+        oct_k[threadIdx.x] = P.oct_k[threadIdx.x];
     }
     __syncthreads();
     const int tile = (int)blockIdx.x + P.tile0;
@@ -1218,7 +1349,7 @@ __global__ void __launch_bounds__(128, 7) render_tiles_kernel(const __grid_const
     V3 from = cam, from2;  // the start a hit position is measured from (moved by depth-field jumps)
     if (valid) {
         rd = primary_dir(u, px, py, V.width, V.height, V.map.inv_w, V.map.inv_h);
-        pr = cast_box<DF, DEBUG>(P, alive, clip_k, cam, rd, u.maxSteps, u.maxSteps, cd, axis, sgn, steps, hit, refills, from);
+        pr = cast_ray<DF, DEBUG>(P, alive, clip_k, oct_k, cam, rd, u.maxSteps, u.maxSteps, cd, axis, sgn, steps, hit, refills, from);
         res.primary_steps = steps;
     }
     const bool lit = valid && pr == T_HIT && u.viewDepthField != 1;
@@ -1271,7 +1402,7 @@ __global__ void __launch_bounds__(128, 7) render_tiles_kernel(const __grid_const
                     }
                 }
                 if (cast) {
-                    const int sr = cast_box<DF, DEBUG>(P, alive, clip_k, add3(hp, mul3s(dir, 0.001f)), dir, n, u.maxSteps, c2, a2,
+                    const int sr = cast_ray<DF, DEBUG>(P, alive, clip_k, oct_k, add3(hp, mul3s(dir, 0.001f)), dir, n, u.maxSteps, c2, a2,
                                                 s2, steps, dummy, refills, from2);
                     const unsigned bit = 1u << (j + 1);
                     res.cast |= bit;
@@ -1485,6 +1616,23 @@ static int launch_tiles(const vrt_world* w, const ViewDev* h_views, int nviews, 
     for (int a = 0; a < 3; a++) {
         P.cl[a] = exact ? 0 : std::max(0, std::min(P.bb[a], dims[a]));
         P.cl[3 + a] = exact ? dims[a] : std::min(dims[a], std::max(P.bb[3 + a] + 1, P.cl[a]));
+    }
+    for (int t = 0; t < 27; t++) {
+        const int sx = t % 3 - 1, sy = (t / 3) % 3 - 1, sz = t / 9 - 1;
+        P.clip_k[t] = make_int4(sx > 0 ? P.cl[3] - 1 : (sx < 0 ? -P.cl[0] : INT_MAX),
+                                sy > 0 ? P.cl[4] - 1 : (sy < 0 ? -P.cl[1] : INT_MAX),
+                                sz > 0 ? P.cl[5] - 1 : (sz < 0 ? -P.cl[2] : INT_MAX),
+                                (sx > 0) | ((sy > 0) << 1) | ((sz > 0) << 2));
+    }
+    const int mx = 4 * P.L.BWp, my = 4 * P.L.BHp;
+    for (int o = 0; o < 8; o++) {
+        const bool x = o & 1, y = o & 2, z = o & 4;
+        P.oct_k[o] = make_int4(x ? P.cl[3] - 1 : mx - 1 - P.cl[0], y ? P.cl[4] - 1 : my - 1 - P.cl[1],
+                               z ? P.cl[5] - 1 : mx - 1 - P.cl[2],
+                               (x ? 0 : P.L.BWp - 1) + (y ? 0 : P.L.BWp * (P.L.BHp - 1)) +
+                                   (z ? 0 : P.L.BWp * P.L.BHp * (P.L.BWp - 1)));
+        P.oct_k[8 + o] = make_int4(x ? 0 : mx - P.L.W, y ? 0 : my - P.L.H, z ? 0 : mx - P.L.W,
+                                   (x ? 3 : 0) | (y ? 12 : 0) | (z ? 48 : 0));
     }
     // DEBUG launches store side outputs and count box lookups: any view with a debug output
     // or counters (whoever reads no more of the counters than rays, hits and pixels can do

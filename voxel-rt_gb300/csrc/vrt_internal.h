@@ -49,13 +49,16 @@ struct Layout {
 constexpr int kDistCap = 15;
 
 // Directed brick distances: 8 bytes per brick, stored like the brick masks.  Byte o
-// (octant o: bit a set = the + direction along axis a, x=0 y=1 z=2) is the capped
-// Chebyshev distance from the brick to the nearest non-empty brick n in that octant
-// (n_a >= b_a where bit a is set, n_a <= b_a where it is clear).  At distance d >= 1
+// (octant o: bit a set = the + direction along axis a, x=0 y=1 z=2) holds, as the
+// dist_code that a lookup adds to a box, the capped Chebyshev distance from the brick to
+// the nearest non-empty brick n in that octant (n_a >= b_a where bit a is set, n_a <= b_a
+// where it is clear).  At distance d >= 1
 // the cube of bricks from b to b + (d-1) in the octant's directions is empty: a ray
 // moving into that octant leaves its brick only through that cube's far faces, so the
 // cube bounds it as well as a centred cube of the same radius would, while solids
-// behind or beside the ray no longer shrink it.
+// behind or beside the ray no longer shrink it.  The code is the cells of the cube beyond the
+// brick itself: 4 (d - 1), and 0 for a non-empty brick.
+constexpr int dist_code(int d) { return d > 0 ? 4 * (d - 1) : 0; }
 
 __host__ __device__ inline uint64_t region_linear(const Layout& L, int rx, int ry, int rz) {
     return (uint64_t)rx + (uint64_t)L.RWp * ((uint64_t)ry + (uint64_t)L.RHp * rz);

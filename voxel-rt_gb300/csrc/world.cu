@@ -243,7 +243,7 @@ int vrt_world_create(int32_t width, int32_t height, vrt_world** out) {
     if (e == cudaSuccess) e = cudaMemset(w->d_bricks, 0, w->L.n_bricks * 8);
     if (e == cudaSuccess) e = cudaMemset(w->d_regions, 0, w->L.n_regions * 8);
     if (e == cudaSuccess) e = cudaMemset(w->d_supers, 0, w->L.n_supers * 8);
-    if (e == cudaSuccess) e = cudaMemset(w->d_bdir, kDistCap, w->L.n_bricks * 8);  // an all-air world
+    if (e == cudaSuccess) e = cudaMemset(w->d_bdir, dist_code(kDistCap), w->L.n_bricks * 8);  // an all-air world
     if (e == cudaSuccess) e = cudaMemset(w->d_rdist, kDistCap, rbytes);
     if (e == cudaSuccess) {  // an all-air world: empty box (min > max), no depth-field word
         const int empty[8] = {INT_MAX, INT_MAX, INT_MAX, INT_MIN, INT_MIN, INT_MIN, 0, 0};
@@ -371,12 +371,18 @@ int vrt_world_download_masks(const vrt_world* w, uint64_t* bricks, uint64_t* reg
 
 int vrt_world_download_distances(const vrt_world* w, uint8_t* brick_dir, uint8_t* region_dist, void* stream) {
     if (!w) return set_error(VRT_EINVAL, "NULL world");
-    if (brick_dir)
+    std::vector<uint64_t> masks;  // the stored codes are 0 for distances 0 and 1: the masks tell them apart
+    if (brick_dir) {
+        masks.resize(w->L.n_bricks);
         VRT_CUDA(cudaMemcpyAsync(brick_dir, w->d_bdir, w->L.n_bricks * 8, cudaMemcpyDeviceToHost, S(stream)));
+        VRT_CUDA(cudaMemcpyAsync(masks.data(), w->d_bricks, w->L.n_bricks * 8, cudaMemcpyDeviceToHost, S(stream)));
+    }
     if (region_dist)
         VRT_CUDA(cudaMemcpyAsync(region_dist, w->d_rdist, (uint64_t)w->L.RWp * w->L.RHp * w->L.RWp,
                                  cudaMemcpyDeviceToHost, S(stream)));
     VRT_CUDA(cudaStreamSynchronize(S(stream)));
+    for (size_t i = 0; i < masks.size(); i++)
+        for (int o = 0; o < 8; o++) brick_dir[8 * i + o] = masks[i] ? 0 : (uint8_t)(brick_dir[8 * i + o] / 4 + 1);
     return VRT_OK;
 }
 

@@ -392,8 +392,8 @@ __device__ void dir_tile(const NodePass& P, int tile, DirSmem& s) {
         const int word = xs ? 0 : 1;
         const bool plus = xs != 0;
         uint32_t cur = 0xffffffffu;
-        auto level = [&](int r, uint32_t e) {  // E_r: the nodes that end here have r - 1
-            add_planes(p, r - 1, cur & ~e);
+        auto level = [&](int r, uint32_t e) {  // E_r: the nodes that end here have D = r - 1
+            add_planes(p, r < 2 ? 0 : r - 2, cur & ~e);
             cur = e;
         };
         level(1, (uint32_t)(s.e1[lz * kDirYY + (ys ? 14 + ly : 21 - ly)] >> 16));
@@ -411,7 +411,7 @@ __device__ void dir_tile(const NodePass& P, int tile, DirSmem& s) {
         level(13, corners<15, 5>(e8, word, plus));
         level(14, corners<15, 6>(e8, word, plus));
         level(15, corners<15, 7>(e8, word, plus));
-        add_planes(p, kDistCap, cur);
+        add_planes(p, kDistCap - 1, cur);
     }
     uint4* planes = reinterpret_cast<uint4*>(s.nodes);  // [octant of this z direction][row]
     planes[(xs + 2 * ys) * 64 + (t & 63)] = p;
@@ -423,8 +423,8 @@ __device__ void dir_tile(const NodePass& P, int tile, DirSmem& s) {
 #pragma unroll
         for (int g = 0; g < 2; g++) {
             const int sh = 8 * seg + 4 * g;
-            const uint32_t a0 = plane_bytes(planes[row], sh), a1 = plane_bytes(planes[64 + row], sh);
-            const uint32_t a2 = plane_bytes(planes[128 + row], sh), a3 = plane_bytes(planes[192 + row], sh);
+            const uint32_t a0 = plane_bytes(planes[row], sh) << 2, a1 = plane_bytes(planes[64 + row], sh) << 2;
+            const uint32_t a2 = plane_bytes(planes[128 + row], sh) << 2, a3 = plane_bytes(planes[192 + row], sh) << 2;
             const uint32_t l0 = __byte_perm(a0, a1, 0x5140), l1 = __byte_perm(a2, a3, 0x5140);
             const uint32_t h0 = __byte_perm(a0, a1, 0x7362), h1 = __byte_perm(a2, a3, 0x7362);
             *reinterpret_cast<uint4*>(out + 32 * row + sh) =
