@@ -60,7 +60,7 @@ struct FixPass {
 
 struct NodePass {
     const uint64_t* regions;
-    uint32_t* bdir;              // directed distances, 4 octants to a word (the -z ones first)
+    uint16_t* bdir;              // directed distances, the two x directions of an octant pair to a value
     const uint64_t* supers;
     uint8_t* rdist;
     int* aabb;                   // solid box, then the depth-field flag
@@ -279,26 +279,27 @@ __device__ void fix_tile(const FixPass& P, int tile, FixSmem& s) {
 // up to 16 byte minima per brick and octant took 92 us for the 512 x 96 x 512 level, and
 // three more for the regions 19 us; this whole launch takes 19 us, bound by its instructions.)
 //
-// One tile: 32 x 8 x 8 bricks and the four octants of one z direction.  Rows are held as
-// 64-bit windows from 16 bricks before the tile, so no carry between words is needed: a
+// One tile: 32 x 8 x 8 bricks and the two octants of one y and one z direction.  Rows are held
+// as 64-bit windows from 16 bricks before the tile, so no carry between words is needed: a
 // window end spoils at most 14 bits, which end before the tile's own.  Smaller tiles in y and
-// z would read more halo (14 rows each), larger ones leave an edit's few tiles too long.
+// z would read more halo (14 rows each); four directions to a CTA made an edit's few tiles,
+// whose latency is the edit's, twice as long.
 
 constexpr int kDirRows = 22;  // 8 + 14 rows along the octant's y and z
-constexpr int kDirYY = 36;    // both y directions
-constexpr int kDirNodes = 16 * 10 * 6;
+constexpr int kDirNodes = 16 * 6 * 6;
 
 struct alignas(16) DirSmem {
     uint64_t nodes[kDirNodes];  // region masks; later the distance bit planes
-    uint64_t e1[kDirRows * kDirYY];
-    ulonglong2 e2[2][21 * 21];  // [y direction]: .x toward +x, .y toward -x; later the output
-    ulonglong2 e4[2][19 * 19];
-    ulonglong2 e8[2][15 * 15];
+    uint64_t e1[kDirRows * kDirRows];
+    ulonglong2 e2[21 * 21];  // .x toward +x, .y toward -x; later the output
+    ulonglong2 e4[19 * 19];
+    ulonglong2 e8[15 * 15];
 };
 
-// The 64-bit row window at row (py, pz) of 16 x 10 x n masks held in shared memory.
+// The 64-bit row window at row (py, pz) of 16 x NY x n masks held in shared memory.
+template <int NY>
 __device__ __forceinline__ uint64_t row_window(const uint32_t* n32, int py, int pz) {
-    const uint32_t* n = n32 + 2 * ((py >> 2) * 16 + (pz >> 2) * 160) + ((pz & 3) >> 1);
+    const uint32_t* n = n32 + 2 * ((py >> 2) * 16 + (pz >> 2) * 16 * NY) + ((pz & 3) >> 1);
     const int shift = 4 * (py & 3) + 16 * (pz & 1);
     uint64_t w = 0;
 #pragma unroll
@@ -338,105 +339,105 @@ __device__ __forceinline__ void add_planes(uint4& p, int r, uint32_t now) {
 
 __device__ void dir_tile(const NodePass& P, int tile, DirSmem& s) {
     const Layout& L = P.L;
-    const int zs = tile & 1;  // 1: toward +z
-    tile >>= 1;
+    const int ys = tile & 1, zs = tile >> 1 & 1;  // 1: toward +
+    tile >>= 2;
     const int x0 = (P.dx0 + tile % P.ndx) * 32, y0 = (P.dy0 + tile / P.ndx % P.ndy) * 8;
     const int z0 = (P.dz0 + tile / (P.ndx * P.ndy)) * 8;
     const int t = threadIdx.x;
 
     // the regions the tile and its halo span; beyond the grid everything is empty
-    const int rx0 = x0 / 4 - 4, ry0 = y0 / 4 - 4, rz0 = zs ? z0 / 4 : z0 / 4 - 4;
+    const int rx0 = x0 / 4 - 4, ry0 = y0 / 4 - (ys ? 0 : 4), rz0 = z0 / 4 - (zs ? 0 : 4);
     for (int i = t; i < kDirNodes; i += 256) {
-        const int rx = rx0 + (i & 15), ry = ry0 + (i >> 4) % 10, rz = rz0 + i / 160;
+        const int rx = rx0 + (i & 15), ry = ry0 + (i >> 4) % 6, rz = rz0 + i / 96;
         uint64_t m = 0;
         if (rx >= 0 && ry >= 0 && rz >= 0 && rx < L.RWp && ry < L.RHp && rz < L.RWp)
             m = P.regions[region_index(L, rx, ry, rz)];
         s.nodes[i] = m;
     }
     __syncthreads();
-    // E_1: rows yy = y - (y0 - 14), and lz along the z direction (0..7 the tile's own)
+    // E_1: rows (ly, lz) along the octants' directions, 0..7 the tile's own
     const uint32_t* n32 = reinterpret_cast<const uint32_t*>(s.nodes);
-    for (int i = t; i < kDirRows * kDirYY; i += 256) {
-        const int lz = i / kDirYY;
-        s.e1[i] = ~row_window(n32, i % kDirYY + 2, zs ? lz : 23 - lz);
+    for (int i = t; i < kDirRows * kDirRows; i += 256) {
+        const int ly = i % kDirRows, lz = i / kDirRows;
+        s.e1[i] = ~row_window<6>(n32, ys ? ly : 23 - ly, zs ? lz : 23 - lz);
     }
     __syncthreads();
-    for (int i = t; i < 2 * 21 * 21; i += 256) {
-        const int ys = i / 441, r = i % 441, ly = r % 21, lz = r / 21;
-        const int yy = ys ? 14 + ly : 21 - ly, step = ys ? 1 : -1;
-        const uint64_t* e = s.e1 + lz * kDirYY + yy;
-        const uint64_t v = e[0] & e[step] & e[kDirYY] & e[kDirYY + step];
-        s.e2[ys][r] = make_ulonglong2(v & v >> 1, v & v << 1);
+    for (int i = t; i < 21 * 21; i += 256) {
+        const uint64_t* e = s.e1 + i / 21 * kDirRows + i % 21;
+        const uint64_t v = e[0] & e[1] & e[kDirRows] & e[kDirRows + 1];
+        s.e2[i] = make_ulonglong2(v & v >> 1, v & v << 1);
     }
     __syncthreads();
-    for (int i = t; i < 2 * 19 * 19; i += 256) {
-        const int ys = i / 361, r = i % 361;
-        const ulonglong2 v = and4(&s.e2[ys][r % 19 + r / 19 * 21], 21, 2);
-        s.e4[ys][r] = make_ulonglong2(v.x & v.x >> 2, v.y & v.y << 2);
+    for (int i = t; i < 19 * 19; i += 256) {
+        const ulonglong2 v = and4(&s.e2[i % 19 + i / 19 * 21], 21, 2);
+        s.e4[i] = make_ulonglong2(v.x & v.x >> 2, v.y & v.y << 2);
     }
     __syncthreads();
-    for (int i = t; i < 2 * 15 * 15; i += 256) {
-        const int ys = i / 225, r = i % 225;
-        const ulonglong2 v = and4(&s.e4[ys][r % 15 + r / 15 * 19], 19, 4);
-        s.e8[ys][r] = make_ulonglong2(v.x & v.x >> 4, v.y & v.y << 4);
+    if (t < 15 * 15) {
+        const ulonglong2 v = and4(&s.e4[t % 15 + t / 15 * 19], 19, 4);
+        s.e8[t] = make_ulonglong2(v.x & v.x >> 4, v.y & v.y << 4);
     }
     __syncthreads();
-    // One of the tile's 64 rows, and one of the four octants, per thread
-    const int ya = t & 7, za = t >> 3 & 7, xs = t >> 6 & 1, ys = t >> 7;
-    uint4 p = make_uint4(0, 0, 0, 0);
+    // One of the tile's 64 rows, one of the two octants and the lower or upper half of the
+    // levels per thread
+    uint4* planes = reinterpret_cast<uint4*>(s.nodes);  // [half][x direction][row]
     {
+        const int ya = t & 7, za = t >> 3 & 7, xs = t >> 6 & 1, half = t >> 7;
         const int ly = ys ? ya : 7 - ya, lz = zs ? za : 7 - za;
-        const ulonglong2* e2 = &s.e2[ys][lz * 21 + ly];
-        const ulonglong2* e4 = &s.e4[ys][lz * 19 + ly];
-        const ulonglong2* e8 = &s.e8[ys][lz * 15 + ly];
+        const ulonglong2* e2 = s.e2 + lz * 21 + ly;
+        const ulonglong2* e4 = s.e4 + lz * 19 + ly;
+        const ulonglong2* e8 = s.e8 + lz * 15 + ly;
         const int word = xs ? 0 : 1;
         const bool plus = xs != 0;
+        uint4 p = make_uint4(0, 0, 0, 0);
         uint32_t cur = 0xffffffffu;
         auto level = [&](int r, uint32_t e) {  // E_r: the nodes that end here have D = r - 1
             add_planes(p, r < 2 ? 0 : r - 2, cur & ~e);
             cur = e;
         };
-        level(1, (uint32_t)(s.e1[lz * kDirYY + (ys ? 14 + ly : 21 - ly)] >> 16));
-        level(2, corners<21, 0>(e2, word, plus));
-        level(3, corners<21, 1>(e2, word, plus));
-        level(4, corners<19, 0>(e4, word, plus));
-        level(5, corners<19, 1>(e4, word, plus));
-        level(6, corners<19, 2>(e4, word, plus));
-        level(7, corners<19, 3>(e4, word, plus));
-        level(8, corners<15, 0>(e8, word, plus));
-        level(9, corners<15, 1>(e8, word, plus));
-        level(10, corners<15, 2>(e8, word, plus));
-        level(11, corners<15, 3>(e8, word, plus));
-        level(12, corners<15, 4>(e8, word, plus));
-        level(13, corners<15, 5>(e8, word, plus));
-        level(14, corners<15, 6>(e8, word, plus));
-        level(15, corners<15, 7>(e8, word, plus));
-        add_planes(p, kDistCap - 1, cur);
+        if (half == 0) {
+            level(1, (uint32_t)(s.e1[lz * kDirRows + ly] >> 16));
+            level(2, corners<21, 0>(e2, word, plus));
+            level(3, corners<21, 1>(e2, word, plus));
+            level(4, corners<19, 0>(e4, word, plus));
+            level(5, corners<19, 1>(e4, word, plus));
+            level(6, corners<19, 2>(e4, word, plus));
+            level(7, corners<19, 3>(e4, word, plus));
+            level(8, corners<15, 0>(e8, word, plus));
+        } else {
+            cur = corners<15, 0>(e8, word, plus);
+            level(9, corners<15, 1>(e8, word, plus));
+            level(10, corners<15, 2>(e8, word, plus));
+            level(11, corners<15, 3>(e8, word, plus));
+            level(12, corners<15, 4>(e8, word, plus));
+            level(13, corners<15, 5>(e8, word, plus));
+            level(14, corners<15, 6>(e8, word, plus));
+            level(15, corners<15, 7>(e8, word, plus));
+            add_planes(p, kDistCap - 1, cur);
+        }
+        planes[t] = p;
     }
-    uint4* planes = reinterpret_cast<uint4*>(s.nodes);  // [octant of this z direction][row]
-    planes[(xs + 2 * ys) * 64 + (t & 63)] = p;
     __syncthreads();
-    // planes -> one byte per octant: 8 bricks of one row per thread, four octants to a word
-    uint32_t* out = reinterpret_cast<uint32_t*>(s.e2);  // 64 rows x 32 bricks
+    // planes -> one byte per octant: 8 bricks of one row per thread, two octants to 16 bits
+    uint16_t* out = reinterpret_cast<uint16_t*>(s.e2);  // 64 rows x 32 bricks
     {
         const int row = t >> 2, seg = t & 3;
+        const uint4 u0 = planes[row], v0 = planes[128 + row], u1 = planes[64 + row], v1 = planes[192 + row];
+        const uint4 p0 = make_uint4(u0.x | v0.x, u0.y | v0.y, u0.z | v0.z, u0.w | v0.w);
+        const uint4 p1 = make_uint4(u1.x | v1.x, u1.y | v1.y, u1.z | v1.z, u1.w | v1.w);
 #pragma unroll
         for (int g = 0; g < 2; g++) {
             const int sh = 8 * seg + 4 * g;
-            const uint32_t a0 = plane_bytes(planes[row], sh) << 2, a1 = plane_bytes(planes[64 + row], sh) << 2;
-            const uint32_t a2 = plane_bytes(planes[128 + row], sh) << 2, a3 = plane_bytes(planes[192 + row], sh) << 2;
-            const uint32_t l0 = __byte_perm(a0, a1, 0x5140), l1 = __byte_perm(a2, a3, 0x5140);
-            const uint32_t h0 = __byte_perm(a0, a1, 0x7362), h1 = __byte_perm(a2, a3, 0x7362);
-            *reinterpret_cast<uint4*>(out + 32 * row + sh) =
-                make_uint4(__byte_perm(l0, l1, 0x5410), __byte_perm(l0, l1, 0x7632), __byte_perm(h0, h1, 0x5410),
-                           __byte_perm(h0, h1, 0x7632));
+            const uint32_t a0 = plane_bytes(p0, sh) << 2, a1 = plane_bytes(p1, sh) << 2;
+            *reinterpret_cast<uint2*>(out + 32 * row + sh) =
+                make_uint2(__byte_perm(a0, a1, 0x5140), __byte_perm(a0, a1, 0x7362));
         }
     }
     __syncthreads();
     const int lane = t & 31;
     if (x0 + lane < L.BWp)
         for (int row = t >> 5; row < 64; row += 8)  // BHp and BWp are multiples of 16: y and z lie in the grid
-            P.bdir[2 * brick_index(L, x0 + lane, y0 + (row & 7), z0 + (row >> 3)) + zs] = out[32 * row + lane];
+            P.bdir[4 * brick_index(L, x0 + lane, y0 + (row & 7), z0 + (row >> 3)) + ys + 2 * zs] = out[32 * row + lane];
 }
 
 // ------------------------------------------------------------------ region distances
@@ -464,28 +465,28 @@ __device__ __forceinline__ uint64_t cube_from(const uint64_t* e) {
     return v & v >> O;
 }
 
-// Whether the cube of radius K around the row's nodes is empty; (ly, lz) the row in the tile.
+// Whether the cube of radius K around the row's nodes is empty; (a, b) the row in the tile.
 template <int K>
-__device__ __forceinline__ uint32_t centred(const RegSmem& s, int ly, int lz) {
-    const int y = ly + 14 - K, z = lz + 14 - K;
+__device__ __forceinline__ uint32_t centred(const RegSmem& s, int a, int b) {
+    const int z = a + 14 - K, y = b + 14 - K;
     uint64_t v;
-    if constexpr (K == 0) v = s.e1[z * 36 + y];
-    else if constexpr (K < 2) v = cube_from<35, 2 * K + 1 - 2>(s.e2 + z * 35 + y);
-    else if constexpr (K < 4) v = cube_from<33, 2 * K + 1 - 4>(s.e4 + z * 33 + y);
-    else if constexpr (K < 8) v = cube_from<29, 2 * K + 1 - 8>(s.e8 + z * 29 + y);
-    else v = cube_from<21, 2 * K + 1 - 16>(s.e16 + z * 21 + y);
+    if constexpr (K == 0) v = s.e1[y * 36 + z];
+    else if constexpr (K < 2) v = cube_from<35, 2 * K + 1 - 2>(s.e2 + y * 35 + z);
+    else if constexpr (K < 4) v = cube_from<33, 2 * K + 1 - 4>(s.e4 + y * 33 + z);
+    else if constexpr (K < 8) v = cube_from<29, 2 * K + 1 - 8>(s.e8 + y * 29 + z);
+    else v = cube_from<21, 2 * K + 1 - 16>(s.e16 + y * 21 + z);
     return (uint32_t)(v >> (16 - K));
 }
 
 // The distances K0 .. K0 + 3 of a row
 template <int K0>
-__device__ __forceinline__ uint4 centred_planes(const RegSmem& s, int ly, int lz) {
+__device__ __forceinline__ uint4 centred_planes(const RegSmem& s, int a0, int b0) {
     uint4 p = make_uint4(0, 0, 0, 0);
     uint32_t prev = 0xffffffffu;
-    if constexpr (K0 > 0) prev = centred<K0 - 1>(s, ly, lz);
-    const uint32_t a = centred<K0>(s, ly, lz), b = centred<K0 + 1>(s, ly, lz), c = centred<K0 + 2>(s, ly, lz);
+    if constexpr (K0 > 0) prev = centred<K0 - 1>(s, a0, b0);
+    const uint32_t a = centred<K0>(s, a0, b0), b = centred<K0 + 1>(s, a0, b0), c = centred<K0 + 2>(s, a0, b0);
     uint32_t d = 0;  // 15: "15 or more"
-    if constexpr (K0 + 3 < kDistCap) d = centred<K0 + 3>(s, ly, lz);
+    if constexpr (K0 + 3 < kDistCap) d = centred<K0 + 3>(s, a0, b0);
     add_planes(p, K0, prev & ~a);
     add_planes(p, K0 + 1, a & ~b);
     add_planes(p, K0 + 2, b & ~c);
@@ -493,9 +494,11 @@ __device__ __forceinline__ uint4 centred_planes(const RegSmem& s, int ly, int lz
     return p;
 }
 
+// E of side 2 STEP from E of side STEP; a thread keeps its place z along a row of the plane.
 template <int N, int PREV, int STEP>
-__device__ __forceinline__ void cube_level(uint64_t* out, const uint64_t* in) {
-    for (int i = threadIdx.x; i < N * N; i += 256) out[i] = cube_from<PREV, STEP>(in + i / N * PREV + i % N);
+__device__ __forceinline__ void cube_level(uint64_t* out, const uint64_t* in, int z, int y0) {
+    if (z < N)
+        for (int y = y0; y < N; y += 7) out[y * N + z] = cube_from<PREV, STEP>(in + y * PREV + z);
     __syncthreads();
 }
 
@@ -515,24 +518,30 @@ __device__ void region_tile(const NodePass& P, int tile, RegSmem& s) {
     }
     __syncthreads();
     const uint32_t* n32 = reinterpret_cast<const uint32_t*>(s.nodes);
-    for (int i = t; i < 36 * 36; i += 256) s.e1[i] = ~row_window(n32, i % 36 + 2, i / 36 + 2);
+    // 36 threads along z, 7 rows of them along y (4 threads idle); rows beyond the grid in y, more
+    // than half of them in flat worlds, are skipped by whole warps
+    const int tz = t % 36, ty = t / 36;
+    if (ty < 7)
+        for (int y = ty; y < 36; y += 7)
+            s.e1[y * 36 + tz] = (unsigned)(y0 - 14 + y) < (unsigned)L.RHp ? ~row_window<10>(n32, y + 2, tz + 2) : ~0ull;
     (&s.planes[0][0])[t] = 0;
     __syncthreads();
-    cube_level<35, 36, 1>(s.e2, s.e1);
-    cube_level<33, 35, 2>(s.e4, s.e2);
-    cube_level<29, 33, 4>(s.e8, s.e4);
-    cube_level<21, 29, 8>(s.e16, s.e8);
-    const int row = t & 63, ly = row & 7, lz = row >> 3;
+    const int first = ty < 7 ? ty : 99;
+    cube_level<35, 36, 1>(s.e2, s.e1, tz, first);
+    cube_level<33, 35, 2>(s.e4, s.e2, tz, first);
+    cube_level<29, 33, 4>(s.e8, s.e4, tz, first);
+    cube_level<21, 29, 8>(s.e16, s.e8, tz, first);
+    const int row = t & 63, lz = row & 7, ly = row >> 3;
     const int part = t >> 6;  // four distances of the row each; warp-uniform
-    const uint4 p = part == 0 ? centred_planes<0>(s, ly, lz)
-                              : (part == 1 ? centred_planes<4>(s, ly, lz)
-                                           : (part == 2 ? centred_planes<8>(s, ly, lz) : centred_planes<12>(s, ly, lz)));
+    const uint4 p = part == 0 ? centred_planes<0>(s, lz, ly)
+                              : (part == 1 ? centred_planes<4>(s, lz, ly)
+                                           : (part == 2 ? centred_planes<8>(s, lz, ly) : centred_planes<12>(s, lz, ly)));
     atomicOr(&s.planes[row][0], p.x);
     atomicOr(&s.planes[row][1], p.y);
     atomicOr(&s.planes[row][2], p.z);
     atomicOr(&s.planes[row][3], p.w);
     __syncthreads();
-    const int r2 = t >> 2, y = y0 + (r2 & 7), z = z0 + (r2 >> 3);
+    const int r2 = t >> 2, z = z0 + (r2 & 7), y = y0 + (r2 >> 3);
     const uint4 q = *reinterpret_cast<const uint4*>(s.planes[r2]);
     for (int g = 0; g < 2; g++) {
         const int sh = 8 * (t & 3) + 4 * g;  // RWp is a multiple of 4: all four regions or none
@@ -832,7 +841,7 @@ static void node_tiles(NodePass& P, const int b[6]) {
     }
     P.dx0 = lo[0] >> 5; P.ndx = ((hi[0] + 31) >> 5) - P.dx0;
     P.dy0 = lo[1] >> 3; P.ndy = ((hi[1] + 7) >> 3) - P.dy0;
-    P.dz0 = lo[2] >> 3; P.n_dir = 2 * P.ndx * P.ndy * (((hi[2] + 7) >> 3) - P.dz0);
+    P.dz0 = lo[2] >> 3; P.n_dir = 4 * P.ndx * P.ndy * (((hi[2] + 7) >> 3) - P.dz0);
     P.rx0 = rlo[0] >> 5; P.nrx = ((rhi[0] + 31) >> 5) - P.rx0;
     P.ry0 = rlo[1] >> 3; P.nry = ((rhi[1] + 7) >> 3) - P.ry0;
     P.rz0 = rlo[2] >> 3; P.n_reg = P.nrx * P.nry * (((rhi[2] + 7) >> 3) - P.rz0);
@@ -908,7 +917,7 @@ int change_words(vrt_world* w, const WordChange& c, cudaStream_t s) {
     NodePass N{};
     N.L = L;
     N.regions = w->d_regions;
-    N.bdir = reinterpret_cast<uint32_t*>(w->d_bdir);
+    N.bdir = reinterpret_cast<uint16_t*>(w->d_bdir);
     N.supers = w->d_supers;
     N.rdist = w->d_rdist;
     N.aabb = w->d_aabb;
@@ -956,7 +965,7 @@ int refresh_stop_masks(vrt_world* w, cudaStream_t s) {
     N.L = L;
     node_tiles(N, b);
     N.regions = w->d_stop_regions;
-    N.bdir = reinterpret_cast<uint32_t*>(w->d_sdir);
+    N.bdir = reinterpret_cast<uint16_t*>(w->d_sdir);
     N.n_reg = 0;
     return run_node_pass(N, s);
 }
