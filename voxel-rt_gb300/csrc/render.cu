@@ -204,28 +204,35 @@ struct WordRay {
 // true.  (Only y: in terrain worlds the solid box spans x and z, and two registers per
 // ray are what this latency-bound kernel can spare.)
 //
-// What bounds it: instruction issue (72 % of the slots while an SM is busy), 52 M warp
+// What bounds it: instruction issue (75 % of the slots while an SM is busy), 49 M warp
 // instructions for an 800x600 frame of the level with three lights.  An iteration is about 40
 // instructions, a jump 45 more, a ray's set-up and shading 400.  The jump's three IEEE
-// divisions as div_by, the intersect adds left to the iterations that do not jump, and no
-// prefetch of the words ahead (24 instructions in each iteration, once worth it for its long
-// dependent chain): that frame 77.7 -> 66.6 us, the app's first frame 67.2 -> 60.3 us (of
-// which the divisions alone are nothing and the prefetch 8 us).  Tried without gain: 8x4 tiles
-// of the words instead of the second copy (96 us on the app's first frame), both copies' loads
-// predicated (75.7), 5 to 8 CTAs per SM by fewer registers (67.0-69.3), one warp per CTA (63.6
-// against 60.3 us with 16x8 tiles).
+// divisions as div_by and no prefetch of the words ahead (24 instructions in each iteration,
+// once worth it for its long dependent chain): that frame 77.7 -> 66.6 us, the app's first
+// frame 67.2 -> 60.3 us (of which the divisions alone are nothing and the prefetch 8 us).  The
+// intersect adds in the shadow of the load, and not behind it for the iterations that turn out
+// not to jump: 67.2 -> 62.7 and 59.9 -> 54.1 us; the ray's six reciprocals by rcp_near: 61.8
+// and 53.7 us.  Tried without gain: 8x4 tiles of the words instead of the second copy (96 us on
+// the app's first frame), both copies' loads predicated (75.7 then; one load with a predicated
+// address now: 61.5 and 53.9), the hit's results taken after the loop (62.1 and 56.1), 5 to 8
+// CTAs per SM by fewer registers (67.0-69.3 of 66.6), one warp per CTA (63.6 of 60.3 us with
+// 16x8 tiles).
 __device__ WordRay cast_word(const Layout& L, const WordParams& p, V3 start, V3 dir, int dist, int maxSteps) {
     WordRay o;
     o.hit = -1; o.cd = 0.0f; o.axis = 2; o.s = 0; o.steps = 0;
     RaySetup r;
     // The divisions by the ray's direction, here and at each jump: see div_by.
-    const V3 inv{frcp(dir.x), frcp(dir.y), frcp(dir.z)};
+    const V3 b{fadd(dir.x, 0.000001f), fadd(dir.y, 0.000001f), fadd(dir.z, 0.000001f)};
     const float lo = min3_nan(start.x, start.y, start.z);
-    const bool fast = all_within(dir, kDivMinB, kDivMaxB) & (lo == lo);
+    const bool fast = all_within(dir, kDivMinB, kDivMaxB) & all_within(b, kDivMinB, 2.5f) & (lo == lo);
     r.sx = isign(dir.x); r.sy = isign(dir.y); r.sz = isign(dir.z);
-    r.dx = frcp(fabsf(fadd(dir.x, 0.000001f)));
-    r.dy = frcp(fabsf(fadd(dir.y, 0.000001f)));
-    r.dz = frcp(fabsf(fadd(dir.z, 0.000001f)));
+    V3 inv{0.0f, 0.0f, 0.0f};
+    if (fast) {
+        inv = V3{rcp_near(dir.x), rcp_near(dir.y), rcp_near(dir.z)};
+        r.dx = rcp_near(fabsf(b.x)); r.dy = rcp_near(fabsf(b.y)); r.dz = rcp_near(fabsf(b.z));
+    } else {
+        r.dx = frcp(fabsf(b.x)); r.dy = frcp(fabsf(b.y)); r.dz = frcp(fabsf(b.z));
+    }
     enter_cell(r, start, dir, inv, fast);
     int lo_y = 0, span_y = L.H;
     if (!p.exact) {
@@ -250,6 +257,12 @@ __device__ WordRay cast_word(const Layout& L, const WordParams& p, V3 start, V3 
         if (bx) r.cx += r.sx;
         if (by) r.cy += r.sy;
         if (bz) r.cz += r.sz;
+        // The intersect moves on before the word is there: the adds run in the load's shadow,
+        // and a jump, which they don't concern, sets all three anew.
+        const float cd = bx ? r.tx : (by ? r.ty : r.tz);
+        pred_fadd(r.tx, r.dx, bx);
+        pred_fadd(r.ty, r.dy, by);
+        pred_fadd(r.tz, r.dz, bz);
         // Outside the world (getVoxelIndex == -1), or no solid voxel ahead: the ray ends as at a
         // solid voxel (word 0), without a hit.
         const bool in = ((unsigned)r.cx < (unsigned)L.W) & ((unsigned)(r.cy - lo_y) < (unsigned)span_y) &
@@ -260,9 +273,7 @@ __device__ WordRay cast_word(const Layout& L, const WordParams& p, V3 start, V3 
         // ray along z for hundreds of steps, which set the frame's length.
         int32_t v = 0;
         if (in) v = __ldg((bz ? p.words_z : p.words) + ((bz ? r.cz : r.cx) + W * r.cy + WH * (bz ? r.cx : r.cz)));
-        const bool plain = v == -1;
-        if (!plain) {
-            const float cd = bx ? r.tx : (by ? r.ty : r.tz);
+        if (v != -1) {
             if (v >= 0) {
                 if (in) {
                     o.hit = r.cx + W * r.cy + WH * r.cz;
@@ -279,9 +290,6 @@ __device__ WordRay cast_word(const Layout& L, const WordParams& p, V3 start, V3 
             start = add3(mul3s(dir, fadd(cd, toJump)), start);
             enter_cell(r, start, dir, inv, fast);
         }
-        pred_fadd(r.tx, r.dx, bx & plain);
-        pred_fadd(r.ty, r.dy, by & plain);
-        pred_fadd(r.tz, r.dz, bz & plain);
     }
     return o;
 }
