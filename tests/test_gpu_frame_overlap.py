@@ -1,0 +1,165 @@
+"""Frames in a row on one stream, where the next one may begin before the last has ended:
+each leaves its own image, side outputs and counters, whatever is put between two of them."""
+import numpy as np
+import pytest
+
+import vrt
+from helpers import make_world
+
+pytestmark = pytest.mark.gpu
+
+W, H = 96, 64
+
+
+def scene(jumps):
+    rng = np.random.default_rng(5)
+    words = np.where(rng.random(W * H * W) < 0.004, 0x01000000 | rng.integers(0, 1 << 24, W * H * W), -1).astype(np.int32)
+    words.reshape(W, H, W)[:, :3, :] = 0x01808080
+    w = make_world(words, W, H)
+    if jumps:
+        w.fix_depth_field()
+    return w
+
+
+def views(n, steps=300):
+    us = []
+    for i in range(n):
+        u = vrt.default_uniforms()
+        u.camPos[:] = (20.3 + i, 12.6 + 3 * (i % 5), 19.7)
+        u.rotateMatrix[:] = vrt.rotate_matrix(0.1 * (i % 4), 0.9 * i)
+        u.lightPos[:] = [20.0 + 5 * i, 120.0, 3.0]
+        u.maxSteps = steps
+        u.aspectRatio = 1.0
+        us.append(u)
+    return us
+
+
+def frame(torch, r, w, u, width, height, kernel, out, stream, stats=None):
+    opts = vrt.RenderOpts()
+    opts.kernel = kernel
+    r.render(w, u, width, height, out.data_ptr(), None, stats.data_ptr() if stats is not None else 0, opts, stream)
+
+
+def alone(torch, w, u, width, height, kernel):
+    out = torch.zeros(width * height * 4, dtype=torch.uint8, device="cuda")
+    stats = torch.zeros(vrt.STAT_COUNT, dtype=torch.int64, device="cuda")
+    frame(torch, vrt.Renderer(), w, u, width, height, kernel, out, torch.cuda.current_stream().cuda_stream, stats)
+    torch.cuda.synchronize()
+    return out.cpu(), stats.cpu()[:4]
+
+
+# a grid of one CTA, one that fits at once, and one several times as large
+@pytest.mark.parametrize("size", [(5, 3), (320, 200), (1501, 700)])
+@pytest.mark.parametrize("kernel,jumps", [(vrt.KERNEL_MASK_PIXEL, False), (vrt.KERNEL_MASK_PIXEL, True),
+                                          (vrt.KERNEL_WORD, True)])
+@pytest.mark.parametrize("own_stream", [False, True])
+def test_frames_in_a_row(cuda, size, kernel, jumps, own_stream):
+    torch = pytest.importorskip("torch")
+    w, us = scene(jumps), views(6)
+    n = size[0] * size[1] * 4
+    expect = [alone(torch, w, u, *size, kernel) for u in us]
+    s = torch.cuda.Stream() if own_stream else torch.cuda.current_stream()
+    side = torch.cuda.Stream()
+    r = vrt.Renderer()
+    img = torch.zeros(n, dtype=torch.uint8, device="cuda")
+    host = [torch.zeros(n, dtype=torch.uint8).pin_memory() for _ in range(40)]
+    copies, stats = [], torch.zeros(vrt.STAT_COUNT, dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        order = []
+        for k in range(40):  # one image: copied away by the copy engine, a kernel, another stream, or overwritten
+            i = (k * k + k // 7) % 6
+            order.append(i)
+            frame(torch, r, w, us[i], *size, kernel, img, s.cuda_stream, stats)
+            if k % 4 == 0:
+                host[k].copy_(img, non_blocking=True)
+            elif k % 4 == 1:
+                copies.append((i, img.clone()))
+            elif k % 4 == 2:
+                ev = s.record_event()
+                side.wait_event(ev)
+                with torch.cuda.stream(side):
+                    torch.cuda._sleep(200000)
+                    copies.append((i, img.clone()))
+                    done = side.record_event()
+                s.wait_event(done)
+    torch.cuda.synchronize()
+    for k in range(0, 40, 4):
+        assert torch.equal(host[k], expect[order[k]][0]), k
+    for i, c in copies:
+        assert torch.equal(c.cpu(), expect[i][0])
+    assert torch.equal(img.cpu(), expect[order[-1]][0])
+    assert torch.equal(stats.cpu()[:4], sum(expect[i][1] for i in order))
+
+
+@pytest.mark.parametrize("kernel,jumps", [(vrt.KERNEL_MASK_PIXEL, False), (vrt.KERNEL_MASK_PIXEL, True),
+                                          (vrt.KERNEL_WORD, True)])
+def test_changes_between_frames(cuda, kernel, jumps):
+    """Edits, uploads and other worlds between frames: no frame sees a change from behind it
+    or misses one ahead of it."""
+    torch = pytest.importorskip("torch")
+    size = (1301, 700)
+    us = views(3)
+    n = size[0] * size[1] * 4
+    s = torch.cuda.current_stream().cuda_stream
+
+    def run(together):
+        w, other = scene(jumps), scene(not jumps if kernel == vrt.KERNEL_MASK_PIXEL else jumps)
+        r = vrt.Renderer()
+        imgs = [torch.zeros(n, dtype=torch.uint8, device="cuda") for _ in range(24)]
+        row = torch.full((W,), 0x01ff0000, dtype=torch.int32, device="cuda")
+        for k, img in enumerate(imgs):
+            if not together:
+                torch.cuda.synchronize()
+                r = vrt.Renderer()
+            frame(torch, r, other if k % 5 == 3 else w, us[k % 3], *size, kernel, img, s)
+            if not together:
+                torch.cuda.synchronize()
+            if k % 3 == 1:
+                w.remove_sphere(10 + 3 * k, 3, 30 + k, 6, 1 if jumps else 0)
+            if k % 8 == 6:
+                w.place_voxel(20 + k, 20, 30, 0x0100ff00)
+            if k == 13:
+                w.upload_device(row.data_ptr(), 5 * W, W)
+        torch.cuda.synchronize()
+        return [i.cpu() for i in imgs]
+
+    for k, (a, b) in enumerate(zip(run(True), run(False))):
+        assert torch.equal(a, b), k
+
+
+def test_captured_frames(cuda):
+    """A captured frame replays alone, after its renderer is gone, between frames of others."""
+    torch = pytest.importorskip("torch")
+    size, us, kernel = (801, 600), views(3), vrt.KERNEL_MASK_PIXEL
+    n = size[0] * size[1] * 4
+    w = scene(False)
+    expect = [alone(torch, w, u, *size, kernel)[0] for u in us]
+    img = torch.zeros(n, dtype=torch.uint8, device="cuda")
+    out = torch.zeros(n, dtype=torch.uint8, device="cuda")
+    r, gone, s = vrt.Renderer(), vrt.Renderer(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        frame(torch, r, w, us[0], *size, kernel, img, s.cuda_stream)
+        frame(torch, gone, w, us[0], *size, kernel, img, s.cuda_stream)
+        s.synchronize()
+        g = torch.cuda.CUDAGraph()
+        g.capture_begin()
+        frame(torch, gone, w, us[1], *size, kernel, out, s.cuda_stream)
+        g.capture_end()
+        s.synchronize()
+        gone.close()
+        kept = []
+        for k in range(40):
+            frame(torch, r, w, us[k % 3], *size, kernel, img, s.cuda_stream)
+            kept.append(img.clone())
+            out.zero_()
+            g.replay()
+            kept.append(out.clone())
+            frame(torch, r, w, us[k % 2], *size, kernel, img, s.cuda_stream)
+            g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(img.cpu(), expect[39 % 2])
+    for k in range(40):
+        assert torch.equal(kept[2 * k].cpu(), expect[k % 3]), k
+        assert torch.equal(kept[2 * k + 1].cpu(), expect[1]), k

@@ -98,6 +98,7 @@ struct WordParams {
 // order changes no result, only when each tile runs.  No kernel or host work is added:
 // the lists are written and read by the render kernels themselves.
 constexpr int kTileClasses = 16;
+constexpr int kClassReuses = 31;  // overlapped frames that may go by one frame's classes
 
 // Costs 0-7 -> class 0, 8-11 -> 1, 12-15 -> 2, 16-23 -> 3, ..., 768-1023 -> 14, >= 1024 -> 15.
 __device__ __forceinline__ int tile_class(int cost) {
@@ -300,6 +301,7 @@ template <bool DEBUG>
 __global__ void __launch_bounds__(128, 4) render_word_kernel(const int32_t* __restrict__ words, Layout L,
                                                           const __grid_constant__ WordParams p) {
     __shared__ int s_cost, s_done, s_tile;
+    cudaTriggerProgrammaticLaunchCompletion();  // see frame_launch
     if (threadIdx.x < 32) {
         const int b = (int)(blockIdx.x + gridDim.x * blockIdx.y), lane = threadIdx.x;
         int tile = b;
@@ -405,6 +407,9 @@ __global__ void __launch_bounds__(128, 4) render_word_kernel(const int32_t* __re
         }
         res.mr = mr; res.mg = mg; res.mb = mb;
         res.rgba = pack_color_tab(u, pr.hit >= 0, word, mr, mg, mb, pr.steps);
+    }
+    cudaGridDependencySynchronize();  // nothing is written before the frame ahead has ended
+    if (valid) {
         if (DEBUG) store_pixel(p.dbg, p.rgba, (uint64_t)py * p.width + px, res);
         else reinterpret_cast<uint32_t*>(p.rgba)[(uint64_t)py * p.width + px] = res.rgba;
     }
@@ -1323,14 +1328,15 @@ __device__ __forceinline__ int view_of_tile(const MaskParams& P, int t) {
 // and count box lookups; DF launches render a world with depth-field words (the masks are
 // its stop masks).
 template <bool EXACT, bool DEBUG, bool DF>
-// A minimum of 7 CTAs of 128 threads per SM lets the compiler use up to 73 registers.  It
-// takes 63 for the timed variant (so 8 CTAs still fit per SM) and 69 for the debug ones,
-// and the code it makes for the unrolled loop runs the 1080p frame in 0.1706 ms against
-// 0.1727 ms under a minimum of 8 (64 registers), the stress camera 0.423 against 0.427 ms.
+// A minimum of 7 CTAs of 128 threads per SM lets the compiler use up to 73 registers; it takes
+// 63 or 64 for every variant (so 8 CTAs still fit per SM), and the code it makes for the
+// unrolled loop is faster than under a minimum of 8 (1080p frame 0.1706 against 0.1727 ms, the
+// stress camera 0.423 against 0.427 ms when measured).
 __global__ void __launch_bounds__(128, 7) render_tiles_kernel(const __grid_constant__ MaskParams P) {
     __shared__ int2 alive[24];  // read by enter_box, i.e. only with depth-field words
     __shared__ int4 clip_s[27];  // enter_box's octants
     __shared__ int4 oct_k[16];   // cast_lean's constants
+    cudaTriggerProgrammaticLaunchCompletion();  // see frame_launch
     const int4* clip_k = DF ? clip_s : P.clip_k;
     if (DF) {
         fill_alive_ranges(alive, P, EXACT);
@@ -1442,6 +1448,9 @@ __global__ void __launch_bounds__(128, 7) render_tiles_kernel(const __grid_const
         res.steps = steps;
         res.mr = mr; res.mg = mg; res.mb = mb;
         res.rgba = pack_color_tab(u, pr == T_HIT, word, mr, mg, mb, res.primary_steps);
+    }
+    cudaGridDependencySynchronize();  // nothing is written before the frame ahead has ended
+    if (valid) {
         if (DEBUG) store_pixel(V.dbg, V.rgba, (uint64_t)py * V.width + px, res);
         else reinterpret_cast<uint32_t*>(V.rgba)[(uint64_t)py * V.width + px] = res.rgba;
     }
@@ -1505,7 +1514,12 @@ struct vrt_renderer {
     int* d_class_list = nullptr;
     int tile_cap = 0;
     int tile_gx = 0, tile_gy = 0;         // the grid of the frames recorded (0: none)
-    uint64_t tile_frames = 0;             // word-kernel frames launched on that grid
+    uint64_t tile_frames = 0;             // word-kernel frames that recorded classes on that grid
+    int tile_reuses = 0;                  // frames since then that went by the same classes
+    // the last frame's world (its stamp) and stream: see frame_launch
+    std::mutex seen_mu;
+    uint64_t seen_stamp = 0;
+    cudaStream_t seen_stream = nullptr;
 };
 
 struct vrt_batch_graph {
@@ -1601,10 +1615,56 @@ static int launch_mask(vrt_renderer* r, const vrt_world* w, const ViewDev* h_vie
     return VRT_OK;
 }
 
+// How a frame's kernel is launched.  A frame is bound by its longest chains: the SMs stand idle
+// from where the first runs out of tiles to the next launch, 5 % of a 1080p frame, 11 % of a
+// 4K frame along the ground, 15 of the 54 us of the app's first frame, 4 of the 13 us of a
+// 256x256 one, and 2 us of launch each.  So a frame of the world that the stream's last frame
+// showed, unchanged since (its stamp), is a programmatic dependent of that one: its CTAs begin
+// as soon as all of the frame ahead have begun.  What they read was there before both frames;
+// what they write waits for the end of the frame ahead (cudaGridDependencySynchronize, behind the
+// trace), so images, counters and whatever follows on the stream see the frames one after the
+// other.  Frames in a row, each alone before: 256x256 16.9 -> 7.4 us, 1080p 192.5 -> 184.2, 4K
+// 551 -> 544 (the CTAs that wait hold their places), the app's first frame 58.9 -> 38.4, the
+// 800x600 level frame with three lights 65.8 -> 47.8 us.
+// A captured launch is a plain one, and is not taken for the stream's last frame; the streams
+// of cudaStreamPerThread share a handle, so theirs are plain too.
+enum { kPlainFrame, kOverlappedFrame, kCapturedFrame };
+static int frame_launch(vrt_renderer* r, const vrt_world* w, cudaStream_t s) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return kCapturedFrame;
+    }
+    if (w->stamp == 0 || s == cudaStreamPerThread) return kPlainFrame;
+    std::lock_guard<std::mutex> lock(r->seen_mu);
+    return r->seen_stamp == w->stamp && r->seen_stream == s ? kOverlappedFrame : kPlainFrame;
+}
+
+template <class... Params, class... Args>
+static cudaError_t launch_frame(vrt_renderer* r, const vrt_world* w, int how, void (*kern)(Params...), dim3 grid,
+                                int threads, cudaStream_t s, const Args&... args) {
+    cudaLaunchAttribute pdl{};
+    pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    pdl.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.stream = s;
+    cfg.attrs = &pdl;
+    cfg.numAttrs = how == kOverlappedFrame ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
+    if (how != kCapturedFrame) {
+        std::lock_guard<std::mutex> lock(r->seen_mu);
+        r->seen_stamp = e == cudaSuccess ? w->stamp : 0;
+        r->seen_stream = s;
+    }
+    return e;
+}
+
 // Tile kernel launch over the views' tile space (1 view: h_views[0] as a parameter).
 static int launch_tiles(const vrt_world* w, const ViewDev* h_views, int nviews, int total_tiles,
                         const ViewDev* d_views, int threads, cudaStream_t s, int tile0 = 0, int ntiles = -1,
-                        bool count_lookups = true) {
+                        bool count_lookups = true, vrt_renderer* frame_of = nullptr) {
     MaskParams P;
     std::memset(&P, 0, sizeof(P));
     P.words = w->d_words;
@@ -1668,6 +1728,10 @@ static int launch_tiles(const vrt_world* w, const ViewDev* h_views, int nviews, 
     const Kern kern = kernels[exact][debug][df];
     P.tile0 = tile0;
     if (ntiles < 0) ntiles = total_tiles - tile0;
+    if (frame_of) {  // a renderer's whole frame
+        VRT_CUDA(launch_frame(frame_of, w, frame_launch(frame_of, w, s), kern, dim3(ntiles), threads, s, P));
+        return VRT_OK;
+    }
     if (ntiles > 0) kern<<<ntiles, threads, 0, s>>>(P);
     VRT_CUDA(cudaGetLastError());
     return VRT_OK;
@@ -1762,9 +1826,13 @@ int vrt_renderer_destroy(vrt_renderer* r) {
 // The tile-order buffers of a word-kernel launch over grid g.  Frame f of a grid reads the
 // classes frame f-1 wrote (count buffer f%3, lists f%2), appends to count buffer (f+1)%3
 // and lists (f+1)%2, and clears count buffer (f+2)%3 for frame f+1: that buffer was last
-// read by frame f-1, which ended before frame f began (one stream per renderer).  The
-// order only speeds frames up: without room for its buffers the launch runs in row order.
-static int word_tile_order(vrt_renderer* r, dim3 g, cudaStream_t s, WordParams* p) {
+// read by frame f-1, which ended before frame f began (one stream per renderer).  These are the
+// frames that begin when all before has ended.  One that overlaps the frame ahead goes by the
+// same classes as the last of these, which are not written to until the next, and records
+// none; every 32nd frame at least is a whole one, so that the classes follow a moving camera.
+// The order only speeds frames up: without room for its buffers, and captured into a graph
+// (whose runs would append to the same lists), the launch runs in row order.
+static int word_tile_order(vrt_renderer* r, dim3 g, cudaStream_t s, int* how, WordParams* p) {
     const int nt = (int)(g.x * g.y);
     p->tiles = nt;
     p->class_count_in = nullptr;
@@ -1772,6 +1840,7 @@ static int word_tile_order(vrt_renderer* r, dim3 g, cudaStream_t s, WordParams* 
     p->class_count_out = nullptr;
     p->class_list_out = nullptr;
     p->class_count_clear = nullptr;
+    if (*how == kCapturedFrame) return VRT_OK;
     if (nt > r->tile_cap) {
         cudaFree(r->d_class_count);
         cudaFree(r->d_class_list);
@@ -1797,12 +1866,15 @@ static int word_tile_order(vrt_renderer* r, dim3 g, cudaStream_t s, WordParams* 
         r->tile_gy = (int)g.y;
         r->tile_frames = 0;
     }
-    const uint64_t f = r->tile_frames;
     int* counts = r->d_class_count;
     int* lists = r->d_class_list;
     const size_t list = (size_t)kTileClasses * nt;
+    if (*how == kOverlappedFrame && (r->tile_frames < 2 || r->tile_reuses >= kClassReuses)) *how = kPlainFrame;
+    // an overlapped frame reads what the last plain one read, which was whole before that one began
+    const uint64_t f = *how == kOverlappedFrame ? r->tile_frames - 1 : r->tile_frames;
     p->class_count_in = f > 0 ? counts + (f % 3) * kTileClasses : nullptr;
     p->class_list_in = f > 0 ? lists + (f % 2) * list : nullptr;
+    if (*how == kOverlappedFrame) return VRT_OK;
     p->class_count_out = counts + ((f + 1) % 3) * kTileClasses;
     p->class_list_out = lists + ((f + 1) % 2) * list;
     p->class_count_clear = counts + ((f + 2) % 3) * kTileClasses;
@@ -1847,18 +1919,24 @@ int vrt_render(vrt_renderer* r, const vrt_world* w, const vrt_uniforms* u, int32
         if (st) return st;
         p.words = w->d_words;
         p.words_z = w->d_words_z;
-        st = word_tile_order(r, grid, S(stream), &p);
+        int how = frame_launch(r, w, S(stream));
+        st = word_tile_order(r, grid, S(stream), &how, &p);
         if (st) return st;
         const bool debug = dbg && (dbg->hit_index || dbg->cast_mask || dbg->occ_mask || dbg->steps ||
                                    dbg->primary_steps || dbg->shade);
-        if (debug) render_word_kernel<true><<<grid, threads, 0, S(stream)>>>(w->d_words, w->L, p);
-        else render_word_kernel<false><<<grid, threads, 0, S(stream)>>>(w->d_words, w->L, p);
-        const cudaError_t le = cudaGetLastError();
+        const cudaError_t le = launch_frame(r, w, how, debug ? render_word_kernel<true> : render_word_kernel<false>,
+                                            grid, threads, S(stream), (const int32_t*)w->d_words, w->L, p);
         if (le != cudaSuccess) {
+            cudaGetLastError();
             r->tile_gx = r->tile_gy = 0;  // the classes of this frame were not written
             return cuda_error(le, "render_word_kernel");
         }
-        r->tile_frames++;
+        if (how == kOverlappedFrame) {
+            r->tile_reuses++;
+        } else if (how == kPlainFrame) {
+            r->tile_frames++;
+            r->tile_reuses = 0;
+        }
         return VRT_OK;
     }
     if (kernel == VRT_KERNEL_MASK_PIXEL) {  // follows depth-field jumps too
@@ -1867,7 +1945,7 @@ int vrt_render(vrt_renderer* r, const vrt_world* w, const vrt_uniforms* u, int32
         if (st) return st;
         ViewDev v;
         fill_view(v, *u, width, height, d_rgba, dbg, d_stats, t, 0);
-        return launch_tiles(w, &v, 1, tiles_of(width, height, t), nullptr, t.tile_w * t.tile_h, S(stream));
+        return launch_tiles(w, &v, 1, tiles_of(width, height, t), nullptr, t.tile_w * t.tile_h, S(stream), 0, -1, true, r);
     }
     if (kernel != VRT_KERNEL_BITMASK) return set_error(VRT_EINVAL, "unknown kernel %d", kernel);
     Tuning t = tuning_of(opts);

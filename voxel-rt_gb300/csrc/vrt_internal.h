@@ -109,6 +109,9 @@ struct vrt_world {
     uint64_t device_bytes = 0;
     int device = 0;
     int num_sms = 0;
+    uint64_t stamp = 0;             // a new one with every change of what renders read (mark_changed),
+                                    // 0 for a world with a change in a captured graph
+    bool in_graph = false;          // such a graph's runs change the world unseen
     bool reads_pageable = false;    // kernels read pageable host memory through the host's page tables
 };
 
@@ -131,6 +134,8 @@ struct WordChange {
 // Change the words, and bring the masks, distances, solid box and flag up to date: at most two
 // launches.
 int change_words(vrt_world* w, const WordChange& c, cudaStream_t s);
+// Called with every launch that changes what renders read of the world.
+void mark_changed(vrt_world* w, cudaStream_t s);
 // Note that the words of the box changed: the stop masks follow, and there the z-major copy
 // if it has not been changed with them.
 void mark_words(vrt_world* w, const int64_t box[6], bool z_copy);
@@ -146,6 +151,6 @@ int refresh_stop(vrt_world* w, cudaStream_t s);
 // run on another stream.
 int refresh_words_z(vrt_world* w, cudaStream_t s);
 // vrt_render_batch without the box-lookup counter: the launch that stores no side output
-// (63 registers, 8 CTAs per SM) instead of the one that does (69, 7 CTAs).
+// and counts no lookups, a burst of requests in 2755 us instead of 2830.
 int render_batch_rays(vrt_renderer* r, const vrt_view* views, int32_t count, void* stream);
 }  // namespace vrt

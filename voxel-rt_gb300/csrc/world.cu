@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <climits>
 #include <cstdio>
 #include <cstring>
@@ -38,12 +39,24 @@ Layout make_layout(int W, int H) {
 
 static inline unsigned blocks_for(uint64_t n, int threads) { return (unsigned)((n + threads - 1) / threads); }
 
+void mark_changed(vrt_world* w, cudaStream_t s) {
+    static std::atomic<uint64_t> next{1};
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    const bool now = cudaStreamIsCapturing(s, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
+    if (!now) {
+        cudaGetLastError();
+        w->in_graph = true;
+    }
+    w->stamp = w->in_graph ? 0 : next++;
+}
+
 int refresh_stop(vrt_world* w, cudaStream_t s) {
     if (!w->stop_stale) {
         VRT_CUDA(cudaStreamWaitEvent(s, w->stop_ready, 0));  // the last rebuild, on whichever stream
         return VRT_OK;
     }
     const Layout& L = w->L;
+    mark_changed(w, s);
     if (!w->d_stop) {
         cudaError_t e = cudaMalloc(&w->d_stop, L.n_bricks * 8);
         if (e == cudaSuccess) e = cudaMalloc(&w->d_sdir, L.n_bricks * 8);
@@ -134,6 +147,7 @@ int refresh_words_z(vrt_world* w, cudaStream_t s) {
         VRT_CUDA(cudaStreamWaitEvent(s, w->z_ready, 0));  // the last update, on whichever stream
         return VRT_OK;
     }
+    mark_changed(w, s);
     if (!w->d_words_z) {
         cudaError_t e = cudaMalloc(&w->d_words_z, L.n_words * sizeof(int32_t));
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&w->z_ready, cudaEventDisableTiming);
@@ -258,6 +272,7 @@ int vrt_world_create(int32_t width, int32_t height, vrt_world** out) {
                                               : cuda_error(e, "vrt_world_create");
     }
     w->device_bytes = bytes;
+    mark_changed(w, nullptr);
     *out = w;
     return VRT_OK;
 }

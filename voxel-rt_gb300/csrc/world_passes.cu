@@ -912,6 +912,7 @@ constexpr int64_t kWriteThrough = 1 << 16;
 
 int change_words(vrt_world* w, const WordChange& c, cudaStream_t s) {
     const Layout& L = w->L;
+    mark_changed(w, s);
     const bool through = w->d_words_z && (c.op == kRemoveSphere || c.op == kPlaceVoxel) &&
                          volume(L, c.box) <= kWriteThrough && (!c.fix || volume(L, c.fix_box) <= kWriteThrough);
     NodePass N{};
