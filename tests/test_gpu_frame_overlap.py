@@ -163,3 +163,37 @@ def test_captured_frames(cuda):
     for k in range(40):
         assert torch.equal(kept[2 * k].cpu(), expect[k % 3]), k
         assert torch.equal(kept[2 * k + 1].cpu(), expect[1]), k
+
+
+def test_changes_and_probes_in_a_row(cuda):
+    """Edits, probes of what they left and uploads queued without a wait give the words, masks
+    and answers of the same calls one by one."""
+    torch = pytest.importorskip("torch")
+    xyz = torch.tensor([[x, 2, z] for x in range(0, W, 5) for z in range(0, W, 5)], dtype=torch.int32, device="cuda")
+    row = torch.full((3 * W + 1,), 0x01ff0000, dtype=torch.int32, device="cuda")
+
+    def run(together, jumps):
+        w = scene(jumps)
+        found = [torch.zeros(len(xyz), dtype=torch.int32, device="cuda") for _ in range(30)]
+        torch.cuda.synchronize()
+        for k, f in enumerate(found):
+            w.remove_sphere(7 + 11 * k % 80, 3, 9 + 17 * k % 80, 5 + k % 4, 1 if jumps else 0)
+            if not together:
+                torch.cuda.synchronize()
+            w.probe(xyz.data_ptr(), len(xyz), f.data_ptr())
+            if k % 6 == 2:
+                w.place_voxel(5 * (k % 19), 2, 10, 0x0100ff00)
+            if k % 10 == 5:
+                w.upload_device(row.data_ptr(), 2 * W + 9 + k, row.numel() - 1)
+            if not together:
+                torch.cuda.synchronize()
+        words = np.empty(W * H * W, np.int32)
+        w.download(words)
+        return [f.cpu() for f in found], words, w.masks(), w.distances()
+
+    for jumps in (False, True):
+        a, b = run(True, jumps), run(False, jumps)
+        assert all(torch.equal(x, y) for x, y in zip(a[0], b[0]))
+        assert np.array_equal(a[1], b[1])
+        for p, q in zip(a[2:], b[2:]):
+            assert all(np.array_equal(x, y) for x, y in zip(p, q))

@@ -1643,16 +1643,7 @@ static int frame_launch(vrt_renderer* r, const vrt_world* w, cudaStream_t s) {
 template <class... Params, class... Args>
 static cudaError_t launch_frame(vrt_renderer* r, const vrt_world* w, int how, void (*kern)(Params...), dim3 grid,
                                 int threads, cudaStream_t s, const Args&... args) {
-    cudaLaunchAttribute pdl{};
-    pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    pdl.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.stream = s;
-    cfg.attrs = &pdl;
-    cfg.numAttrs = how == kOverlappedFrame ? 1 : 0;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
+    const cudaError_t e = launch_behind(how == kOverlappedFrame, kern, grid, threads, s, args...);
     if (how != kCapturedFrame) {
         std::lock_guard<std::mutex> lock(r->seen_mu);
         r->seen_stamp = e == cudaSuccess ? w->stamp : 0;

@@ -39,7 +39,7 @@ Layout make_layout(int W, int H) {
 
 static inline unsigned blocks_for(uint64_t n, int threads) { return (unsigned)((n + threads - 1) / threads); }
 
-void mark_changed(vrt_world* w, cudaStream_t s) {
+bool mark_changed(vrt_world* w, cudaStream_t s) {
     static std::atomic<uint64_t> next{1};
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     const bool now = cudaStreamIsCapturing(s, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
@@ -48,6 +48,7 @@ void mark_changed(vrt_world* w, cudaStream_t s) {
         w->in_graph = true;
     }
     w->stamp = w->in_graph ? 0 : next++;
+    return now;
 }
 
 int refresh_stop(vrt_world* w, cudaStream_t s) {
@@ -56,7 +57,7 @@ int refresh_stop(vrt_world* w, cudaStream_t s) {
         return VRT_OK;
     }
     const Layout& L = w->L;
-    mark_changed(w, s);
+    const bool behind = mark_changed(w, s);
     if (!w->d_stop) {
         cudaError_t e = cudaMalloc(&w->d_stop, L.n_bricks * 8);
         if (e == cudaSuccess) e = cudaMalloc(&w->d_sdir, L.n_bricks * 8);
@@ -78,7 +79,7 @@ int refresh_stop(vrt_world* w, cudaStream_t s) {
         }
         w->device_bytes += L.n_bricks * 16 + L.n_regions * 8;
     }
-    const int st = refresh_stop_masks(w, s);
+    const int st = refresh_stop_masks(w, s, behind);
     if (st) return st;
     VRT_CUDA(cudaEventRecord(w->stop_ready, s));
     w->stop_stale = false;
@@ -206,8 +207,11 @@ static int read_state(vrt_world* w, int& flag, cudaStream_t s) {
     return VRT_OK;
 }
 
-__global__ void probe_kernel(const int32_t* __restrict__ words, Layout L, const int32_t* __restrict__ xyz, int n,
-                             int32_t* __restrict__ out) {
+// Reads that a kernel ahead may have written, behind the wait: no __restrict__, which would let
+// them go through the read-only path.
+__global__ void probe_kernel(const int32_t* words, Layout L, const int32_t* xyz, int n, int32_t* out) {
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
@@ -419,8 +423,11 @@ int vrt_world_sync_flags(vrt_world* w, void* stream) {
 int vrt_world_probe(const vrt_world* w, const int32_t* d_xyz, int32_t n, int32_t* d_words, void* stream) {
     if (!w || n < 0 || (n > 0 && (!d_xyz || !d_words))) return set_error(VRT_EINVAL, "bad probe arguments");
     if (n == 0) return VRT_OK;
-    probe_kernel<<<blocks_for((uint64_t)n, 256), 256, 0, S(stream)>>>(w->d_words, w->L, d_xyz, n, d_words);
-    VRT_CUDA(cudaGetLastError());
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    const bool now = cudaStreamIsCapturing(S(stream), &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
+    if (!now) cudaGetLastError();
+    VRT_CUDA(launch_behind(now, probe_kernel, dim3(blocks_for((uint64_t)n, 256)), 256, S(stream),
+                           (const int32_t*)w->d_words, w->L, d_xyz, (int)n, d_words));
     return VRT_OK;
 }
 

@@ -582,7 +582,8 @@ union NodeSmem {
 // read what the brick pass wrote, and write different arrays.
 __global__ void __launch_bounds__(256) node_pass_kernel(const __grid_constant__ NodePass P) {
     __shared__ NodeSmem s;
-    cudaGridDependencySynchronize();  // the brick pass before it (see run_node_pass)
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();  // the brick pass before it
     int b = blockIdx.x;
     if (b < P.n_fix) return fix_tile(P.fix, b, s.fix);
     b -= P.n_fix;
@@ -596,6 +597,8 @@ __global__ void __launch_bounds__(256) node_pass_kernel(const __grid_constant__ 
 // a fourth CTA fits on each SM.
 __global__ void __launch_bounds__(256, 4) fix_depth_field_kernel(const __grid_constant__ FixPass P) {
     __shared__ FixSmem s;
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     fix_tile(P, blockIdx.x, s);
 }
 
@@ -654,6 +657,7 @@ __device__ __forceinline__ void level_row(int (&v)[4], int x0, int y, int z, int
 template <int OP>
 __global__ void __launch_bounds__(256, 4) brick_pass_kernel(const __grid_constant__ BrickPass P) {
     cudaTriggerProgrammaticLaunchCompletion();  // the node pass may be put in place behind this
+    cudaGridDependencySynchronize();
     const Layout& L = P.L;
     const int lane = threadIdx.x & 31, b = lane >> 2, q = lane & 3;
     const bool vec = (L.W & 3) == 0;
@@ -803,12 +807,11 @@ static bool brick_box(const Layout& L, const int64_t v[6], int b[6]) {
 }
 
 template <int OP>
-static int run_brick_pass(BrickPass& P, int num_sms, cudaStream_t s, int* blocks) {
+static int run_brick_pass(BrickPass& P, int num_sms, cudaStream_t s, bool behind, int* blocks) {
     // Whole worlds: as many CTAs as fit at once, each looping over its share
     const unsigned need = (P.tasks + 7) / 8;
     *blocks = (int)std::min<unsigned>(need, (unsigned)num_sms * kBrickCtasPerSm);
-    brick_pass_kernel<OP><<<*blocks, 256, 0, s>>>(P);
-    VRT_CUDA(cudaGetLastError());
+    VRT_CUDA(launch_behind(behind, brick_pass_kernel<OP>, dim3(*blocks), 256, s, P));
     return VRT_OK;
 }
 
@@ -876,24 +879,10 @@ static bool fix_tiles(NodePass& N, vrt_world* w, const int64_t v[6], int cx, int
     return true;
 }
 
-static int run_node_pass(const NodePass& P, cudaStream_t s) {
+static int run_node_pass(const NodePass& P, cudaStream_t s, bool behind) {
     const int blocks = P.n_fix + P.n_dir + P.n_reg + (P.n_boxes > 0 ? 1 : 0);
-    if (blocks > 0 && blocks == P.n_fix) fix_depth_field_kernel<<<blocks, 256, 0, s>>>(P.fix);
-    else if (blocks > 0) {
-        // Launched as a programmatic dependent of the brick pass: its CTAs are set up while the
-        // brick pass runs and begin when it has ended.
-        cudaLaunchAttribute pdl{};
-        pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        pdl.val.programmaticStreamSerializationAllowed = 1;
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(blocks);
-        cfg.blockDim = dim3(256);
-        cfg.stream = s;
-        cfg.attrs = &pdl;
-        cfg.numAttrs = 1;
-        VRT_CUDA(cudaLaunchKernelEx(&cfg, node_pass_kernel, P));
-    }
-    VRT_CUDA(cudaGetLastError());
+    if (blocks > 0 && blocks == P.n_fix) VRT_CUDA(launch_behind(behind, fix_depth_field_kernel, dim3(blocks), 256, s, P.fix));
+    else if (blocks > 0) VRT_CUDA(launch_behind(behind, node_pass_kernel, dim3(blocks), 256, s, P));
     return VRT_OK;
 }
 
@@ -912,7 +901,7 @@ constexpr int64_t kWriteThrough = 1 << 16;
 
 int change_words(vrt_world* w, const WordChange& c, cudaStream_t s) {
     const Layout& L = w->L;
-    mark_changed(w, s);
+    const bool behind = mark_changed(w, s);
     const bool through = w->d_words_z && (c.op == kRemoveSphere || c.op == kPlaceVoxel) &&
                          volume(L, c.box) <= kWriteThrough && (!c.fix || volume(L, c.fix_box) <= kWriteThrough);
     NodePass N{};
@@ -932,11 +921,11 @@ int change_words(vrt_world* w, const WordChange& c, cudaStream_t s) {
         P.x = c.x; P.y = c.y; P.z = c.z; P.r = c.r; P.word = c.word;
         int st = VRT_OK;
         switch (c.op) {
-            case kReadWords: st = run_brick_pass<kReadWords>(P, w->num_sms, s, &N.n_boxes); break;
-            case kRemoveSphere: st = run_brick_pass<kRemoveSphere>(P, w->num_sms, s, &N.n_boxes); break;
-            case kInitLevel: st = run_brick_pass<kInitLevel>(P, w->num_sms, s, &N.n_boxes); break;
-            case kPlaceVoxel: st = run_brick_pass<kPlaceVoxel>(P, w->num_sms, s, &N.n_boxes); break;
-            default: st = run_brick_pass<kCopyWords>(P, w->num_sms, s, &N.n_boxes); break;
+            case kReadWords: st = run_brick_pass<kReadWords>(P, w->num_sms, s, behind, &N.n_boxes); break;
+            case kRemoveSphere: st = run_brick_pass<kRemoveSphere>(P, w->num_sms, s, behind, &N.n_boxes); break;
+            case kInitLevel: st = run_brick_pass<kInitLevel>(P, w->num_sms, s, behind, &N.n_boxes); break;
+            case kPlaceVoxel: st = run_brick_pass<kPlaceVoxel>(P, w->num_sms, s, behind, &N.n_boxes); break;
+            default: st = run_brick_pass<kCopyWords>(P, w->num_sms, s, behind, &N.n_boxes); break;
         }
         if (st) return st;
         node_tiles(N, b);
@@ -948,10 +937,10 @@ int change_words(vrt_world* w, const WordChange& c, cudaStream_t s) {
         N.fix.words_z = through ? w->d_words_z : nullptr;
         mark_words(w, c.fix_box, !through);
     }
-    return run_node_pass(N, s);
+    return run_node_pass(N, s, behind);
 }
 
-int refresh_stop_masks(vrt_world* w, cudaStream_t s) {
+int refresh_stop_masks(vrt_world* w, cudaStream_t s, bool behind) {
     const Layout& L = w->L;
     const int64_t v[6] = {0, 0, 0, L.W, L.H, L.W};
     int b[6], blocks = 0;
@@ -960,7 +949,7 @@ int refresh_stop_masks(vrt_world* w, cudaStream_t s) {
     P.bricks = w->d_stop;
     P.regions = w->d_stop_regions;
     P.supers = nullptr;
-    const int st = run_brick_pass<kStopWords>(P, w->num_sms, s, &blocks);
+    const int st = run_brick_pass<kStopWords>(P, w->num_sms, s, behind, &blocks);
     if (st) return st;
     NodePass N{};
     N.L = L;
@@ -968,7 +957,7 @@ int refresh_stop_masks(vrt_world* w, cudaStream_t s) {
     N.regions = w->d_stop_regions;
     N.bdir = reinterpret_cast<uint16_t*>(w->d_sdir);
     N.n_reg = 0;
-    return run_node_pass(N, s);
+    return run_node_pass(N, s, behind);
 }
 
 }  // namespace vrt
