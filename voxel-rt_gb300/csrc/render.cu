@@ -205,19 +205,21 @@ struct WordRay {
 // true.  (Only y: in terrain worlds the solid box spans x and z, and two registers per
 // ray are what this latency-bound kernel can spare.)
 //
-// What bounds it: instruction issue (75 % of the slots while an SM is busy), 49 M warp
-// instructions for an 800x600 frame of the level with three lights.  An iteration is about 40
+// What bounds it: instruction issue (75 % of the slots while an SM is busy), 47 M warp
+// instructions for an 800x600 frame of the level with three lights.  An iteration is about 35
 // instructions, a jump 45 more, a ray's set-up and shading 400.  The jump's three IEEE
 // divisions as div_by and no prefetch of the words ahead (24 instructions in each iteration,
 // once worth it for its long dependent chain): that frame 77.7 -> 66.6 us, the app's first
 // frame 67.2 -> 60.3 us (of which the divisions alone are nothing and the prefetch 8 us).  The
 // intersect adds in the shadow of the load, and not behind it for the iterations that turn out
 // not to jump: 67.2 -> 62.7 and 59.9 -> 54.1 us; the ray's six reciprocals by rcp_near: 61.8
-// and 53.7 us.  Tried without gain: 8x4 tiles of the words instead of the second copy (96 us on
-// the app's first frame), both copies' loads predicated (75.7 then; one load with a predicated
-// address now: 61.5 and 53.9), the hit's results taken after the loop (62.1 and 56.1), 5 to 8
-// CTAs per SM by fewer registers (67.0-69.3 of 66.6), one warp per CTA (63.6 of 60.3 us with
-// 16x8 tiles).
+// and 53.7 us.  Frames in a row that overlap take 47.8 and 38.4 us, and with the word's load
+// predicated instead of branched around 44.9 and 34.4 us.  Tried without gain: 8x4 tiles of the
+// words instead of the second copy (96 us on the app's first frame), both copies' loads
+// predicated (75.7 of 68.1), the hit's results taken after the loop (62.1 and 56.1 of 61.5 and
+// 54.0), 5 to 8 CTAs per SM by fewer registers (67.0-69.3 of 66.6), one warp per CTA (63.6 of
+// 60.3 us with 16x8 tiles), one call site for all shadow rays (46.0 and 35.0 of 44.9 and 34.4),
+// two iterations per trip (46.6 and 35.2).
 __device__ WordRay cast_word(const Layout& L, const WordParams& p, V3 start, V3 dir, int dist, int maxSteps) {
     WordRay o;
     o.hit = -1; o.cd = 0.0f; o.axis = 2; o.s = 0; o.steps = 0;
@@ -266,14 +268,26 @@ __device__ WordRay cast_word(const Layout& L, const WordParams& p, V3 start, V3 
         pred_fadd(r.tz, r.dz, bz);
         // Outside the world (getVoxelIndex == -1), or no solid voxel ahead: the ray ends as at a
         // solid voxel (word 0), without a hit.
-        const bool in = ((unsigned)r.cx < (unsigned)L.W) & ((unsigned)(r.cy - lo_y) < (unsigned)span_y) &
-                        ((unsigned)r.cz < (unsigned)L.W);
+        const bool in = (max((unsigned)r.cx, (unsigned)r.cz) < (unsigned)L.W) &
+                        ((unsigned)(r.cy - lo_y) < (unsigned)span_y);
         // A step along z reads the copy in which z is the fastest index: a run of z steps then
         // reads consecutive words instead of one cache line per step (W*H words apart).  That
         // run is the longest ray of the reference's own frame: the shader's x == y tie sends a
         // ray along z for hundreds of steps, which set the frame's length.
+        // One load, predicated: the compiler's branch around it parts and joins the lanes again in
+        // every iteration.
         int32_t v = 0;
-        if (in) v = __ldg((bz ? p.words_z : p.words) + ((bz ? r.cz : r.cx) + W * r.cy + WH * (bz ? r.cx : r.cz)));
+        {
+            const int wy = W * r.cy;
+            asm("{.reg .pred pz, pi; .reg .b64 q;\n\t"
+                "setp.ne.b32 pz, %3, 0; setp.ne.b32 pi, %4, 0;\n\t"
+                "mad.wide.s32 q, %1, 4, %5;\n\t"
+                "@pz mad.wide.s32 q, %2, 4, %6;\n\t"
+                "@pi ld.global.nc.b32 %0, [q];}"
+                : "+r"(v)
+                : "r"(r.cx + wy + WH * r.cz), "r"(r.cz + wy + WH * r.cx), "r"((int)bz), "r"((int)in), "l"(p.words),
+                  "l"(p.words_z));
+        }
         if (v != -1) {
             if (v >= 0) {
                 if (in) {
