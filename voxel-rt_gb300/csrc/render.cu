@@ -189,6 +189,30 @@ __device__ __forceinline__ void enter_cell(RaySetup& r, V3 start, V3 dir, V3 inv
     }
 }
 
+// Whether the words a warp's rays are about to read lie in HBM rather than in L2: one load 40 cell
+// lengths ahead of the camera, timed.  A frame that follows others finds its words in L2 (the
+// load takes 300 to 500 cycles); one whose words were never read or were displaced waits for HBM
+// at every new line, and then prefetching 24 cell lengths ahead pays for its ten instructions an
+// iteration, which cost an 800x600 level frame with three lights 11 us otherwise.  L2 flushed
+// before each frame: 107 and 124 us without prefetching, 89 and 99 with it (two cameras), the
+// app's first frame 92 and 77; frames in a row 45.0 -> 46.2 and 34.5 -> 35.4 us.  Limits of 350
+// and 450 cycles took 48.7 and 46.8 us in a row, 1000 gained nothing.
+constexpr float kPrefetchCells = 24.0f, kProbeCells = 40.0f;
+constexpr uint32_t kFarCycles = 600;
+__device__ __forceinline__ bool words_are_far(const Layout& L, const WordParams& p, V3 cam, V3 dir) {
+    const int x = min(max(f2i(fadd(fmul(dir.x, kProbeCells), cam.x)), 0), L.W - 1);
+    const int y = min(max(f2i(fadd(fmul(dir.y, kProbeCells), cam.y)), 0), L.H - 1);
+    const int z = min(max(f2i(fadd(fmul(dir.z, kProbeCells), cam.z)), 0), L.W - 1);
+    uint32_t from, to;
+    int32_t v;
+    asm volatile("mov.u32 %0, %%clock;" : "=r"(from));
+    asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p.words + (x + L.W * y + L.W * L.H * z)));
+    // the clock is read under a condition on the word, so behind its arrival
+    asm volatile("{.reg .pred q;\n\tsetp.eq.s32 q, %1, 0x7fffffff;\n\t@q mov.u32 %0, 0;\n\t@!q mov.u32 %0, %%clock;}"
+                 : "=r"(to) : "r"(v));
+    return to - from > kFarCycles;
+}
+
 struct WordRay {
     int32_t hit;   // voxel index or -1
     float cd;      // currDist at the hit
@@ -208,9 +232,9 @@ struct WordRay {
 // What bounds it: instruction issue (75 % of the slots while an SM is busy), 47 M warp
 // instructions for an 800x600 frame of the level with three lights.  An iteration is about 35
 // instructions, a jump 45 more, a ray's set-up and shading 400.  The jump's three IEEE
-// divisions as div_by and no prefetch of the words ahead (24 instructions in each iteration,
-// once worth it for its long dependent chain): that frame 77.7 -> 66.6 us, the app's first
-// frame 67.2 -> 60.3 us (of which the divisions alone are nothing and the prefetch 8 us).  The
+// divisions as div_by and no prefetch of the words ahead where they lie in L2 (24 instructions
+// in each iteration): that frame 77.7 -> 66.6 us, the app's first frame 67.2 -> 60.3 us (of which
+// the divisions alone are nothing and the prefetch 8 us; see words_are_far).  The
 // intersect adds in the shadow of the load, and not behind it for the iterations that turn out
 // not to jump: 67.2 -> 62.7 and 59.9 -> 54.1 us; the ray's six reciprocals by rcp_near: 61.8
 // and 53.7 us.  Frames in a row that overlap take 47.8 and 38.4 us, and with the word's load
@@ -220,7 +244,8 @@ struct WordRay {
 // 54.0), 5 to 8 CTAs per SM by fewer registers (67.0-69.3 of 66.6), one warp per CTA (63.6 of
 // 60.3 us with 16x8 tiles), one call site for all shadow rays (46.0 and 35.0 of 44.9 and 34.4),
 // two iterations per trip (46.6 and 35.2).
-__device__ WordRay cast_word(const Layout& L, const WordParams& p, V3 start, V3 dir, int dist, int maxSteps) {
+__device__ WordRay cast_word(const Layout& L, const WordParams& p, V3 start, V3 dir, int dist, int maxSteps,
+                             bool far) {
     WordRay o;
     o.hit = -1; o.cd = 0.0f; o.axis = 2; o.s = 0; o.steps = 0;
     RaySetup r;
@@ -249,6 +274,9 @@ __device__ WordRay cast_word(const Layout& L, const WordParams& p, V3 start, V3 
     float travelled = 0.0f;
     const float lim = fminf((float)dist, (float)maxSteps);
     const int W = L.W, WH = L.W * L.H;
+    const unsigned ax = (unsigned)f2i(fmul(dir.x, kPrefetchCells)), ay = (unsigned)f2i(fmul(dir.y, kPrefetchCells)),
+                   az = (unsigned)f2i(fmul(dir.z, kPrefetchCells));
+    const unsigned ahead = ax + (unsigned)W * ay + (unsigned)WH * az, ahead_z = az + (unsigned)W * ay + (unsigned)WH * ax;
     while (travelled < lim) {
         o.steps++;
         travelled = fadd(travelled, 1.0f);
@@ -287,6 +315,13 @@ __device__ WordRay cast_word(const Layout& L, const WordParams& p, V3 start, V3 
                 : "+r"(v)
                 : "r"(r.cx + wy + WH * r.cz), "r"(r.cz + wy + WH * r.cx), "r"((int)bz), "r"((int)in), "l"(p.words),
                   "l"(p.words_z));
+        }
+        if (far) {  // the word some way ahead in both copies (any word at all where the sum leaves them)
+            const unsigned n = (unsigned)L.n_words, wy = (unsigned)W * (unsigned)r.cy;
+            const unsigned i = (unsigned)r.cx + wy + (unsigned)WH * (unsigned)r.cz + ahead;
+            const unsigned iz = (unsigned)r.cz + wy + (unsigned)WH * (unsigned)r.cx + ahead_z;
+            if (i < n) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.words + i));
+            if (iz < n) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.words_z + iz));
         }
         if (v != -1) {
             if (v >= 0) {
@@ -346,12 +381,14 @@ __global__ void __launch_bounds__(128, 4) render_word_kernel(const int32_t* __re
     PixelResult res{};
     const vrt_uniforms& u = p.u;
     const V3 cam{u.camPos[0], u.camPos[1], u.camPos[2]};
+    bool far = false;
     V3 rd{0.f, 0.f, 0.f};
     WordRay pr;
     pr.hit = -1; pr.cd = 0.f; pr.axis = 2; pr.s = 0; pr.start = cam; pr.steps = 0;
     if (valid) {
         rd = primary_dir(u, px, py, p.width, p.height, p.map.inv_w, p.map.inv_h);
-        pr = cast_word(L, p, cam, rd, u.maxSteps, u.maxSteps);
+        far = words_are_far(L, p, cam, rd);
+        pr = cast_word(L, p, cam, rd, u.maxSteps, u.maxSteps, far);
     }
     const bool lit = valid && pr.hit >= 0 && u.viewDepthField != 1;
     const V3 hp = lit ? add3(mul3s(rd, pr.cd), pr.start) : V3{0.f, 0.f, 0.f};
@@ -368,7 +405,7 @@ __global__ void __launch_bounds__(128, 4) render_word_kernel(const int32_t* __re
             V3 hn = axis_normal(pr.axis, pr.s);
             V3 lp{u.lightPos[0], u.lightPos[1], u.lightPos[2]};
             V3 toLight = norm3(sub3(lp, hp));
-            WordRay sr = cast_word(L, p, add3(hp, mul3s(toLight, 0.001f)), toLight, u.maxSteps, u.maxSteps);
+            WordRay sr = cast_word(L, p, add3(hp, mul3s(toLight, 0.001f)), toLight, u.maxSteps, u.maxSteps, far);
             res.steps += sr.steps;
             res.cast |= 1u;
             if (sr.hit < 0) {
@@ -401,7 +438,7 @@ __global__ void __launch_bounds__(128, 4) render_word_kernel(const int32_t* __re
                 if (ld <= R) {
                     V3 tl = norm3(dl);
                     WordRay lr = cast_word(L, p, add3(hp, mul3s(tl, 0.001f)), tl, f2i(fadd(ld, 1.0f)),
-                                           u.maxSteps);
+                                           u.maxSteps, far);
                     res.steps += lr.steps;
                     res.cast |= 2u << i;
                     if (lr.hit < 0) {
