@@ -190,15 +190,16 @@ __device__ __forceinline__ void enter_cell(RaySetup& r, V3 start, V3 dir, V3 inv
 }
 
 // Whether the words a warp's rays are about to read lie in HBM rather than in L2: one load 40 cell
-// lengths ahead of the camera, timed.  A frame that follows others finds its words in L2 (the
-// load takes 300 to 500 cycles); one whose words were never read or were displaced waits for HBM
-// at every new line, and then prefetching 24 cell lengths ahead pays for its ten instructions an
-// iteration, which cost an 800x600 level frame with three lights 11 us otherwise.  L2 flushed
-// before each frame: 107 and 124 us without prefetching, 89 and 99 with it (two cameras), the
-// app's first frame 92 and 77; frames in a row 45.0 -> 46.2 and 34.5 -> 35.4 us.  Limits of 350
-// and 450 cycles took 48.7 and 46.8 us in a row, 1000 gained nothing.
+// lengths ahead of the camera, timed.  A frame that follows others finds its words in L2; one
+// whose words were never read or were displaced waits for HBM at every new line, and then
+// prefetching 24 cell lengths ahead pays for its ten instructions an iteration, which cost an
+// 800x600 level frame with three lights 11 us otherwise.  L2 flushed before each frame: 107 and
+// 124 us without prefetching, 89 and 99 with it (two cameras), the app's first frame 92 and 75;
+// frames in a row 44.9 -> 46.6 and 34.4 -> 35.7 us.  The limit lies where both hold: at 420
+// cycles the frames in a row take 47.3 and 36.8 us, at 600 (46.1 and 35.4) the app's first frame
+// takes 81 to 91 us after a flush.
 constexpr float kPrefetchCells = 24.0f, kProbeCells = 40.0f;
-constexpr uint32_t kFarCycles = 600;
+constexpr uint32_t kFarCycles = 480;
 __device__ __forceinline__ bool words_are_far(const Layout& L, const WordParams& p, V3 cam, V3 dir) {
     const int x = min(max(f2i(fadd(fmul(dir.x, kProbeCells), cam.x)), 0), L.W - 1);
     const int y = min(max(f2i(fadd(fmul(dir.y, kProbeCells), cam.y)), 0), L.H - 1);
