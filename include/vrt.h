@@ -232,10 +232,10 @@ int vrt_terrain_height(int32_t width, uint64_t seed, int32_t x, int32_t z);
 /* ---- rendering ---- */
 /* A renderer owns per-launch scratch: the view table of batches, the persistent kernel's
  * tile counter, the staging image and streams of vrt_render_to_host, and the word
- * kernel's tile order (128 bytes per pixel tile).  Each word-kernel render sorts its tiles
- * into cost classes as they end, and the next word-kernel render of the same tile grid on
- * the same renderer launches them heaviest class first; the order changes no result (and
- * without device memory for it, frames run in row order).
+ * kernel's tile order (128 bytes per pixel tile).  A word-kernel render that overlaps no other
+ * sorts its tiles into cost classes as they end, and the next word-kernel renders of the same
+ * tile grid on the same renderer launch them heaviest class first; the order changes no result
+ * (and without device memory for it, or captured into a graph, frames run in row order).
  * Creating the first renderer on a device also fills a 1 KiB table the pixel colour reads
  * (synchronises the device once).  One renderer per concurrently used stream. */
 int vrt_renderer_create(vrt_renderer** out);
@@ -247,9 +247,12 @@ int vrt_renderer_destroy(vrt_renderer* r);
  * 0 = bottom row (GL order); pixel (px,py) sees vPos = ((2px+1)/width-1, (2py+1)/height-1).  dbg,
  * d_stats and opts may be NULL.  The tile kernel's first render of a depth-field world
  * after its words changed also rebuilds the world's stop masks on this stream (allocated
- * on first use, 16 bytes per brick).  The word kernel's first render after the words
- * changed brings the world's z-major copy of the words up to date over the changed box
- * on this stream (allocated and filled on first use: as large as the words). */
+ * on first use, 16 bytes per brick and 8 per region).  The word kernel's first render after
+ * a large change of the words brings the world's z-major copy of them up to date over the
+ * changed box on this stream (allocated and filled on first use: as large as the words).
+ * A render of the world that this renderer's last render on the same stream showed, unchanged
+ * since, may trace while that one's last tiles run; it writes after that one has ended, so
+ * work on the stream sees the renders one after the other. */
 int vrt_render(vrt_renderer* r, const vrt_world* w, const vrt_uniforms* u, int32_t width,
                int32_t height, uint8_t* d_rgba, const vrt_debug_out* dbg, uint64_t* d_stats,
                const vrt_render_opts* opts, void* stream);

@@ -12,16 +12,18 @@ commands in profiles/*.md name the case and the kernel (-k) they capture.
   batch          the 64 cameras of the bench's batch over the 1080p world, tile kernel with
                  a tile shape per resolution class, replayed twice from a CUDA graph
   edits          removeSphere of radius 8 at 8 surface points of the 1080p world
-                 (remove_sphere_kernel, then the mask and distance refresh of each edit)
+                 (brick_pass_kernel<1>, then node_pass_kernel, for each edit)
   depth_edits    the reference world (initVoxels + fixDepthField) edited by removeSphere
-                 of radius 7 with the depth-field refresh, 4 times: the first
-                 fix_depth_field_kernel launch is the whole world, the next are edit-sized
+                 of radius 7 with the depth-field refresh, 4 times: brick_pass_kernel<1> and
+                 a node_pass_kernel with depth-field tiles each
   stop_masks     the reference world after an edit, rendered by the tile kernel
-                 (stop_mask_kernel rebuilds the stop masks, then the render), 2 rounds
+                 (brick_pass_kernel<5> and node_pass_kernel rebuild the stop masks, then the
+                 render), 2 rounds
   probe          1 Mi voxel probes of the 1080p world (probe_kernel), 3 launches
-  world_build    upload of the 1080p world (brick_mask, parent_mask, dir_pass, cheb_pass)
-  reference_build  the reference world on the device: initVoxels (init_reference_layers,
-                 init_reference_trees), then fixDepthField over the whole world
+  world_build    upload of the 1080p world (brick_pass_kernel<3>, node_pass_kernel)
+  reference_build  the reference world on the device: initVoxels (brick_pass_kernel<4>,
+                 node_pass_kernel), then fixDepthField over the whole world
+                 (fix_depth_field_kernel)
   reference_frame  the reference app's first frame (its world with the depth field, camera
                  (195,55,155), 800x600, 384 steps), rendered as bench.py --workload reference
                  does: the kernel AUTO picks (the word kernel) with its own 16x8 pixel tiles,
