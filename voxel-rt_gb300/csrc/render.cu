@@ -85,6 +85,7 @@ struct WordParams {
     int* class_list_out;
     int* class_count_clear;
     int tiles;
+    int wait_first;  // 1: the kernel ahead may be changing the words (see frame_launch)
 };
 
 // The word kernel's tile order.  The frame's length is set by its heaviest tiles: on the
@@ -312,7 +313,7 @@ __device__ WordRay cast_word(const Layout& L, const WordParams& p, V3 start, V3 
                 "setp.ne.b32 pz, %3, 0; setp.ne.b32 pi, %4, 0;\n\t"
                 "mad.wide.s32 q, %1, 4, %5;\n\t"
                 "@pz mad.wide.s32 q, %2, 4, %6;\n\t"
-                "@pi ld.global.nc.b32 %0, [q];}"
+                "@pi ld.global.b32 %0, [q];}"
                 : "+r"(v)
                 : "r"(r.cx + wy + WH * r.cz), "r"(r.cz + wy + WH * r.cx), "r"((int)bz), "r"((int)in), "l"(p.words),
                   "l"(p.words_z));
@@ -348,22 +349,23 @@ __device__ WordRay cast_word(const Layout& L, const WordParams& p, V3 start, V3 
 // A minimum of 4 CTAs per SM gives the compiler up to 128 registers; it takes 72 (7 CTAs
 // per SM).
 template <bool DEBUG>
-__global__ void __launch_bounds__(128, 4) render_word_kernel(const int32_t* __restrict__ words, Layout L,
+__global__ void __launch_bounds__(128, 4) render_word_kernel(const int32_t* words, Layout L,
                                                           const __grid_constant__ WordParams p) {
     __shared__ int s_cost, s_done, s_tile;
     cudaTriggerProgrammaticLaunchCompletion();  // see frame_launch
+    if (p.wait_first) cudaGridDependencySynchronize();
     if (threadIdx.x < 32) {
         const int b = (int)(blockIdx.x + gridDim.x * blockIdx.y), lane = threadIdx.x;
         int tile = b;
         if (p.class_count_in) {  // the b-th tile of the last frame's classes, heaviest class first
             const int c = kTileClasses - 1 - lane;  // lane l: class 15 - l, and how many lie before it
-            const int n = lane < kTileClasses ? __ldg(p.class_count_in + c) : 0;
+            const int n = lane < kTileClasses ? p.class_count_in[c] : 0;
             int end = n;
             for (int o = 1; o < kTileClasses; o *= 2) {
                 const int u = __shfl_up_sync(0xffffffffu, end, o);
                 if (lane >= o) end += u;
             }
-            if (b < end && b >= end - n) tile = __ldg(p.class_list_in + c * p.tiles + (b - (end - n)));
+            if (b < end && b >= end - n) tile = p.class_list_in[c * p.tiles + (b - (end - n))];
             const unsigned found = __ballot_sync(0xffffffffu, b < end && b >= end - n);
             tile = __shfl_sync(0xffffffffu, tile, found ? __ffs(found) - 1 : 0);
         }
@@ -455,7 +457,7 @@ __global__ void __launch_bounds__(128, 4) render_word_kernel(const int32_t* __re
                 }
             }
             if (!clamped && last < VRT_MAX_LOCAL_LIGHTS - 1 && mr >= ob && mg >= ob && mb >= ob) mr = mg = mb = ob;
-            word = __ldg(words + pr.hit);
+            word = words[pr.hit];
         }
         res.mr = mr; res.mg = mg; res.mb = mb;
         res.rgba = pack_color_tab(u, pr.hit >= 0, word, mr, mg, mb, pr.steps);
@@ -1678,8 +1680,11 @@ static int launch_mask(vrt_renderer* r, const vrt_world* w, const ViewDev* h_vie
 // other.  Frames in a row, each alone before: 256x256 16.9 -> 7.4 us, 1080p 192.5 -> 184.2, 4K
 // 551 -> 544 (the CTAs that wait hold their places), the app's first frame 58.9 -> 38.4, the
 // 800x600 level frame with three lights 65.8 -> 47.8 us.
+// Any other frame waits for all ahead.  The word kernel is a dependent then too and waits before
+// its first access, as edits do (launch_behind): probe, edit and frame 80.1 -> 77.0 us.  It reads
+// the words by plain loads therefore.  (The tile kernel's loads stay on the read-only path.)
 // A captured launch is a plain one, and is not taken for the stream's last frame; the streams
-// of cudaStreamPerThread share a handle, so theirs are plain too.
+// of cudaStreamPerThread share a handle, so theirs overlap nothing.
 enum { kPlainFrame, kOverlappedFrame, kCapturedFrame };
 static int frame_launch(vrt_renderer* r, const vrt_world* w, cudaStream_t s) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
@@ -1693,9 +1698,9 @@ static int frame_launch(vrt_renderer* r, const vrt_world* w, cudaStream_t s) {
 }
 
 template <class... Params, class... Args>
-static cudaError_t launch_frame(vrt_renderer* r, const vrt_world* w, int how, void (*kern)(Params...), dim3 grid,
-                                int threads, cudaStream_t s, const Args&... args) {
-    const cudaError_t e = launch_behind(how == kOverlappedFrame, kern, grid, threads, s, args...);
+static cudaError_t launch_frame(vrt_renderer* r, const vrt_world* w, int how, bool behind, void (*kern)(Params...),
+                                dim3 grid, int threads, cudaStream_t s, const Args&... args) {
+    const cudaError_t e = launch_behind(behind, kern, grid, threads, s, args...);
     if (how != kCapturedFrame) {
         std::lock_guard<std::mutex> lock(r->seen_mu);
         r->seen_stamp = e == cudaSuccess ? w->stamp : 0;
@@ -1772,7 +1777,8 @@ static int launch_tiles(const vrt_world* w, const ViewDev* h_views, int nviews, 
     P.tile0 = tile0;
     if (ntiles < 0) ntiles = total_tiles - tile0;
     if (frame_of) {  // a renderer's whole frame
-        VRT_CUDA(launch_frame(frame_of, w, frame_launch(frame_of, w, s), kern, dim3(ntiles), threads, s, P));
+        const int how = frame_launch(frame_of, w, s);
+        VRT_CUDA(launch_frame(frame_of, w, how, how == kOverlappedFrame, kern, dim3(ntiles), threads, s, P));
         return VRT_OK;
     }
     if (ntiles > 0) kern<<<ntiles, threads, 0, s>>>(P);
@@ -1965,9 +1971,10 @@ int vrt_render(vrt_renderer* r, const vrt_world* w, const vrt_uniforms* u, int32
         int how = frame_launch(r, w, S(stream));
         st = word_tile_order(r, grid, S(stream), &how, &p);
         if (st) return st;
+        p.wait_first = how == kPlainFrame;
         const bool debug = dbg && (dbg->hit_index || dbg->cast_mask || dbg->occ_mask || dbg->steps ||
                                    dbg->primary_steps || dbg->shade);
-        const cudaError_t le = launch_frame(r, w, how, debug ? render_word_kernel<true> : render_word_kernel<false>,
+        const cudaError_t le = launch_frame(r, w, how, how != kCapturedFrame, debug ? render_word_kernel<true> : render_word_kernel<false>,
                                             grid, threads, S(stream), (const int32_t*)w->d_words, w->L, p);
         if (le != cudaSuccess) {
             cudaGetLastError();
