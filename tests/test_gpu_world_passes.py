@@ -127,3 +127,20 @@ def test_frames_after_edits_that_write_the_z_major_copy(cuda, oracle, W, H):
             e()
         now = w.download(np.empty(W * H * W, np.int32))
         assert_same_frame(oracle.render(now, W, H, u, 60, 40), gpu_render(w, u, 60, 40, kernel=vrt.KERNEL_WORD))
+
+
+@pytest.mark.parametrize("W,H", [(33, 17), (97, 41)])
+@pytest.mark.parametrize("density", [0.0006, 0.01, 0.2])
+def test_edits_with_small_and_large_depth_field_tiles(cuda, oracle, W, H, density):
+    """Edits whose boxes end on either side of the tiles' edges, take a few small tiles or, from
+    radius 34 in the larger world, the large ones; solids at the rim of the depth field's radius."""
+    words = sparse_words(W, H, 3 * W + H, density)
+    w = make_world(words, W, H)
+    ref = words.copy()
+    centres = [(0, 0, 0), (8, 8, 8), (W - 1, H - 1, W - 1), (15, 9, 24), (16, 7, 25), (W // 2, H // 2, W // 2)]
+    for r in (0, 1, 4, 5, 12, 34):
+        for c in centres if r < 34 else centres[-1:]:
+            w.remove_sphere(*c, r, 1)
+            oracle.remove_sphere(ref, W, H, *c, r, 1)
+            got = w.download(np.empty_like(ref))
+            assert np.array_equal(got, ref), (c, r, np.flatnonzero(got != ref)[:4])

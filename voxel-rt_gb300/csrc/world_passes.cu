@@ -54,6 +54,7 @@ struct FixPass {
     Layout L;
     int x0, y0, z0, x1, y1, z1;  // the voxels to refresh, within the world
     int cx, cy, cz, r2;          // r2 > 0: of those, the ones inside this sphere
+    int small;                   // tiles of 8 x 8 rows instead of 16 x 16
     int tx0, ty0, tz0, ntx, nty; // the tiles that cover the box
     int32_t word[kFixLevels + 1];
 };
@@ -89,29 +90,40 @@ struct NodePass {
 // S.  Going up the levels, each (row, k) pair is ORed in once: about 600 ORs for 32 voxels,
 // where testing the 1413 offsets voxel by voxel took 45,000 loads.
 
-constexpr int kFixX = 32, kFixY = 16, kFixZ = 16;  // voxels per tile: one row word x 16 x 16 rows
+constexpr int kFixX = 32;                          // voxels per tile along x: one row word
 constexpr int kFixHalo = 7;                        // DEPTH_FIELD_RADIUS, render.hpp:7
-constexpr int kFixRows = kFixY + 2 * kFixHalo;     // rows per axis with the halo
-// Row pitch of a D_k plane: a warp's lanes are 16 rows in y of two z, so a pitch of 16
-// modulo 32 puts them into 32 different banks.
-constexpr int kFixPitch = 48;
-constexpr int kFixPlane = kFixRows * kFixPitch;
-constexpr int kFixK = 6;               // D_1 .. D_6 (|x| = 7 alone gives s = 36)
-constexpr int kFixNodes = 12 * 8 * 8;  // bricks spanned: 8 + 2 x 2 in x, 4 + 2 x 2 in y and z
+constexpr int kFixK = 6;                           // D_1 .. D_6 (|x| = 7 alone gives s = 36)
 
-struct FixSmem {
-    uint64_t nodes[kFixNodes];
-    uint32_t d[kFixK * kFixPlane];
-    uint32_t out[7][kFixY * kFixZ];  // per row: the 6 bits of s, and the voxels to write
-    int32_t word[kFixLevels + 1];    // the depth-field word of each s; [36]: no solid neighbour
+// A tile of SIDE x SIDE rows by 256 threads: one thread per row of 16 x 16, or four per row of
+// 8 x 8, which take a fourth of the levels each.  The large tile reads the least halo per voxel.
+// The small one is for an edit's few tiles, whose time is one tile's chain: some 600 reads of
+// shared memory by each of 8 warps at 16 x 16, 150 at 8 x 8.
+template <int SIDE>
+struct FixTile {
+    static constexpr int kShift = SIDE == 16 ? 4 : 3;
+    static constexpr int kRows = SIDE + 2 * kFixHalo;  // rows per axis with the halo
+    // Row pitch of a D_k plane: a warp's lanes are SIDE rows in y of 32 / SIDE z, so a pitch of SIDE
+    // modulo 32 puts them into 32 different banks.
+    static constexpr int kPitch = SIDE + 32, kPlane = kRows * kPitch;
+    static constexpr int kSpan = SIDE / 4 + 4;         // bricks spanned in y and z; 8 + 2 x 2 in x
+    static constexpr int kNodes = 12 * kSpan * kSpan;
+    static constexpr int kParts = 256 / (SIDE * SIDE);  // threads of a row
+    struct Smem {
+        uint64_t nodes[kNodes];
+        uint32_t d[kFixK * kPlane];
+        uint32_t out[7][SIDE * SIDE];              // per row: the 6 bits of s, and the voxels to write
+        uint32_t part[kParts > 1 ? kParts - 1 : 1][7][kParts > 1 ? SIDE * SIDE : 1];  // the other threads' bits and found
+        int32_t word[kFixLevels + 1];              // the depth-field word of each s; [36]: no solid neighbour
+    };
 };
 
-// Offsets (into FixSmem::d, from a row's own place in D_1) of the planes that level S adds.
+// Offsets (into Smem::d, from a row's own place in D_1) of the planes that level S adds.
 // Level 3 stands for every s <= 3, whose voxels all keep their word.
 struct FixLevel {
     int n = 0;
     int off[160] = {};
 };
+template <class T>
 constexpr FixLevel fix_level(int S) {
     FixLevel r;
     for (int dz = -7; dz <= 7; dz++)
@@ -126,32 +138,41 @@ constexpr FixLevel fix_level(int S) {
                 const int s = c + (k - 1) * (k - 1);
                 if (S == 3 ? s <= 3 : s == S) best = k;
             }
-            if (best) r.off[r.n++] = (best - 1) * kFixPlane + dz * kFixPitch + dy;
+            if (best) r.off[r.n++] = (best - 1) * T::kPlane + dz * T::kPitch + dy;
         }
     return r;
 }
 
-template <int S>
+template <class T, int S>
 struct FixTable {
-    static constexpr FixLevel L = fix_level(S);
+    static constexpr FixLevel L = fix_level<T>(S);
 };
 
-template <int S, int... I>
+// The first level of a row's part g of n: parts of about as many reads each.
+constexpr int fix_part(int g, int n) {
+    int total = 0, sum = 0, S = 3;
+    for (int i = 3; i < kFixLevels; i++) total += fix_level<FixTile<16>>(i).n;
+    while (S < kFixLevels && sum * n < total * g) sum += fix_level<FixTile<16>>(S++).n;
+    return S;
+}
+constexpr int kFixPart1 = fix_part(1, 4), kFixPart2 = fix_part(2, 4), kFixPart3 = fix_part(3, 4);
+
+template <class T, int S, int... I>
 __device__ __forceinline__ uint32_t fix_or(const uint32_t* d, std::integer_sequence<int, I...>) {
     uint32_t f = 0;
-    ((f |= d[std::integral_constant<int, FixTable<S>::L.off[I]>::value]), ...);
+    ((f |= d[std::integral_constant<int, FixTable<T, S>::L.off[I]>::value]), ...);
     return f;
 }
 
 // Add level S (and the levels after it) to a row: found = voxels whose smallest s is known.
 // Now and then the warp looks whether every air voxel of its rows has been found.
-template <int S>
+template <class T, int S, int END>
 __device__ __forceinline__ void fix_levels(const uint32_t* d, uint32_t air, uint32_t& found, uint32_t (&bit)[6]) {
-    if constexpr (S < kFixLevels) {
+    if constexpr (S < END) {
         if constexpr (S == 5 || S == 10 || S == 17 || S == 26)
             if (!__any_sync(0xffffffffu, (air & ~found) != 0)) return;
-        if constexpr (FixTable<S>::L.n > 0) {
-            const uint32_t now = fix_or<S>(d, std::make_integer_sequence<int, FixTable<S>::L.n>{}) & ~found;
+        if constexpr (FixTable<T, S>::L.n > 0) {
+            const uint32_t now = fix_or<T, S>(d, std::make_integer_sequence<int, FixTable<T, S>::L.n>{}) & ~found;
             found |= now;
             if (S & 1) bit[0] |= now;
             if (S & 2) bit[1] |= now;
@@ -160,23 +181,26 @@ __device__ __forceinline__ void fix_levels(const uint32_t* d, uint32_t air, uint
             if (S & 16) bit[4] |= now;
             if (S & 32) bit[5] |= now;
         }
-        fix_levels<S + 1>(d, air, found, bit);
+        fix_levels<T, S + 1, END>(d, air, found, bit);
     }
 }
 
-// One 32 x 16 x 16 tile by 256 threads, one row each.  Only the air voxels of P.box (and of
+// One 32 x SIDE x SIDE tile.  Only the air voxels of P.box (and of
 // the sphere, if there is one) are written; only solidity is read, which no thread changes.
-__device__ void fix_tile(const FixPass& P, int tile, FixSmem& s) {
+template <int SIDE>
+__device__ void fix_tile(const FixPass& P, int tile, typename FixTile<SIDE>::Smem& s) {
+    using T = FixTile<SIDE>;
     const Layout& L = P.L;
     const int tx = tile % P.ntx, ty = (tile / P.ntx) % P.nty, tz = tile / (P.ntx * P.nty);
-    const int x0 = (P.tx0 + tx) * kFixX, y0 = (P.ty0 + ty) * kFixY, z0 = (P.tz0 + tz) * kFixZ;
-    const int t = threadIdx.x;
+    const int x0 = (P.tx0 + tx) * kFixX, y0 = (P.ty0 + ty) * SIDE, z0 = (P.tz0 + tz) * SIDE;
+    const int t = threadIdx.x, row = t & (SIDE * SIDE - 1);
+    const int part = T::kParts == 1 ? 0 : t >> 2 * T::kShift;  // the same for a warp's lanes
 
     // the bricks the tile and its halo span; bricks beyond the grid hold no solid voxel
     const int bx0 = x0 / 4 - 2, by0 = y0 / 4 - 2, bz0 = z0 / 4 - 2;
     bool solid = false;
-    for (int i = t; i < kFixNodes; i += 256) {
-        const int bx = bx0 + i % 12, by = by0 + (i / 12) % 8, bz = bz0 + i / 96;
+    for (int i = t; i < T::kNodes; i += 256) {
+        const int bx = bx0 + i % 12, by = by0 + (i / 12) % T::kSpan, bz = bz0 + i / (12 * T::kSpan);
         uint64_t m = 0;
         if (bx >= 0 && by >= 0 && bz >= 0 && bx < L.BWp && by < L.BHp && bz < L.BWp)
             m = P.bricks[brick_index(L, bx, by, bz)];
@@ -187,11 +211,11 @@ __device__ void fix_tile(const FixPass& P, int tile, FixSmem& s) {
     const bool any_solid = __syncthreads_or(solid);
 
     // this thread's own row, and the voxels of it that may be written
-    const int y = y0 + (t & 15), z = z0 + (t >> 4);
+    const int ly = row & (SIDE - 1), lz = row >> T::kShift, y = y0 + ly, z = z0 + lz;
     const uint32_t* n32 = reinterpret_cast<const uint32_t*>(s.nodes);
     uint32_t air = 0;
     if (y >= P.y0 && y < P.y1 && z >= P.z0 && z < P.z1) {
-        const int node = ((y >> 2) - by0) * 12 + ((z >> 2) - bz0) * 96;
+        const int node = ((y >> 2) - by0) * 12 + ((z >> 2) - bz0) * 12 * T::kSpan;
         uint32_t own = 0;
         for (int i = 0; i < 8; i++)
             own |= (n32[2 * (node + 2 + i) + ((z & 3) >> 1)] >> (4 * (y & 3) + 16 * (z & 1)) & 15) << (4 * i);
@@ -203,41 +227,72 @@ __device__ void fix_tile(const FixPass& P, int tile, FixSmem& s) {
     uint32_t found = 0, bit[6] = {0, 0, 0, 0, 0, 0};
     if (any_solid) {
         // D_1 .. D_6 of every row: window bits [8, 40) are the tile's voxels
-        for (int i = t; i < kFixRows * kFixRows; i += 256) {
-            const int ry = i % kFixRows, rz = i / kFixRows;
+        for (int i = t; i < T::kRows * T::kRows; i += 256) {
+            const int ry = i % T::kRows, rz = i / T::kRows;
             const int py = ry + 1, pz = rz + 1;  // rows start at y0 - 7 = 4 * by0 + 1
-            const int node = (py >> 2) * 12 + (pz >> 2) * 96, half = (pz & 3) >> 1;
+            const int node = (py >> 2) * 12 + (pz >> 2) * 12 * T::kSpan, half = (pz & 3) >> 1;
             const int shift = 4 * (py & 3) + 16 * (pz & 1);
             uint64_t w = 0;
 #pragma unroll
             for (int j = 0; j < 12; j++)
                 w |= (uint64_t)(n32[2 * (node + j) + half] >> shift & 15) << (4 * j);
-            uint32_t* d = s.d + rz * kFixPitch + ry;
+            uint32_t* d = s.d + rz * T::kPitch + ry;
             uint32_t c = (uint32_t)(w >> 8);
 #pragma unroll
             for (int k = 1; k <= kFixK; k++) {
                 c |= (uint32_t)(w >> (8 + k)) | (uint32_t)(w >> (8 - k));
-                d[(k - 1) * kFixPlane] = c;
+                d[(k - 1) * T::kPlane] = c;
             }
         }
         __syncthreads();
-        if (__any_sync(0xffffffffu, air != 0))
-            fix_levels<3>(s.d + ((t >> 4) + kFixHalo) * kFixPitch + (t & 15) + kFixHalo, air, found, bit);
+        if (__any_sync(0xffffffffu, air != 0)) {
+            const uint32_t* d = s.d + (lz + kFixHalo) * T::kPitch + ly + kFixHalo;
+            if constexpr (T::kParts == 1) {
+                fix_levels<T, 3, kFixLevels>(d, air, found, bit);
+            } else {
+                switch (part) {
+                    case 0: fix_levels<T, 3, kFixPart1>(d, air, found, bit); break;
+                    case 1: fix_levels<T, kFixPart1, kFixPart2>(d, air, found, bit); break;
+                    case 2: fix_levels<T, kFixPart2, kFixPart3>(d, air, found, bit); break;
+                    default: fix_levels<T, kFixPart3, kFixLevels>(d, air, found, bit); break;
+                }
+            }
+        }
+    }
+    if constexpr (T::kParts > 1) {  // the nearer part's answer counts
+        static_assert(T::kParts == 4 || T::kParts == 1);
+        if (part) {
+#pragma unroll
+            for (int k = 0; k < 6; k++) s.part[part - 1][k][row] = bit[k];
+            s.part[part - 1][6][row] = found;
+        }
+        __syncthreads();
+        if (part == 0) {
+#pragma unroll
+            for (int g = 0; g < T::kParts - 1; g++) {
+                const uint32_t now = s.part[g][6][row] & ~found;
+                found |= now;
+#pragma unroll
+                for (int k = 0; k < 6; k++) bit[k] |= s.part[g][k][row] & now;
+            }
+        }
     }
     // s <= 3 was recorded as 3: those voxels keep their word
     const uint32_t keep = found & ~(bit[2] | bit[3] | bit[4] | bit[5]);
+    if (part == 0) {
 #pragma unroll
-    for (int k = 0; k < 6; k++) s.out[k][t] = bit[k];
-    s.out[6][t] = air & ~keep;
+        for (int k = 0; k < 6; k++) s.out[k][row] = bit[k];
+        s.out[6][row] = air & ~keep;
+    }
     __syncthreads();
 
     // write: four voxels of a row per thread, one 16-byte store where all four change
     const bool vec = (L.W & 3) == 0;
     const int seg = 4 * (t & 7);
-    for (int row = t >> 3; row < kFixY * kFixZ; row += 32) {
+    for (int row = t >> 3; row < SIDE * SIDE; row += 32) {
         uint32_t wr = s.out[6][row] >> seg & 15;
         if (!wr) continue;
-        const int ry = y0 + (row & 15), rz = z0 + (row >> 4), rx = x0 + seg;
+        const int ry = y0 + (row & (SIDE - 1)), rz = z0 + (row >> T::kShift), rx = x0 + seg;
         uint32_t b[6];
 #pragma unroll
         for (int k = 0; k < 6; k++) b[k] = s.out[k][row] >> seg;
@@ -571,21 +626,28 @@ __device__ void merge_boxes(const NodePass& P, int* box) {
 
 // ------------------------------------------------------------------ launches
 
+template <int SIDE>
 union NodeSmem {
     DirSmem dir;
     RegSmem reg;
-    FixSmem fix;
+    typename FixTile<SIDE>::Smem fix;
     int box[8];
 };
 
 // The kinds of work lie one after the other in the grid, the longest first.  All of them only
 // read what the brick pass wrote, and write different arrays.
-__global__ void __launch_bounds__(256) node_pass_kernel(const __grid_constant__ NodePass P) {
-    __shared__ NodeSmem s;
+// SIDE is that of the depth-field tiles.  8 stands for few CTAs, which an edit has: their time is
+// one CTA's chain, and with the 94 registers that the compiler takes without a minimum of CTAs
+// per SM it is shorter than with the 80 of a minimum of 3, with which a whole world's passes
+// are faster.  An edit of radius 8 takes 10.1 us with both launches instead of 10.6, one of
+// radius 7 with its depth field 10.0 instead of 12.5 (11.1 with the small tiles alone).
+template <int SIDE>
+__global__ void __launch_bounds__(256, SIDE == 8 ? 1 : 3) node_pass_kernel(const __grid_constant__ NodePass P) {
+    __shared__ NodeSmem<SIDE> s;
     cudaTriggerProgrammaticLaunchCompletion();
     cudaGridDependencySynchronize();  // the brick pass before it
     int b = blockIdx.x;
-    if (b < P.n_fix) return fix_tile(P.fix, b, s.fix);
+    if (b < P.n_fix) return fix_tile<SIDE>(P.fix, b, s.fix);
     b -= P.n_fix;
     if (b < P.n_dir) return dir_tile(P, b, s.dir);
     b -= P.n_dir;
@@ -596,10 +658,10 @@ __global__ void __launch_bounds__(256) node_pass_kernel(const __grid_constant__ 
 // The depth field alone (fixDepthField over a box): without the distance tiles' 80 registers
 // a fourth CTA fits on each SM.
 __global__ void __launch_bounds__(256, 4) fix_depth_field_kernel(const __grid_constant__ FixPass P) {
-    __shared__ FixSmem s;
+    __shared__ FixTile<16>::Smem s;
     cudaTriggerProgrammaticLaunchCompletion();
     cudaGridDependencySynchronize();
-    fix_tile(P, blockIdx.x, s);
+    fix_tile<16>(P, blockIdx.x, s);
 }
 
 // ------------------------------------------------------------------ brick pass
@@ -872,17 +934,25 @@ static bool fix_tiles(NodePass& N, vrt_world* w, const int64_t v[6], int cx, int
         const float d = i < kFixLevels ? (float)(-std::sqrt((double)i)) : -6.0f;
         std::memcpy(&P.word[i], &d, 4);
     }
-    P.tx0 = P.x0 / kFixX; P.ty0 = P.y0 / kFixY; P.tz0 = P.z0 / kFixZ;
-    P.ntx = (P.x1 - 1) / kFixX - P.tx0 + 1;
-    P.nty = (P.y1 - 1) / kFixY - P.ty0 + 1;
-    N.n_fix = P.ntx * P.nty * ((P.z1 - 1) / kFixZ - P.tz0 + 1);
+    // small tiles where they don't outnumber the SMs; larger boxes pay for their halo, and the depth
+    // field alone (no brick pass ahead) always covers large ones
+    for (int side = 8;; side = 16) {
+        P.small = side == 8;
+        P.tx0 = P.x0 / kFixX; P.ty0 = P.y0 / side; P.tz0 = P.z0 / side;
+        P.ntx = (P.x1 - 1) / kFixX - P.tx0 + 1;
+        P.nty = (P.y1 - 1) / side - P.ty0 + 1;
+        N.n_fix = P.ntx * P.nty * ((P.z1 - 1) / side - P.tz0 + 1);
+        if (side == 16 || (N.n_boxes > 0 && N.n_fix <= w->num_sms)) break;
+    }
     return true;
 }
 
-static int run_node_pass(const NodePass& P, cudaStream_t s, bool behind) {
+static int run_node_pass(const NodePass& P, int num_sms, cudaStream_t s, bool behind) {
     const int blocks = P.n_fix + P.n_dir + P.n_reg + (P.n_boxes > 0 ? 1 : 0);
     if (blocks > 0 && blocks == P.n_fix) VRT_CUDA(launch_behind(behind, fix_depth_field_kernel, dim3(blocks), 256, s, P.fix));
-    else if (blocks > 0) VRT_CUDA(launch_behind(behind, node_pass_kernel, dim3(blocks), 256, s, P));
+    else if (blocks > 0)
+        VRT_CUDA(launch_behind(behind, (P.n_fix ? P.fix.small : blocks <= 2 * num_sms) ? node_pass_kernel<8> : node_pass_kernel<16>,
+                               dim3(blocks), 256, s, P));
     return VRT_OK;
 }
 
@@ -937,7 +1007,7 @@ int change_words(vrt_world* w, const WordChange& c, cudaStream_t s) {
         N.fix.words_z = through ? w->d_words_z : nullptr;
         mark_words(w, c.fix_box, !through);
     }
-    return run_node_pass(N, s, behind);
+    return run_node_pass(N, w->num_sms, s, behind);
 }
 
 int refresh_stop_masks(vrt_world* w, cudaStream_t s, bool behind) {
@@ -957,7 +1027,7 @@ int refresh_stop_masks(vrt_world* w, cudaStream_t s, bool behind) {
     N.regions = w->d_stop_regions;
     N.bdir = reinterpret_cast<uint16_t*>(w->d_sdir);
     N.n_reg = 0;
-    return run_node_pass(N, s, behind);
+    return run_node_pass(N, w->num_sms, s, behind);
 }
 
 }  // namespace vrt
