@@ -716,10 +716,10 @@ __device__ __forceinline__ void level_row(int (&v)[4], int x0, int y, int z, int
     }
 }
 
-template <int OP>
-// 64 registers, so that 4 CTAs of a whole world's pass fit on each SM; an edit's few CTAs take 101
-// (10.13 -> 9.91 us for an edit of radius 8 with both launches).
-__global__ void __launch_bounds__(256, OP == kRemoveSphere || OP == kPlaceVoxel ? 1 : 4) brick_pass_kernel(const __grid_constant__ BrickPass P) {
+template <int OP, int MIN_CTAS>
+// 64 registers, so that 4 CTAs of a large pass fit on each SM; an edit's few CTAs take 101 (MIN_CTAS
+// 1: 10.13 -> 9.91 us for an edit of radius 8 with both launches, but 101.8 -> 116.8 at radius 200).
+__global__ void __launch_bounds__(256, MIN_CTAS) brick_pass_kernel(const __grid_constant__ BrickPass P) {
     cudaTriggerProgrammaticLaunchCompletion();  // the node pass may be put in place behind this
     cudaGridDependencySynchronize();
     const Layout& L = P.L;
@@ -875,7 +875,9 @@ static int run_brick_pass(BrickPass& P, int num_sms, cudaStream_t s, bool behind
     // Whole worlds: as many CTAs as fit at once, each looping over its share
     const unsigned need = (P.tasks + 7) / 8;
     *blocks = (int)std::min<unsigned>(need, (unsigned)num_sms * kBrickCtasPerSm);
-    VRT_CUDA(launch_behind(behind, brick_pass_kernel<OP>, dim3(*blocks), 256, s, P));
+    constexpr int kFew = OP == kRemoveSphere || OP == kPlaceVoxel ? 1 : 4;
+    VRT_CUDA(launch_behind(behind, *blocks <= 2 * num_sms ? brick_pass_kernel<OP, kFew> : brick_pass_kernel<OP, 4>,
+                           dim3(*blocks), 256, s, P));
     return VRT_OK;
 }
 
