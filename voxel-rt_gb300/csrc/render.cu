@@ -1974,7 +1974,7 @@ int vrt_render(vrt_renderer* r, const vrt_world* w, const vrt_uniforms* u, int32
         p.wait_first = how == kPlainFrame;
         const bool debug = dbg && (dbg->hit_index || dbg->cast_mask || dbg->occ_mask || dbg->steps ||
                                    dbg->primary_steps || dbg->shade);
-        const cudaError_t le = launch_frame(r, w, how, how != kCapturedFrame, debug ? render_word_kernel<true> : render_word_kernel<false>,
+        const cudaError_t le = launch_frame(r, w, how, how != kCapturedFrame && w->stamp != 0, debug ? render_word_kernel<true> : render_word_kernel<false>,
                                             grid, threads, S(stream), (const int32_t*)w->d_words, w->L, p);
         if (le != cudaSuccess) {
             cudaGetLastError();

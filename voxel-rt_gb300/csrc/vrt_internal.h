@@ -134,7 +134,8 @@ struct WordChange {
 // Change the words, and bring the masks, distances, solid box and flag up to date: at most two
 // launches.
 int change_words(vrt_world* w, const WordChange& c, cudaStream_t s);
-// Called with every launch that changes what renders read of the world.  False under capture.
+// Called with every launch that changes what renders read of the world.  False under capture, and
+// for a world that a captured graph changes: its launches are plain ones.
 bool mark_changed(vrt_world* w, cudaStream_t s);
 // A launch that may begin, as far as its cudaGridDependencySynchronize, while the kernel ahead on
 // the stream runs, from when all CTAs of that one have begun or let it

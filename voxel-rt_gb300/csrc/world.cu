@@ -48,7 +48,7 @@ bool mark_changed(vrt_world* w, cudaStream_t s) {
         w->in_graph = true;
     }
     w->stamp = w->in_graph ? 0 : next++;
-    return now;
+    return !w->in_graph;
 }
 
 int refresh_stop(vrt_world* w, cudaStream_t s) {
