@@ -197,3 +197,78 @@ def test_changes_and_probes_in_a_row(cuda):
         assert np.array_equal(a[1], b[1])
         for p, q in zip(a[2:], b[2:]):
             assert all(np.array_equal(x, y) for x, y in zip(p, q))
+
+
+UNDRAWN = 7  # fills an image before its frame; a pixel's fourth byte is 255
+
+
+def fresh_images(torch, n, count):
+    return [torch.full((n,), UNDRAWN, dtype=torch.uint8, device="cuda") for _ in range(count)]
+
+
+# Grids whose CTAs all fit at once: a frame, the changes behind it and the frames behind those
+# can all be in place while the first still runs.
+ONE_WAVE = [(5, 3), (96, 96), (228, 120), (320, 200)]
+
+
+@pytest.mark.parametrize("size", ONE_WAVE)
+def test_small_word_frames_of_a_turning_camera(cuda, size):
+    """A renderer's first 71 word frames on a grid, nothing between them, each into an image of
+    its own: the plain frames that record the tiles' classes and those that go by them draw
+    every tile."""
+    torch = pytest.importorskip("torch")
+    w, us = scene(True), views(12)
+    n = size[0] * size[1] * 4
+    expect = [alone(torch, w, u, *size, vrt.KERNEL_WORD)[0] for u in us]
+    s = torch.cuda.current_stream().cuda_stream
+    r, imgs = vrt.Renderer(), fresh_images(torch, n, 71)
+    order = [(k * k + k // 7) % 12 for k in range(71)]
+    torch.cuda.synchronize()
+    for i, img in zip(order, imgs):
+        frame(torch, r, w, us[i], *size, vrt.KERNEL_WORD, img, s)
+    torch.cuda.synchronize()
+    for k, (i, img) in enumerate(zip(order, imgs)):
+        assert torch.equal(img.cpu(), expect[i]), k
+
+
+# the kernels of the three frames behind each change: word frames on a world with jumps, and a word
+# frame followed by tile frames on one without
+@pytest.mark.parametrize("size", ONE_WAVE)
+@pytest.mark.parametrize("kernels,jumps", [((vrt.KERNEL_WORD,) * 3, True),
+                                           ((vrt.KERNEL_WORD, vrt.KERNEL_MASK_PIXEL, vrt.KERNEL_MASK_PIXEL), False)])
+def test_small_frames_behind_changes(cuda, size, kernels, jumps):
+    """Changes of the world, each with three frames behind it, all queued without a wait: no frame
+    sees the world of before the change, the second and third ones included."""
+    torch = pytest.importorskip("torch")
+    us, n, rounds = views(3), size[0] * size[1] * 4, 16
+    s = torch.cuda.current_stream().cuda_stream
+    rng = np.random.default_rng(8)
+    slabs = [torch.from_numpy(np.where(rng.random(W * H * 40) < 0.01, 0x01ff0000 + k, -1).astype(np.int32)).cuda()
+             for k in range(rounds)]
+
+    def change(w, k):
+        if k % 4 == 3:
+            w.upload_device(slabs[k].data_ptr(), (7 + 2 * k) * W * H + 11, W * H * 40 - 13)
+        if jumps and k % 3 == 0:
+            w.fix_depth_field()
+        if k % 5 != 4:  # else the frames follow the slab or the whole depth field directly
+            w.remove_sphere(10 + 5 * k, 6, 30 + 3 * k, (9, 21, 12)[k % 3], 1 if jumps else 0)
+            w.place_voxel(20 + k, 13, 21 + k, 0x0100ff00)
+
+    def run(together):
+        w, r = scene(jumps), vrt.Renderer()
+        imgs = fresh_images(torch, n, 3 * rounds)
+        for k in range(4):  # the renderer's first frames on the grid are plain ones
+            frame(torch, r, w, us[k % 3], *size, kernels[0], torch.empty_like(imgs[0]), s)
+        for k in range(rounds):
+            change(w, k)
+            for j in range(3):
+                if not together:
+                    torch.cuda.synchronize()
+                    r = vrt.Renderer()
+                frame(torch, r, w, us[(k + j) % 3], *size, kernels[j], imgs[3 * k + j], s)
+        torch.cuda.synchronize()
+        return [i.cpu() for i in imgs]
+
+    for k, (a, b) in enumerate(zip(run(True), run(False))):
+        assert torch.equal(a, b), k

@@ -135,3 +135,28 @@ def test_counter_hash_follows_code_not_comments(tmp_path, monkeypatch):
     assert bench.kernel_source_hash() == committed
     cu.write_text(text.replace("__launch_bounds__(128, 7)", "__launch_bounds__(128, 8)"))
     assert bench.kernel_source_hash() != committed
+
+
+def test_kernels_let_the_next_begin_only_as_its_reads_allow():
+    """A kernel that may have to wait for the kernels ahead before its own first access triggers
+    behind that wait, because what is launched behind it (an overlapped frame) reads without one.
+    Kernels that always wait before they read may trigger first; a kernel whose wait stands
+    behind its reads is launched behind a wait of others or plainly."""
+    import re
+    src = os.path.join(ROOT, "voxel-rt_gb300", "csrc")
+    seen = 0
+    for name in ("render.cu", "world.cu", "world_passes.cu"):
+        with open(os.path.join(src, name), encoding="utf-8") as f:
+            text = re.sub(r"//[^\n]*", "", f.read())
+        for kernel in re.split(r"\b__global__\b", text)[1:]:
+            kernel = kernel[:kernel.index("\n}")]
+            trigger = [m.start() for m in re.finditer("cudaTriggerProgrammaticLaunchCompletion", kernel)]
+            waits = [m for m in re.finditer(r"(if \([^;{}]*\) )?cudaGridDependencySynchronize", kernel)]
+            if not trigger:
+                continue
+            seen += 1
+            assert len(trigger) == 1 and waits
+            for m in waits:
+                if m.group(1):
+                    assert m.start() < trigger[0], kernel[:120]
+    assert seen >= 6

@@ -144,6 +144,10 @@ bool mark_changed(vrt_world* w, cudaStream_t s);
 // 10.7 us each, probe, edit and frame 86.7 -> 84.3 us, the level built with four edits and its
 // depth field 161 -> 156 us.  Kernels launched so read what others wrote by plain loads, never
 // the read-only path, whose lines need not be those of after the wait.
+// A kernel that triggers before its own wait lets what is behind it begin while the kernels ahead
+// of it still run: it may write nothing that a kernel without a wait before its reads (an
+// overlapped frame) goes by.  World changes keep to that by the stamp, which makes the next frame
+// wait; a frame that waits first triggers behind its wait.
 template <class... Params, class... Args>
 cudaError_t launch_behind(bool dependent, void (*kern)(Params...), dim3 grid, int threads, cudaStream_t s,
                           const Args&... args) {
