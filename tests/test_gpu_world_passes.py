@@ -144,3 +144,30 @@ def test_edits_with_small_and_large_depth_field_tiles(cuda, oracle, W, H, densit
             oracle.remove_sphere(ref, W, H, *c, r, 1)
             got = w.download(np.empty_like(ref))
             assert np.array_equal(got, ref), (c, r, np.flatnonzero(got != ref)[:4])
+
+
+@pytest.mark.parametrize("W,H", [(33, 17), (64, 20)])
+@pytest.mark.parametrize("where", ["pageable", "page-locked", "device"])
+def test_uploads_from_any_byte_address(cuda, W, H, where):
+    """Words at addresses that no 4-byte load can read, in every memory an upload takes them from."""
+    n = W * H * W
+    words = sparse_words(W, H, W, 0.02)
+    w = make_world(words, W, H)
+    for off in (1, 2, 3, 4, 6):
+        first = 5 * off
+        part = sparse_words(W, H, off, 0.05)[: n - first - off]
+        raw = np.zeros(part.nbytes + 16, np.uint8)
+        if where == "pageable":
+            raw[off:off + part.nbytes] = part.view(np.uint8)
+            w.upload(np.frombuffer(raw.data, np.int32, part.size, off), first)
+        else:
+            raw[off:off + part.nbytes] = part.view(np.uint8)
+            t = cuda.from_numpy(raw)
+            t = t.pin_memory() if where == "page-locked" else t.cuda()
+            if where == "page-locked":
+                w.upload(t.numpy()[off:off + part.nbytes].view(np.int32), first)
+            else:
+                w.upload_device(t.data_ptr() + off, first, part.size)
+        words[first:first + part.size] = part
+        assert np.array_equal(w.download(np.empty_like(words)), words), off
+        check_structures(w, words, W, H)

@@ -339,6 +339,7 @@ static int upload_common(vrt_world* w, const int32_t* src, uint64_t first, uint6
     WordChange c{};
     words_box(w->L, first, count, c.box);
     const int32_t* seen = kind == cudaMemcpyDeviceToDevice ? src : device_view(w, src);
+    if ((uintptr_t)seen & 3) seen = nullptr;  // the pass loads whole words; a copy takes any address
     if (seen) {  // copied by the pass that makes the masks
         c.op = kCopyWords;
         c.src = seen;
