@@ -163,9 +163,10 @@ int vrt_world_get_info(const vrt_world* w, vrt_world_info* out);
 /* glBufferData / glBufferSubData (render.cpp:199-202, :219): copy count words from
  * host memory into words [first, first+count), then refresh the occupancy mask of the
  * bricks touched and read back the depth-field flag (synchronises the stream).
- * Pageable or pinned host memory; kernels read it directly where the device can. */
+ * Pageable or pinned host memory; kernels read it directly where the device can, and it is
+ * copied first elsewhere, as it is from an address that is no multiple of four bytes. */
 int vrt_world_upload(vrt_world* w, const int32_t* host_words, uint64_t first, uint64_t count, void* stream);
-/* Same from device memory. */
+/* Same from device memory: this GPU's is read directly, another's copied first. */
 int vrt_world_upload_device(vrt_world* w, const int32_t* d_words, uint64_t first, uint64_t count, void* stream);
 /* Copy words [first, first+count) back to host memory. */
 int vrt_world_download(const vrt_world* w, int32_t* host_words, uint64_t first, uint64_t count, void* stream);

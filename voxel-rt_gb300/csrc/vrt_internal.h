@@ -134,6 +134,23 @@ struct WordChange {
 // Change the words, and bring the masks, distances, solid box and flag up to date: at most two
 // launches.
 int change_words(vrt_world* w, const WordChange& c, cudaStream_t s);
+// The address at which the brick pass reads an upload's words, or NULL where only a copy may take
+// them: at src, whose attributes are at, for a world on GPU `device`.  A copy takes, or refuses, any
+// address, another GPU's memory included, which a kernel without peer access faults on.
+inline const int32_t* upload_view(const int32_t* src, bool from_host, const cudaPointerAttributes& at, int device,
+                                  bool reads_pageable) {
+    if ((uintptr_t)src & 3) return nullptr;  // the pass loads whole words
+    if (!from_host) return at.type == cudaMemoryTypeDevice && at.device == device ? src : nullptr;
+    // Page-locked memory is mapped; where the device walks the host's page tables (Grace), so is every
+    // other page of the host.  The words then cross the host link once, in the pass that masks them,
+    // without the copy's staging: 64 MiB in 369 us from pageable memory seen before and 409 us from
+    // fresh pages, where the copy and a mask pass took 428 and 472 us.
+    if (at.type == cudaMemoryTypeDevice) return nullptr;  // not host memory: the copy says so
+    if (reads_pageable) return src;
+    return at.type == cudaMemoryTypeHost && !((uintptr_t)at.devicePointer & 3)
+               ? static_cast<const int32_t*>(at.devicePointer)
+               : nullptr;
+}
 // Called with every launch that changes what renders read of the world.  False under capture, and
 // for a world that a captured graph changes: its launches are plain ones.
 bool mark_changed(vrt_world* w, cudaStream_t s);

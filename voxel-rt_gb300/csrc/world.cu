@@ -314,21 +314,6 @@ int vrt_world_get_info(const vrt_world* w, vrt_world_info* out) {
     return VRT_OK;
 }
 
-// The address at which kernels can read host memory, or NULL.  Page-locked memory is mapped;
-// where the device walks the host's page tables (Grace), so is every other page.  The words
-// then cross the host link once, in the pass that masks them, without the copy's staging:
-// 64 MiB in 369 us from pageable memory seen before and 409 us from fresh pages, where the
-// copy and a mask pass took 428 and 472 us.
-static const int32_t* device_view(const vrt_world* w, const int32_t* host) {
-    if (w->reads_pageable) return host;
-    cudaPointerAttributes pa;
-    if (cudaPointerGetAttributes(&pa, host) != cudaSuccess) {
-        (void)cudaGetLastError();  // not a pointer the runtime knows
-        return nullptr;
-    }
-    return pa.type == cudaMemoryTypeHost ? static_cast<const int32_t*>(pa.devicePointer) : nullptr;
-}
-
 static int upload_common(vrt_world* w, const int32_t* src, uint64_t first, uint64_t count, void* stream,
                          cudaMemcpyKind kind) {
     if (!w || (!src && count)) return set_error(VRT_EINVAL, "NULL argument");
@@ -338,8 +323,12 @@ static int upload_common(vrt_world* w, const int32_t* src, uint64_t first, uint6
     if (count == 0) return VRT_OK;
     WordChange c{};
     words_box(w->L, first, count, c.box);
-    const int32_t* seen = kind == cudaMemcpyDeviceToDevice ? src : device_view(w, src);
-    if ((uintptr_t)seen & 3) seen = nullptr;  // the pass loads whole words; a copy takes any address
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, src) != cudaSuccess) {
+        (void)cudaGetLastError();  // not a pointer the runtime knows
+        at.type = cudaMemoryTypeUnregistered;
+    }
+    const int32_t* seen = upload_view(src, kind == cudaMemcpyHostToDevice, at, w->device, w->reads_pageable);
     if (seen) {  // copied by the pass that makes the masks
         c.op = kCopyWords;
         c.src = seen;
