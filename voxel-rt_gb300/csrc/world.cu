@@ -338,12 +338,13 @@ static int upload_common(vrt_world* w, const int32_t* src, uint64_t first, uint6
         c.op = kReadWords;
         VRT_CUDA(cudaMemcpyAsync(w->d_words + first, src, count * 4, kind, S(stream)));
     }
-    int st = change_words(w, c, S(stream));
-    if (st) return st;
+    int flag = 0, st = change_words(w, c, S(stream));
     // the kernel choice depends on the depth-field flag: read it back now
-    int flag = 0;
-    st = read_state(w, flag, S(stream));
-    if (st) return st;
+    if (!st) st = read_state(w, flag, S(stream));
+    if (st) {
+        if (seen) cudaStreamSynchronize(S(stream));  // the caller's memory has no reader after the return
+        return st;
+    }
     w->has_depth_field |= flag;
     return VRT_OK;
 }
