@@ -134,7 +134,8 @@ typedef struct vrt_world_info {
     const int32_t* d_words;         /* device voxel words                             */
     const uint64_t* d_brick_mask;   /* device occupancy mask: one uint64 per 4x4x4 brick (linear) */
     const uint64_t* d_region_mask;  /* device: one uint64 per 16x16x16 region, bit per brick */
-    int32_t has_depth_field;        /* 1 if any word is < -1 (as of the last sync)    */
+    int32_t has_depth_field;        /* 1 if any word is < -1 (as of the last sync), or a captured
+                                       edit of the world may bring such words         */
     uint64_t device_bytes;          /* device memory held by the world                */
 } vrt_world_info;
 
@@ -253,7 +254,11 @@ int vrt_renderer_destroy(vrt_renderer* r);
  * changed box on this stream (allocated and filled on first use: as large as the words).
  * A render of the world that this renderer's last render on the same stream showed, unchanged
  * since, may trace while that one's last tiles run; it writes after that one has ended, so
- * work on the stream sees the renders one after the other. */
+ * work on the stream sees the renders one after the other.
+ * Under stream capture: what the render rebuilds, it rebuilds in each run of the graph (order
+ * such runs against other renders of the world).  The runs of a captured edit change the words
+ * without the host's knowledge: renders of that world rebuild the stop masks, or the whole
+ * z-major copy, each time from then on. */
 int vrt_render(vrt_renderer* r, const vrt_world* w, const vrt_uniforms* u, int32_t width,
                int32_t height, uint8_t* d_rgba, const vrt_debug_out* dbg, uint64_t* d_stats,
                const vrt_render_opts* opts, void* stream);

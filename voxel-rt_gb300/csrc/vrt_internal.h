@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <climits>
 #include <cstdint>
 #include <cstdio>
 #include <string>
@@ -80,6 +81,17 @@ Layout make_layout(int W, int H);
 
 }  // namespace vrt
 
+namespace vrt {
+// When a structure that renders derive from the words was last rebuilt: renders on other streams wait
+// for that.  A rebuild within a stream capture belongs to its graph, so it is known by the capture, up to
+// the next change, and leaves the state of the plain launches as it is.
+struct Derived {
+    cudaEvent_t ready = nullptr;     // recorded after each plain rebuild
+    cudaEvent_t captured = nullptr;  // recorded after the rebuild within capture `capture`
+    unsigned long long capture = 0;  // 0: none since the last change
+};
+}  // namespace vrt
+
 struct vrt_world {
     vrt::Layout L;
     int32_t* d_words = nullptr;
@@ -91,13 +103,15 @@ struct vrt_world {
     uint64_t* d_stop = nullptr;     // depth-field worlds: brick masks of the cells a ray stops at
                                     // (word != -1: solid or depth-field), made on first use
     uint8_t* d_sdir = nullptr;      // directed brick distances over the stop masks
-    bool stop_stale = true;         // the stop structures predate the last change of the words
-    cudaEvent_t stop_ready = nullptr;  // recorded after each rebuild: renders on other streams wait on it
+    vrt::Derived stop;              // when the stop structures were rebuilt
+    bool stop_stale = true;         // they predate the last change of the words
+    bool stop_cleared = false;      // they started from 0
     int32_t* d_words_z = nullptr;   // the word kernel's second copy of the words with x and z swapped
                                     // (index z + W*y + W*H*x), made on first use
+    vrt::Derived z;                 // when the copy was brought up to date
+    bool z_filled = false;          // it has been filled once
     int z_dirty[6] = {0, 0, 0, 0, 0, 0};  // box [x0,x1)x[y0,y1)x[z0,z1) of words changed since the
                                     // copy was last brought up to date (empty: x0 >= x1)
-    cudaEvent_t z_ready = nullptr;  // recorded after each copy update: renders on other streams wait on it
     uint64_t* d_stop_regions = nullptr;  // region masks of the stop masks
     int* d_boxes = nullptr;         // the brick pass's record per CTA (8 ints: solid box, flag, 0)
     int* d_aabb = nullptr;          // bounding box of the solid voxels, brick-granular and
@@ -106,12 +120,17 @@ struct vrt_world {
     int h_aabb[6] = {0, 0, 0, -1, -1, -1};  // host copy passed to the render kernels; kept a
                                     // superset of the device box (read back after uploads)
     int has_depth_field = 0;        // host copy (as of the last sync)
+    int graph_box[6] = {INT_MAX, INT_MAX, INT_MAX, INT_MIN, INT_MIN, INT_MIN};  // a world that captured
+    int graph_depth = 0;            // graphs change: the voxels and the flag that their runs may bring,
+                                    // part of both host copies from then on (note_added)
     uint64_t device_bytes = 0;
     int device = 0;
     int num_sms = 0;
     uint64_t stamp = 0;             // a new one with every change of what renders read (mark_changed),
                                     // 0 for a world with a change in a captured graph
-    bool in_graph = false;          // such a graph's runs change the world unseen
+    bool in_graph = false;          // such a graph's runs change the words unseen: the masks and distances
+                                    // with them, but neither the stop structures nor a large change's
+                                    // z-major copy, which every frame that reads them rebuilds then
     bool reads_pageable = false;    // kernels read pageable host memory through the host's page tables
 };
 
@@ -151,8 +170,12 @@ inline const int32_t* upload_view(const int32_t* src, bool from_host, const cuda
                ? static_cast<const int32_t*>(at.devicePointer)
                : nullptr;
 }
-// Called with every launch that changes what renders read of the world.  False under capture, and
-// for a world that a captured graph changes: its launches are plain ones.
+// The stream's capture: its id, or 0 where launches run.  *plain: no capture is known to be in the way
+// of a launch as a programmatic dependent.
+unsigned long long capture_of(cudaStream_t s, bool* plain);
+// Called with every launch that changes the words, or what plain launches derive from them for
+// renders.  False under capture, and for a world that a captured graph changes: its launches are
+// plain ones.
 bool mark_changed(vrt_world* w, cudaStream_t s);
 // A launch that may begin, as far as its cudaGridDependencySynchronize, while the kernel ahead on
 // the stream runs, from when all CTAs of that one have begun or let it

@@ -39,49 +39,91 @@ Layout make_layout(int W, int H) {
 
 static inline unsigned blocks_for(uint64_t n, int threads) { return (unsigned)((n + threads - 1) / threads); }
 
+unsigned long long capture_of(cudaStream_t s, bool* plain) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    const bool known = cudaStreamGetCaptureInfo(s, &status, &id) == cudaSuccess;
+    if (!known) cudaGetLastError();  // the legacy stream beside a capture: launches on it are refused
+    *plain = known && status == cudaStreamCaptureStatusNone;
+    return known && status == cudaStreamCaptureStatusActive ? id : 0;
+}
+
 bool mark_changed(vrt_world* w, cudaStream_t s) {
     static std::atomic<uint64_t> next{1};
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    const bool now = cudaStreamIsCapturing(s, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
-    if (!now) {
-        cudaGetLastError();
-        w->in_graph = true;
-    }
+    bool plain = false;
+    if (capture_of(s, &plain)) w->in_graph = true;
     w->stamp = w->in_graph ? 0 : next++;
-    return !w->in_graph;
+    return plain && !w->in_graph;
+}
+
+// Whether stream s may read a derived structure as it is: the last rebuild that its launches see is
+// waited for.  fresh: the plain launches' one is up to date, as far as the host knows.
+static int see_derived(const vrt_world* w, const Derived& d, bool fresh, unsigned long long capture, cudaStream_t s,
+                       bool* seen) {
+    const bool here = capture && d.capture == capture;
+    *seen = here || (fresh && !w->in_graph);
+    if (here) VRT_CUDA(cudaStreamWaitEvent(s, d.captured, 0));
+    // the last rebuild, on whichever stream; in_graph: another one follows, which writes the same arrays
+    else if (d.ready && (*seen || (w->in_graph && !capture))) VRT_CUDA(cudaStreamWaitEvent(s, d.ready, 0));
+    return VRT_OK;
+}
+
+// Note a rebuild that was launched on stream s.
+static int derived_now(Derived& d, unsigned long long capture, cudaStream_t s) {
+    if (!capture) {
+        VRT_CUDA(cudaEventRecord(d.ready, s));
+        return VRT_OK;
+    }
+    VRT_CUDA(cudaEventRecord(d.captured, s));
+    d.capture = capture;
+    return VRT_OK;
+}
+
+static cudaError_t make_events(Derived& d) {
+    cudaError_t e = cudaEventCreateWithFlags(&d.ready, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&d.captured, cudaEventDisableTiming);
+    return e;
+}
+
+static void destroy_events(Derived& d) {
+    if (d.ready) cudaEventDestroy(d.ready);
+    if (d.captured) cudaEventDestroy(d.captured);
+    d = Derived{};
 }
 
 int refresh_stop(vrt_world* w, cudaStream_t s) {
-    if (!w->stop_stale) {
-        VRT_CUDA(cudaStreamWaitEvent(s, w->stop_ready, 0));  // the last rebuild, on whichever stream
-        return VRT_OK;
-    }
+    bool plain = false, seen = false;
+    const unsigned long long capture = capture_of(s, &plain);
+    int st = see_derived(w, w->stop, !w->stop_stale, capture, s, &seen);
+    if (st || seen) return st;
     const Layout& L = w->L;
-    const bool behind = mark_changed(w, s);
+    const bool behind = !capture && mark_changed(w, s);
     if (!w->d_stop) {
         cudaError_t e = cudaMalloc(&w->d_stop, L.n_bricks * 8);
         if (e == cudaSuccess) e = cudaMalloc(&w->d_sdir, L.n_bricks * 8);
         if (e == cudaSuccess) e = cudaMalloc(&w->d_stop_regions, L.n_regions * 8);
-        if (e == cudaSuccess) e = cudaMemsetAsync(w->d_stop, 0, L.n_bricks * 8, s);
-        if (e == cudaSuccess) e = cudaMemsetAsync(w->d_stop_regions, 0, L.n_regions * 8, s);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&w->stop_ready, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = make_events(w->stop);
         if (e != cudaSuccess) {
             cudaGetLastError();
             cudaFree(w->d_stop);
             cudaFree(w->d_sdir);
             cudaFree(w->d_stop_regions);
-            if (w->stop_ready) cudaEventDestroy(w->stop_ready);
+            destroy_events(w->stop);
             w->d_stop = nullptr;
             w->d_sdir = nullptr;
             w->d_stop_regions = nullptr;
-            w->stop_ready = nullptr;
             return set_error(VRT_ENOMEM, "stop masks: %s", cudaGetErrorString(e));
         }
         w->device_bytes += L.n_bricks * 16 + L.n_regions * 8;
     }
-    const int st = refresh_stop_masks(w, s, behind);
-    if (st) return st;
-    VRT_CUDA(cudaEventRecord(w->stop_ready, s));
+    if (!w->stop_cleared) {
+        VRT_CUDA(cudaMemsetAsync(w->d_stop, 0, L.n_bricks * 8, s));
+        VRT_CUDA(cudaMemsetAsync(w->d_stop_regions, 0, L.n_regions * 8, s));
+    }
+    st = refresh_stop_masks(w, s, behind);
+    if (!st) st = derived_now(w->stop, capture, s);
+    if (st || capture) return st;
+    w->stop_cleared = true;
     w->stop_stale = false;
     return VRT_OK;
 }
@@ -96,7 +138,9 @@ void mark_words(vrt_world* w, const int64_t v[6], bool z_copy) {
         hi[a] = (int)h;
     }
     w->stop_stale = true;
+    w->stop.capture = 0;
     if (!z_copy || !w->d_words_z) return;
+    w->z.capture = 0;
     int* b = w->z_dirty;
     const bool empty = b[0] >= b[3];
     for (int a = 0; a < 3; a++) {
@@ -144,23 +188,24 @@ __global__ void words_z_box_kernel(const int32_t* __restrict__ in, int32_t* __re
 int refresh_words_z(vrt_world* w, cudaStream_t s) {
     const Layout& L = w->L;
     int* b = w->z_dirty;
-    if (w->d_words_z && b[0] >= b[3]) {
-        VRT_CUDA(cudaStreamWaitEvent(s, w->z_ready, 0));  // the last update, on whichever stream
-        return VRT_OK;
-    }
-    mark_changed(w, s);
+    bool plain = false, seen = false;
+    const unsigned long long capture = capture_of(s, &plain);
+    const int st = see_derived(w, w->z, w->z_filled && b[0] >= b[3], capture, s, &seen);
+    if (st || seen) return st;
+    if (!capture) mark_changed(w, s);
     if (!w->d_words_z) {
         cudaError_t e = cudaMalloc(&w->d_words_z, L.n_words * sizeof(int32_t));
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&w->z_ready, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = make_events(w->z);
         if (e != cudaSuccess) {
             cudaGetLastError();
             cudaFree(w->d_words_z);
-            if (w->z_ready) cudaEventDestroy(w->z_ready);
+            destroy_events(w->z);
             w->d_words_z = nullptr;
-            w->z_ready = nullptr;
             return set_error(VRT_ENOMEM, "z-major words: %s", cudaGetErrorString(e));
         }
         w->device_bytes += L.n_words * sizeof(int32_t);
+    }
+    if (!w->z_filled || w->in_graph || capture) {  // a graph's run may follow changes outside the box
         dim3 grid((L.W + 63) / 64, (L.W + 63) / 64, L.H);
         words_z_transpose_kernel<<<grid, 256, 0, s>>>(w->d_words, w->d_words_z, L);
     } else {
@@ -169,7 +214,9 @@ int refresh_words_z(vrt_world* w, cudaStream_t s) {
                                                                b[3] - b[0], b[4] - b[1], b[5] - b[2]);
     }
     VRT_CUDA(cudaGetLastError());
-    VRT_CUDA(cudaEventRecord(w->z_ready, s));
+    const int noted = derived_now(w->z, capture, s);
+    if (noted || capture) return noted;
+    w->z_filled = true;
     b[0] = b[3] = 0;
     return VRT_OK;
 }
@@ -202,9 +249,28 @@ static int read_state(vrt_world* w, int& flag, cudaStream_t s) {
     int st[8];
     VRT_CUDA(cudaMemcpyAsync(st, w->d_aabb, sizeof(st), cudaMemcpyDeviceToHost, s));
     VRT_CUDA(cudaStreamSynchronize(s));
-    for (int i = 0; i < 6; i++) w->h_aabb[i] = st[i];
-    flag = st[6];
+    for (int i = 0; i < 3; i++) {
+        w->h_aabb[i] = std::min(st[i], w->graph_box[i]);
+        w->h_aabb[3 + i] = std::max(st[3 + i], w->graph_box[3 + i]);
+    }
+    flag = st[6] | w->graph_depth;
     return VRT_OK;
+}
+
+// A change that was launched brings depth-field words (depth), or solid voxels within the box [lo, hi]:
+// the host copies of the flag and the solid box hold them from now on, and for a world that captured
+// graphs change, whose runs may bring them at any time, past the next look at the words as well.
+static void note_added(vrt_world* w, bool depth, const int* lo, const int* hi) {
+    if (depth) {
+        w->has_depth_field = 1;
+        if (w->in_graph) w->graph_depth = 1;
+    }
+    for (int i = 0; lo && i < 3; i++) {
+        for (int* box : {w->h_aabb, w->in_graph ? w->graph_box : w->h_aabb}) {
+            box[i] = std::min(box[i], lo[i]);
+            box[3 + i] = std::max(box[3 + i], hi[i]);
+        }
+    }
 }
 
 // Reads that a kernel ahead may have written, behind the wait: no __restrict__, which would let
@@ -291,9 +357,9 @@ int vrt_world_destroy(vrt_world* w) {
     cudaFree(w->d_bdir);
     cudaFree(w->d_stop);
     cudaFree(w->d_sdir);
-    if (w->stop_ready) cudaEventDestroy(w->stop_ready);
+    destroy_events(w->stop);
     cudaFree(w->d_words_z);
-    if (w->z_ready) cudaEventDestroy(w->z_ready);
+    destroy_events(w->z);
     cudaFree(w->d_stop_regions);
     cudaFree(w->d_boxes);
     cudaFree(w->d_aabb);
@@ -414,10 +480,9 @@ int vrt_world_sync_flags(vrt_world* w, void* stream) {
 int vrt_world_probe(const vrt_world* w, const int32_t* d_xyz, int32_t n, int32_t* d_words, void* stream) {
     if (!w || n < 0 || (n > 0 && (!d_xyz || !d_words))) return set_error(VRT_EINVAL, "bad probe arguments");
     if (n == 0) return VRT_OK;
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    const bool now = cudaStreamIsCapturing(S(stream), &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
-    if (!now) cudaGetLastError();
-    VRT_CUDA(launch_behind(now, probe_kernel, dim3(blocks_for((uint64_t)n, 256)), 256, S(stream),
+    bool plain = false;
+    capture_of(S(stream), &plain);
+    VRT_CUDA(launch_behind(plain, probe_kernel, dim3(blocks_for((uint64_t)n, 256)), 256, S(stream),
                            (const int32_t*)w->d_words, w->L, d_xyz, (int)n, d_words));
     return VRT_OK;
 }
@@ -480,14 +545,8 @@ int vrt_place_voxel(vrt_world* w, int32_t x, int32_t y, int32_t z, int32_t word,
     std::memcpy(ch.box, box, sizeof(box));
     const int st = change_words(w, ch, S(stream));
     if (st) return st;
-    if (word < -1) w->has_depth_field = 1;
-    if (word >= 0) {  // grow the host copy of the solid box by the voxel's brick
-        const int c[3] = {x & ~3, y & ~3, z & ~3};
-        for (int i = 0; i < 3; i++) {
-            w->h_aabb[i] = std::min(w->h_aabb[i], c[i]);
-            w->h_aabb[3 + i] = std::max(w->h_aabb[3 + i], c[i] + 3);
-        }
-    }
+    const int lo[3] = {x & ~3, y & ~3, z & ~3}, hi[3] = {lo[0] + 3, lo[1] + 3, lo[2] + 3};  // its brick
+    note_added(w, word < -1, word >= 0 ? lo : nullptr, hi);
     return VRT_OK;
 }
 
@@ -502,8 +561,9 @@ int vrt_fix_depth_field_box(vrt_world* w, int32_t x0, int32_t y0, int32_t z0, in
     const int dim[3] = {w->L.W, w->L.H, w->L.W};
     for (int a = 0; a < 3; a++)
         if (std::max<int64_t>(box[a], 0) >= std::min<int64_t>(box[3 + a], dim[a])) return VRT_OK;
-    w->has_depth_field = 1;
-    return change_words(w, c, S(stream));
+    const int st = change_words(w, c, S(stream));
+    note_added(w, true, nullptr, nullptr);
+    return st;
 }
 
 int vrt_remove_sphere(vrt_world* w, int32_t cx, int32_t cy, int32_t cz, int32_t radius, int32_t refresh_depth_field,
@@ -525,9 +585,10 @@ int vrt_remove_sphere(vrt_world* w, int32_t cx, int32_t cy, int32_t cz, int32_t 
             c.fix_box[a] = at[a] - c.fix_r;
             c.fix_box[3 + a] = at[a] + c.fix_r;
         }
-        w->has_depth_field = 1;
     }
-    return change_words(w, c, S(stream));
+    const int st = change_words(w, c, S(stream));
+    note_added(w, c.fix, nullptr, nullptr);
+    return st;
 }
 
 int vrt_world_init_reference(vrt_world* w, void* stream) {
@@ -535,7 +596,7 @@ int vrt_world_init_reference(vrt_world* w, void* stream) {
     WordChange c = whole_world(w->L);
     c.op = kInitLevel;
     c.reset_flag = true;
-    w->has_depth_field = 0;
+    w->has_depth_field = w->graph_depth;
     int flag = 0;
     int st = change_words(w, c, S(stream));
     if (st) return st;
