@@ -258,7 +258,8 @@ int vrt_renderer_destroy(vrt_renderer* r);
  * Under stream capture: what the render rebuilds, it rebuilds in each run of the graph (order
  * such runs against other renders of the world).  The runs of a captured edit change the words
  * without the host's knowledge: renders of that world rebuild the stop masks, or the whole
- * z-major copy, each time from then on. */
+ * z-major copy, each time from then on.  A captured render keeps the kernel and the solid box of
+ * its capture: capture it again after edits that place voxels beyond that box. */
 int vrt_render(vrt_renderer* r, const vrt_world* w, const vrt_uniforms* u, int32_t width,
                int32_t height, uint8_t* d_rgba, const vrt_debug_out* dbg, uint64_t* d_stats,
                const vrt_render_opts* opts, void* stream);
@@ -323,7 +324,8 @@ int vrt_render_batch_noalloc(const vrt_view* views, int32_t count, const vrt_ren
 
 /* A captured CUDA graph of vrt_render_batch over a fixed view list of a world without
  * depth-field words; replay with vrt_batch_graph_launch.  Uniform or image-pointer changes
- * need a new graph; edits of the world's words do not. */
+ * need a new graph; edits of the world's words do not (a launch after an edit that grew the
+ * box of the solid voxels captures the render again).  The world outlives the graph's launches. */
 typedef struct vrt_batch_graph vrt_batch_graph;
 int vrt_batch_graph_create(vrt_renderer* r, const vrt_view* views, int32_t count,
                            const vrt_render_opts* opts, void* stream, vrt_batch_graph** out);

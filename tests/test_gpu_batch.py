@@ -142,3 +142,45 @@ def test_persistent_kernel_per_view_tiles_and_refill(cuda, batch_setup):
     bad[0].tile_w, bad[0].tile_h = 64, 32  # 2048 pixels
     with pytest.raises(vrt.VrtError):
         r.render_batch(bad, plan.opts())
+
+
+@pytest.mark.parametrize("kernel", [vrt.KERNEL_AUTO, vrt.KERNEL_BITMASK])
+@pytest.mark.parametrize("views", [1, 3])
+def test_batch_graph_follows_voxels_outside_the_solid_box(cuda, kernel, views):
+    """Rays end at the box of the solid voxels: a graph made before a voxel was placed beyond it
+    draws the voxel in its later runs, and the ones queued before are left alone."""
+    import ctypes as C
+    torch = cuda
+    W, H, n = 64, 64, 96 * 64 * 4
+    words = np.full(W * H * W, -1, np.int32)
+    words.reshape(W, H, W)[:, :4, :] = 0x01808080
+    w = vrt.World(W, H)
+    w.upload(words)
+    us = []
+    for k in range(views):
+        u = vrt.default_uniforms()
+        u.camPos[:] = (10.3 + k, 30.6, 5.7)
+        u.rotateMatrix[:] = vrt.rotate_matrix(0.1, 0.6)
+        u.lightPos[:] = [30.0, 160.0, 20.0]
+        u.aspectRatio = 1.5
+        us.append(u)
+    imgs = [torch.zeros(n, dtype=torch.uint8, device="cuda") for _ in us]
+    arr = (vrt.View * views)(*[vrt.make_view(w, u, 96, 64, i.data_ptr()) for u, i in zip(us, imgs)])
+    r, g, opts = vrt.Renderer(), C.c_void_p(), vrt.RenderOpts()
+    opts.kernel = kernel
+    s = torch.cuda.current_stream().cuda_stream
+    vrt.check(vrt.lib().vrt_batch_graph_create(r.handle, arr, views, C.byref(opts), s, C.byref(g)))
+    seen = []
+    for voxel in (None, (24, 24, 24), None, (40, 40, 40), (20, 30, 20)):
+        if voxel:
+            for d in range(4):
+                w.place_voxel(voxel[0] + d, voxel[1], voxel[2], 0x01FF8000, s)
+        vrt.check(vrt.lib().vrt_batch_graph_launch(g, s))
+        got = [i.clone() for i in imgs]
+        r.render_batch(arr, opts, s)
+        seen.append(got)
+        torch.cuda.synchronize()
+        for a, b in zip(got, imgs):
+            assert torch.equal(a, b), voxel
+    vrt.lib().vrt_batch_graph_destroy(g)
+    assert not torch.equal(seen[0][0], seen[1][0]) and not torch.equal(seen[2][0], seen[3][0])

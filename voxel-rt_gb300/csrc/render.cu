@@ -1579,12 +1579,24 @@ struct vrt_renderer {
     cudaStream_t seen_stream = nullptr;
 };
 
+struct Tuning {
+    int tile_w, tile_h, refill_min, blocks_per_sm, exact_steps;
+};
+
 struct vrt_batch_graph {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     ViewDev* d_views = nullptr;
     unsigned int* d_counter = nullptr;
     cudaStream_t capture_stream = nullptr;
+    // what the launch was captured from, for the next capture: its parameters hold the world's solid box
+    const vrt_world* world = nullptr;
+    int box[6] = {};
+    std::vector<ViewDev> views;
+    int total = 0;
+    Tuning t{};
+    bool tiles = true;
+    vrt_renderer shape;  // only its device and SM count are read
 };
 
 static inline cudaStream_t S(void* s) { return reinterpret_cast<cudaStream_t>(s); }
@@ -1600,10 +1612,6 @@ static int check_uniforms(const vrt_uniforms* u) {
         return set_error(VRT_EINVAL, "maxSteps %d outside [0, 2^24]", u->maxSteps);
     return VRT_OK;
 }
-
-struct Tuning {
-    int tile_w, tile_h, refill_min, blocks_per_sm, exact_steps;
-};
 
 static Tuning tuning_of(const vrt_render_opts* o) {
     Tuning t{8, 4, 8, 4, 0};
@@ -2215,6 +2223,31 @@ int vrt_render_batch(vrt_renderer* r, const vrt_view* views, int32_t count, cons
     return render_batch(r, views, count, opts, stream, true);
 }
 
+// Capture a batch graph's launch as the world stands, and make or update the executable graph.  Runs
+// in flight or queued keep what they were launched with.
+static int capture_batch(vrt_batch_graph* g) {
+    VRT_CUDA(cudaStreamBeginCapture(g->capture_stream, cudaStreamCaptureModeThreadLocal));
+    const int st = launch_batch(&g->shape, g->world, g->views.data(), (int)g->views.size(), g->total, g->t, g->tiles,
+                                g->d_views, g->d_counter, g->capture_stream);
+    cudaGraph_t graph = nullptr;
+    cudaError_t e = cudaStreamEndCapture(g->capture_stream, &graph);
+    if (st || e != cudaSuccess) {
+        if (graph) cudaGraphDestroy(graph);
+        return st ? st : cuda_error(e, "cudaStreamEndCapture");
+    }
+    if (g->graph) cudaGraphDestroy(g->graph);
+    g->graph = graph;
+    cudaGraphExecUpdateResultInfo info;
+    if (!g->exec || cudaGraphExecUpdate(g->exec, g->graph, &info) != cudaSuccess) {
+        cudaGetLastError();
+        if (g->exec) cudaGraphExecDestroy(g->exec);
+        g->exec = nullptr;
+        VRT_CUDA(cudaGraphInstantiate(&g->exec, g->graph, 0));
+    }
+    std::memcpy(g->box, g->world->h_aabb, sizeof(g->box));
+    return VRT_OK;
+}
+
 int vrt_batch_graph_create(vrt_renderer* r, const vrt_view* views, int32_t count, const vrt_render_opts* opts,
                            void* stream, vrt_batch_graph** out) {
     if (!r || !out) return set_error(VRT_EINVAL, "NULL argument");
@@ -2229,31 +2262,27 @@ int vrt_batch_graph_create(vrt_renderer* r, const vrt_view* views, int32_t count
     st = build_batch(views, count, t, tiles, hv.data(), &w, &total, false);
     if (st) return st;
     vrt_batch_graph* g = new vrt_batch_graph();
+    g->world = w;
+    g->views = std::move(hv);
+    g->total = total;
+    g->t = t;
+    g->tiles = tiles;
+    g->shape.device = r->device;
+    g->shape.num_sms = r->num_sms;
     cudaError_t e = cudaMalloc(&g->d_views, sizeof(ViewDev) * (size_t)count);
     if (e == cudaSuccess) e = cudaMalloc(&g->d_counter, 256);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(g->d_views, hv.data(), sizeof(ViewDev) * count, cudaMemcpyHostToDevice, S(stream));
+        e = cudaMemcpyAsync(g->d_views, g->views.data(), sizeof(ViewDev) * count, cudaMemcpyHostToDevice, S(stream));
     if (e == cudaSuccess) e = cudaStreamSynchronize(S(stream));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&g->capture_stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) {
         vrt_batch_graph_destroy(g);
         return cuda_error(e, "vrt_batch_graph_create");
     }
-    e = cudaStreamBeginCapture(g->capture_stream, cudaStreamCaptureModeThreadLocal);
-    if (e != cudaSuccess) {
+    st = capture_batch(g);
+    if (st) {
         vrt_batch_graph_destroy(g);
-        return cuda_error(e, "cudaStreamBeginCapture");
-    }
-    st = launch_batch(r, w, hv.data(), count, total, t, tiles, g->d_views, g->d_counter, g->capture_stream);
-    e = cudaStreamEndCapture(g->capture_stream, &g->graph);
-    if (st || e != cudaSuccess) {
-        vrt_batch_graph_destroy(g);
-        return st ? st : cuda_error(e, "cudaStreamEndCapture");
-    }
-    e = cudaGraphInstantiate(&g->exec, g->graph, 0);
-    if (e != cudaSuccess) {
-        vrt_batch_graph_destroy(g);
-        return cuda_error(e, "cudaGraphInstantiate");
+        return st;
     }
     *out = g;
     return VRT_OK;
@@ -2261,6 +2290,15 @@ int vrt_batch_graph_create(vrt_renderer* r, const vrt_view* views, int32_t count
 
 int vrt_batch_graph_launch(vrt_batch_graph* g, void* stream) {
     if (!g || !g->exec) return set_error(VRT_EINVAL, "NULL graph");
+    // Rays end at the solid box, so one that edits have grown goes into the launch again.  (One that
+    // shrank may stay as it is.)
+    bool grown = false;
+    for (int a = 0; a < 3; a++)
+        grown |= g->world->h_aabb[a] < g->box[a] || g->world->h_aabb[3 + a] > g->box[3 + a];
+    if (grown) {
+        const int st = capture_batch(g);
+        if (st) return st;
+    }
     VRT_CUDA(cudaGraphLaunch(g->exec, S(stream)));
     return VRT_OK;
 }
