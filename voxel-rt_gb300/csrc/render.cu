@@ -233,19 +233,10 @@ struct WordRay {
 //
 // What bounds it: instruction issue (75 % of the slots while an SM is busy), 47 M warp
 // instructions for an 800x600 frame of the level with three lights.  An iteration is about 35
-// instructions, a jump 45 more, a ray's set-up and shading 400.  The jump's three IEEE
-// divisions as div_by and no prefetch of the words ahead where they lie in L2 (24 instructions
-// in each iteration): that frame 77.7 -> 66.6 us, the app's first frame 67.2 -> 60.3 us (of which
-// the divisions alone are nothing and the prefetch 8 us; see words_are_far).  The
+// instructions, a jump 45 more, a ray's set-up and shading 400.  On that frame, one by one, the
 // intersect adds in the shadow of the load, and not behind it for the iterations that turn out
-// not to jump: 67.2 -> 62.7 and 59.9 -> 54.1 us; the ray's six reciprocals by rcp_near: 61.8
-// and 53.7 us.  Frames in a row that overlap take 47.8 and 38.4 us, and with the word's load
-// predicated instead of branched around 44.9 and 34.4 us.  Tried without gain: 8x4 tiles of the
-// words instead of the second copy (96 us on the app's first frame), both copies' loads
-// predicated (75.7 of 68.1), the hit's results taken after the loop (62.1 and 56.1 of 61.5 and
-// 54.0), 5 to 8 CTAs per SM by fewer registers (67.0-69.3 of 66.6), one warp per CTA (63.6 of
-// 60.3 us with 16x8 tiles), one call site for all shadow rays (46.0 and 35.0 of 44.9 and 34.4),
-// two iterations per trip (46.6 and 35.2).
+// not to jump, save 4.5 us of 67.2, the ray's six reciprocals by rcp_near another 0.9, and in
+// frames that overlap the load predicated instead of branched around 2.9 of 47.8.
 __device__ WordRay cast_word(const Layout& L, const WordParams& p, V3 start, V3 dir, int dist, int maxSteps,
                              bool far) {
     WordRay o;

@@ -506,7 +506,7 @@ int vrt_server_drain(vrt_server* s) {
         }
         if (!busy && !queued) return VRT_OK;
         if (busy) {
-            // wait for the oldest launch instead of spinning
+            // wait for the first busy slot's launch instead of spinning (others may end before it)
             for (auto& sl : s->slots)
                 if (sl.busy) {
                     VRT_CUDA(cudaEventSynchronize(sl.done));

@@ -13,9 +13,9 @@
 // few KB of masks that it spans, and the neighbourhood work of 32 nodes is done by one
 // instruction.
 //
-// Both are latency chains for an edit (4.5 and 8.6 us, a few dozen CTAs), where ten launches
-// of a few microseconds each took 88 us for removeSphere(8) in the 512 x 256 x 512 world, 12.6
-// now, host included.
+// Both are latency chains for an edit (a few dozen CTAs): removeSphere(8) in the 512 x 256 x 512
+// world, edits in a row, host included, takes 9.4 us, where ten launches of a few microseconds
+// each took 88 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -639,8 +639,8 @@ union NodeSmem {
 // SIDE is that of the depth-field tiles.  8 stands for few CTAs, which an edit has: their time is
 // one CTA's chain, and with the 94 registers that the compiler takes without a minimum of CTAs
 // per SM it is shorter than with the 80 of a minimum of 3, with which a whole world's passes
-// are faster.  An edit of radius 8 takes 10.1 us with both launches instead of 10.6, one of
-// radius 7 with its depth field 10.0 instead of 12.5 (11.1 with the small tiles alone).
+// are faster.  That takes 0.5 us off an edit of radius 8, and with the small tiles 2.5 us off one of
+// radius 7 with its depth field (1.4 of them by the tiles).
 template <int SIDE>
 __global__ void __launch_bounds__(256, SIDE == 8 ? 1 : 3) node_pass_kernel(const __grid_constant__ NodePass P) {
     __shared__ NodeSmem<SIDE> s;
@@ -718,7 +718,7 @@ __device__ __forceinline__ void level_row(int (&v)[4], int x0, int y, int z, int
 
 template <int OP, int MIN_CTAS>
 // 64 registers, so that 4 CTAs of a large pass fit on each SM; an edit's few CTAs take 101 (MIN_CTAS
-// 1: 10.13 -> 9.91 us for an edit of radius 8 with both launches, but 101.8 -> 116.8 at radius 200).
+// 1: 0.2 us off an edit of radius 8, but 101.8 -> 116.8 us at radius 200).
 __global__ void __launch_bounds__(256, MIN_CTAS) brick_pass_kernel(const __grid_constant__ BrickPass P) {
     cudaTriggerProgrammaticLaunchCompletion();  // the node pass may be put in place behind this
     cudaGridDependencySynchronize();
@@ -970,7 +970,7 @@ static int64_t volume(const Layout& L, const int64_t v[6]) {
 
 // Edits of at most this many voxels keep the z-major copy up to date word by word, which
 // saves the next frame a launch (3.6 us); each such word is a store of its own sector, so
-// larger changes leave the copy to the next word-kernel render, which copies the box in tiles.
+// larger changes leave the copy to the next word-kernel render, which copies the box in one launch.
 constexpr int64_t kWriteThrough = 1 << 16;
 
 int change_words(vrt_world* w, const WordChange& c, cudaStream_t s) {
